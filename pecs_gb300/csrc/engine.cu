@@ -509,12 +509,6 @@ void set_error_external(const std::string& m) { g_last_error = m; }
 // Engine
 // ---------------------------------------------------------------------------
 
-struct SetTable {  // device pointer arrays of one SetsView
-  std::vector<DBuf<double*>> b, y, w, x;
-  SetsView view{};
-  int max_nrhs = 0;
-};
-
 struct Engine {
   pecs_options opt{};
   std::unique_ptr<Setup> S;
@@ -1752,9 +1746,7 @@ struct LuHandle {
   bool uploaded = false;
   FactorBank bank;
   int nrhs_cap = 0;
-  DBuf<double> b, y, x;
-  std::vector<DBuf<double>> w;
-  SetTable tab;
+  DBuf<double> b, y, x, w;
   cudaStream_t st = nullptr;
   ~LuHandle() {
     if (st) cudaStreamDestroy(st);
@@ -1763,7 +1755,7 @@ struct LuHandle {
 
 namespace {
 // Loads this file's device module on device `dev` (current) and records the
-// device addresses of the no-alloc solve's static arrays; defined with them.
+// device address of the no-alloc solve's static array; defined with it.
 void noalloc_reserve(int dev);
 }  // namespace
 
@@ -2321,34 +2313,21 @@ static void lu_upload(LuHandle& h, int nrhs) {
     h.b.alloc((size_t)nrhs * n);
     h.y.alloc((size_t)nrhs * n);
     h.x.alloc((size_t)nrhs * n);
-    h.w.resize(nrhs);
-    for (auto& w : h.w) {
-      w.alloc(h.bank.set_wtotal(0));
-      w.zero();
-    }
+    h.w.alloc((size_t)nrhs * h.bank.set_wtotal(0));
     h.nrhs_cap = nrhs;
   }
 }
 
-static void lu_bind(LuHandle& h, int nrhs, const double* b, double* x) {
-  const int n = h.F.n;
-  std::vector<double*> hb(nrhs), hy(nrhs), hw(nrhs), hx(nrhs);
-  for (int r = 0; r < nrhs; ++r) {
-    hb[r] = const_cast<double*>(b) + (size_t)r * n;
-    hy[r] = h.y.p + (size_t)r * n;
-    hw[r] = h.w[r].p;
-    hx[r] = x + (size_t)r * n;
-  }
-  h.tab.b.resize(1);
-  h.tab.y.resize(1);
-  h.tab.w.resize(1);
-  h.tab.x.resize(1);
-  h.tab.b[0].upload(hb);
-  h.tab.y[0].upload(hy);
-  h.tab.w[0].upload(hw);
-  h.tab.x[0].upload(hx);
-  h.tab.view.set[0] = SetView{nrhs, h.tab.b[0].p, h.tab.y[0].p, h.tab.w[0].p, h.tab.x[0].p};
-  h.tab.max_nrhs = nrhs;
+// b and x: nrhs vectors of n doubles one after another, read and written in place
+static RowSets lu_sets(const LuHandle& h, int nrhs, const double* b, double* y, double* w, double* x) {
+  RowSets v;
+  RowSet& s = v.set[0];
+  s.nrhs = nrhs;
+  s.n = h.F.n;
+  s.sd = 1;
+  s.sr = h.F.n;
+  s.b = b, s.x = x, s.y = y, s.w = w;
+  return v;
 }
 
 int pecs_lu_solve_device(pecs_lu* lu, int nrhs, const double* b_dev, double* x_dev, void* stream) {
@@ -2356,9 +2335,8 @@ int pecs_lu_solve_device(pecs_lu* lu, int nrhs, const double* b_dev, double* x_d
     if (!lu || nrhs <= 0 || !b_dev || !x_dev) throw PecsError(PECS_E_ARG, "invalid arguments");
     LuHandle& h = lu->h;
     lu_upload(h, nrhs);
-    lu_bind(h, nrhs, b_dev, x_dev);
     cudaStream_t s = stream ? (cudaStream_t)stream : h.st;
-    h.bank.solve(h.tab.view, nrhs, s);
+    h.bank.solve(lu_sets(h, nrhs, b_dev, h.y.p, h.w.p, x_dev), nrhs, s);
     PECS_CUDA(cudaStreamSynchronize(s));
   })
 }
@@ -2370,8 +2348,7 @@ int pecs_lu_solve(pecs_lu* lu, int nrhs, const double* b, double* x) {
     lu_upload(h, nrhs);
     const size_t bytes = (size_t)nrhs * h.F.n * 8;
     PECS_CUDA(cudaMemcpyAsync(h.b.p, b, bytes, cudaMemcpyHostToDevice, h.st));
-    lu_bind(h, nrhs, h.b.p, h.x.p);
-    h.bank.solve(h.tab.view, nrhs, h.st);
+    h.bank.solve(lu_sets(h, nrhs, h.b.p, h.y.p, h.w.p, h.x.p), nrhs, h.st);
     PECS_CUDA(cudaMemcpyAsync(x, h.x.p, bytes, cudaMemcpyDeviceToHost, h.st));
     PECS_CUDA(cudaStreamSynchronize(h.st));
   })
@@ -2410,38 +2387,29 @@ constexpr size_t kNoAllocScratchDoubles = size_t(1) << 20;  // 8 MiB
 constexpr int kNoAllocMaxRhs = 8;
 constexpr int kNoAllocMaxDevices = 64;
 static __device__ __align__(256) double g_noalloc_scratch[kNoAllocScratchDoubles];
-static __device__ __align__(256) double* g_noalloc_ptrs[4 * kNoAllocMaxRhs];
 
-struct NoAllocSlot {
-  double* scratch = nullptr;
-  double** ptrs = nullptr;
-};
 std::mutex g_noalloc_mu;
-NoAllocSlot g_noalloc_slot[kNoAllocMaxDevices];
+double* g_noalloc_slot[kNoAllocMaxDevices];
 
-// The host-side names of the static arrays are only stand-ins: their device
-// addresses are looked up once per device, with that device current.  Taking
-// the first address loads the module, so this runs at factor upload.
+// The host-side name of the static array is only a stand-in: its device
+// address is looked up once per device, with that device current.  Taking
+// it loads the module, so this runs at factor upload.
 void noalloc_reserve(int dev) {
   if (dev < 0 || dev >= kNoAllocMaxDevices) throw PecsError(PECS_E_ARG, "device ordinal too large");
   std::lock_guard<std::mutex> g(g_noalloc_mu);
-  NoAllocSlot& s = g_noalloc_slot[dev];
-  if (!s.scratch) {
+  if (!g_noalloc_slot[dev]) {
     void* a = nullptr;
-    void* b = nullptr;
     PECS_CUDA(cudaGetSymbolAddress(&a, g_noalloc_scratch));
-    PECS_CUDA(cudaGetSymbolAddress(&b, g_noalloc_ptrs));
-    s.scratch = static_cast<double*>(a);
-    s.ptrs = static_cast<double**>(b);
+    g_noalloc_slot[dev] = static_cast<double*>(a);
   }
 }
 
-// Addresses recorded by noalloc_reserve; never loads anything itself.
-NoAllocSlot noalloc_slot(int dev) {
+// The address recorded by noalloc_reserve; never loads anything itself.
+double* noalloc_slot(int dev) {
   if (dev < 0 || dev >= kNoAllocMaxDevices) throw PecsError(PECS_E_ARG, "device ordinal too large");
   std::lock_guard<std::mutex> g(g_noalloc_mu);
-  const NoAllocSlot s = g_noalloc_slot[dev];
-  if (!s.scratch)
+  double* s = g_noalloc_slot[dev];
+  if (!s)
     throw PecsError(PECS_E_STATE, "the static scratch is not reserved on this device: upload the "
                                   "factors there first (pecs_lu_solve or pecs_lu_solve_device)");
   return s;
@@ -2474,20 +2442,9 @@ int pecs_lu_solve_device_noalloc(pecs_lu* lu, int nrhs, const double* b_dev, dou
     PECS_CUDA(cudaPointerGetAttributes(&pa, h.y.p));
     if (pa.device != dev)
       throw PecsError(PECS_E_ARG, "the current device is not the device holding the factors");
-    NoAllocSlot slot = noalloc_slot(dev);
+    double* slot = noalloc_slot(dev);
     cudaStream_t s = stream ? (cudaStream_t)stream : h.st;
-    double* table[4 * kNoAllocMaxRhs];
-    for (int r = 0; r < nrhs; ++r) {
-      table[r] = const_cast<double*>(b_dev) + (size_t)r * n;
-      table[nrhs + r] = slot.scratch + (size_t)r * n;
-      table[2 * nrhs + r] = slot.scratch + (size_t)nrhs * n + (size_t)r * nw;
-      table[3 * nrhs + r] = x_dev + (size_t)r * n;
-    }
-    // pageable source: the call returns once the table has been staged
-    PECS_CUDA(cudaMemcpyAsync(slot.ptrs, table, sizeof(double*) * 4 * nrhs, cudaMemcpyHostToDevice, s));
-    SetsView sv{};
-    sv.set[0] = SetView{nrhs, slot.ptrs, slot.ptrs + nrhs, slot.ptrs + 2 * nrhs, slot.ptrs + 3 * nrhs};
-    h.bank.solve(sv, nrhs, s);
+    h.bank.solve(lu_sets(h, nrhs, b_dev, slot, slot + (size_t)nrhs * n, x_dev), nrhs, s);
     PECS_CUDA(cudaStreamSynchronize(s));
   })
 }

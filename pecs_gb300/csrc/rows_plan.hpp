@@ -1,0 +1,101 @@
+// Tile plan of the few-right-hand-side solve sweeps (rows.cuh).  Host only.
+#pragma once
+#include <cstddef>
+#include <vector>
+
+#include "mf.hpp"
+
+namespace pecs {
+
+constexpr int kRowsThreads = 256;  // threads of a CTA
+constexpr int kRowsMaxSets = 4;
+constexpr int kRowsSlots = 7;      // child update slots in a record
+
+// Where a front position's value comes from (forward): the right-hand side of
+// dof src (update rows: their own slot) and up to kRowsSlots child update slots (-1: no more); with
+// more of them the last entry is -2 - i, and more[i] holds their number, then them.
+struct alignas(16) RowRec {
+  int src;
+  int slot[kRowsSlots];
+};
+
+// A tile: rows x cols values from value `off` on, [column][padded row], applied
+// by one team of threads.  A batch (ts = 0): `pad` whole nodes of equal shape one
+// after another, [node][column][row], a thread per output.
+struct alignas(16) RowItem {
+  int rows, pad, cols;  // rows, rows padded to the vector width (batch: nodes), columns
+  int set;
+  int src, dst;         // first column in the source list / records, first row in the destination list
+  int pt, npt;          // forward: first record and number of the pass-through rows (the last npt rows)
+  long long off;
+  int magic;            // ceil(2^16 / (pad / values per vector))
+  int node, row0;       // bank-wide node (batch: the first), first row
+  int d, leaf;          // forward: first column in the set's assembled columns; node without children
+  int kc;               // columns whose values are staged at a time
+};
+
+// Sizes of a launch's shared memory: the largest of its tiles.
+struct RowShape {
+  int cols = 0;  // columns
+  int npt = 0;   // pass-through rows of nodes with children
+  int vals = 0;  // values of one chunk of columns
+  int chunks = 0;  // chunks of columns
+};
+
+// One tree level: its tiles (teams of ts threads), then its batches.
+struct RowLevel {
+  int first = 0, n_tile = 0, n_batch = 0, ts = kRowsThreads;
+  bool leaf = true;  // no tile node has children
+  RowShape shape;
+  // forward, per set: the tile nodes' column and update records, and their
+  // columns' first place among the set's assembled columns
+  int col[kRowsMaxSets] = {}, n_col[kRowsMaxSets] = {}, d[kRowsMaxSets] = {}, upd[kRowsMaxSets] = {},
+      n_upd[kRowsMaxSets] = {};
+};
+
+// Flow sweep: an entry is `count` tiles from item `first` on (a team of ts threads
+// each), or a batch (ts = 0) of `count` nodes, in topological order.  Each tile, or
+// node of a batch, has a RowSync (from `sync` on): the counter it waits for (-1:
+// none) with its target, and the counter it adds one to (-1: none).
+struct alignas(16) RowEntry {
+  int ts, first, count, sync;
+};
+struct alignas(16) RowSync {
+  int wait, target, signal, unused;
+};
+
+struct RowsPlan {
+  struct Node {
+    int set, j, s, m, level[2], parent, w_off;
+    bool leaf;
+  };
+  struct Dir {
+    std::vector<RowItem> items;
+    std::vector<RowLevel> levels;
+    RowShape flow_shape[4];  // teams of 32, 64, 128, 256 threads
+    std::vector<RowEntry> entries;
+    std::vector<RowSync> sync;
+    // sources: forward the columns' own dofs, backward own dofs, then ~update
+    // dofs; destinations: own dofs, forward then update slots; nodes in level order
+    std::vector<int> src, dst;
+    std::vector<int> src0, dst0;  // first entry of each node
+    std::vector<int> at, pos;     // nodes in level order, and each node's place there
+    long long n_values = 0;
+  };
+  Dir dir[2];  // forward, backward
+  std::vector<Node> nodes;
+  std::vector<int> wtotal;           // update slots per set
+  std::vector<RowRec> rec, upd;      // forward: columns (as dir[0].src), update rows
+  std::vector<int> more;
+  std::vector<std::vector<int>> order;  // per node: its columns in forward order
+  long long entries = 0;             // stored values of the factors, zeros included
+};
+
+// vr: values per 16 bytes; max_nrhs: right-hand sides per set (0: unknown).
+RowsPlan plan_rows(const std::vector<const MfFactor*>& factors, int vr, int max_nrhs);
+
+// The values of direction d in the items' order (n_values of them).
+void pack_rows(const RowsPlan& P, const std::vector<const MfFactor*>& factors, int d, double* out);
+void pack_rows(const RowsPlan& P, const std::vector<const MfFactor*>& factors, int d, float* out);
+
+}  // namespace pecs

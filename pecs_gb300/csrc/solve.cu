@@ -1,6 +1,7 @@
-// Multifrontal solve kernels and their host-side plans (solve.cuh): one
-// launch per tree level (few-right-hand-side and panel kernels), or one
-// persistent dataflow launch per direction (flow sweeps) over the same items.
+// Multifrontal solve kernels of the panel banks and their host-side plans
+// (solve.cuh): one launch per tree level, or one persistent dataflow launch per
+// direction (flow sweeps) over the same items.  Banks with few right-hand sides
+// per set: rows.cu.
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
@@ -8,561 +9,11 @@
 #include <type_traits>
 
 #include "solve.cuh"
+#include "sweep_sync.cuh"
 
 namespace pecs {
 
 namespace {
-
-// Programmatic dependent launch: a sweep level is launched while the previous
-// level still runs; it stages what does not depend on that level (item
-// records, index metadata, its block tile) and then waits for the previous
-// grid's completion and memory (griddepcontrol.wait) before reading vectors.
-// A level lets the next one start once its CTAs are past their main loop.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-
-// Polls of one wait before it gives up (with 64 ns sleeps and a global load
-// each: tens to hundreds of milliseconds, against a whole sweep of well under
-// a millisecond).
-constexpr unsigned kFlowPollLimit = 1u << 18;
-
-__device__ __forceinline__ int ld_acquire_gpu(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ void red_release_gpu(int* p, int v) {
-  asm volatile("red.release.gpu.global.add.s32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
-}
-
-// Bounded wait for *ctr >= target; false (and the error flag set) when the
-// poll limit runs out.
-__device__ __noinline__ bool flow_wait(const int* ctr, int target, int* err) {
-  if (ld_acquire_gpu(ctr) >= target) return true;
-  for (unsigned n = 0; n < kFlowPollLimit; ++n) {
-    __nanosleep(64);
-    if (ld_acquire_gpu(ctr) >= target) return true;
-  }
-  atomicExch(err, 1);
-  return false;
-}
-
-
-// Loads RB consecutive staged values (16-byte aligned) with vector loads.
-template <typename T, int RB>
-__device__ __forceinline__ void load_rhs(const T* p, T (&v)[RB]) {
-  if constexpr (sizeof(T) == 4 && RB % 4 == 0) {
-#pragma unroll
-    for (int q = 0; q < RB / 4; ++q) {
-      const float4 t = reinterpret_cast<const float4*>(p)[q];
-      v[4 * q] = t.x;
-      v[4 * q + 1] = t.y;
-      v[4 * q + 2] = t.z;
-      v[4 * q + 3] = t.w;
-    }
-  } else if constexpr (sizeof(T) == 8 && RB % 2 == 0) {
-#pragma unroll
-    for (int q = 0; q < RB / 2; ++q) {
-      const double2 t = reinterpret_cast<const double2*>(p)[q];
-      v[2 * q] = t.x;
-      v[2 * q + 1] = t.y;
-    }
-  } else {
-#pragma unroll
-    for (int r = 0; r < RB; ++r) v[r] = p[r];
-  }
-}
-
-template <typename T>
-__device__ __forceinline__ T group_sum(T v, int g) {
-  // xor-butterfly inside aligned groups of g lanes (g a power of two <= 32)
-  for (int o = g >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// Vector access for the two RHS layouts: an array of per-RHS vectors
-// (SetView) or one interleaved [dof][rhs] buffer per set (IlSetView).
-__device__ __forceinline__ double getb(const SetView& s, int r, int d) { return s.b[r][d]; }
-__device__ __forceinline__ double gety(const SetView& s, int r, int d) { return s.y[r][d]; }
-__device__ __forceinline__ double getx(const SetView& s, int r, int d) { return s.x[r][d]; }
-__device__ __forceinline__ double getw(const SetView& s, int r, int d) { return s.w[r][d]; }
-// L2-coherent reads (ld.global.cg) of vectors written inside the same launch
-// (flow sweeps: other CTAs' update and solution rows, which share cache lines
-// with rows this SM may have read earlier)
-__device__ __forceinline__ double getw_cg(const SetView& s, int r, int d) { return __ldcg(s.w[r] + d); }
-__device__ __forceinline__ double getx_cg(const SetView& s, int r, int d) { return __ldcg(s.x[r] + d); }
-__device__ __forceinline__ void puty(const SetView& s, int r, int d, double v) { s.y[r][d] = v; }
-__device__ __forceinline__ void putx(const SetView& s, int r, int d, double v) { s.x[r][d] = v; }
-__device__ __forceinline__ void putw(const SetView& s, int r, int d, double v) { s.w[r][d] = v; }
-__device__ __forceinline__ double getb(const IlSetView& s, int r, int d) {
-  return s.b[(size_t)d * s.nrhs + r];
-}
-__device__ __forceinline__ double gety(const IlSetView& s, int r, int d) {
-  return s.y[(size_t)d * s.nrhs + r];
-}
-__device__ __forceinline__ double getx(const IlSetView& s, int r, int d) {
-  return s.x[(size_t)d * s.nrhs + r];
-}
-__device__ __forceinline__ double getw(const IlSetView& s, int r, int d) {
-  return s.w[(size_t)d * s.nrhs + r];
-}
-__device__ __forceinline__ double getw_cg(const IlSetView& s, int r, int d) {
-  return __ldcg(s.w + (size_t)d * s.nrhs + r);
-}
-__device__ __forceinline__ double getx_cg(const IlSetView& s, int r, int d) {
-  return __ldcg(s.x + (size_t)d * s.nrhs + r);
-}
-__device__ __forceinline__ void puty(const IlSetView& s, int r, int d, double v) {
-  s.y[(size_t)d * s.nrhs + r] = v;
-}
-__device__ __forceinline__ void putx(const IlSetView& s, int r, int d, double v) {
-  s.x[(size_t)d * s.nrhs + r] = v;
-}
-__device__ __forceinline__ void putw(const IlSetView& s, int r, int d, double v) {
-  s.w[(size_t)d * s.nrhs + r] = v;
-}
-
-// Sum of the children's update entries that land on front position p.
-template <bool CG, typename SVi>
-__device__ __forceinline__ double gather_updates(const BankView& B, const SVi& st, int r, int c0,
-                                                 int c1) {
-  double v = 0.0;
-  for (int c = c0; c < c1; ++c) v += CG ? getw_cg(st, r, B.cmap_idx[c]) : getw(st, r, B.cmap_idx[c]);
-  return v;
-}
-
-// Forward sweep, large node: CTA computes rows [r0, r1) of Gf * d.
-template <typename T, int RB, typename SV, bool CG = false>
-__device__ void fwd_large(const BankView& B, const SV& S, int4 it, T* sm, int chunk) {
-  const int j = it.x, r0 = it.y, r1 = it.z;
-  const int s = B.s[j];
-  const auto& st = S.set[B.node_set[j]];
-  const int* own = B.own_idx + B.own_off[j];
-  const int* cptr = B.cmap_ptr + B.cm_off[j];
-  const T* G = static_cast<const T*>(B.G) + B.goff[j];
-  const int wo = B.w_off[j];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  {
-    // one chunk of RB right-hand sides (blockIdx.y in the level kernels)
-    const int rb = chunk * RB;
-    if (rb >= st.nrhs) return;
-    const int nr = min(RB, st.nrhs - rb);
-    for (int p = threadIdx.x; p < s; p += blockDim.x) {
-      const int gd = own[p];
-      const int c0 = cptr[p], c1 = cptr[p + 1];
-#pragma unroll
-      for (int r = 0; r < RB; ++r) {
-        double v = 0.0;
-        if (r < nr) v = getb(st, rb + r, gd) - gather_updates<CG>(B, st, rb + r, c0, c1);
-        sm[r * s + p] = (T)v;  // RHS-major: lanes of a warp read consecutive columns
-      }
-    }
-    __syncthreads();
-    // warps per row: 1 (8 rows per item) .. 8 (1 row per item, columns split)
-    const int nrows = r1 - r0;
-    const int wpr = nrows <= 1 ? 8 : (nrows <= 2 ? 4 : (nrows <= 4 ? 2 : 1));
-    T* red = sm + (size_t)s * RB;  // nw x RB partial sums
-    for (int rbase = r0; rbase < r1; rbase += nw / wpr) {
-      const int row = rbase + warp / wpr, part = warp % wpr;
-      T acc[RB];
-#pragma unroll
-      for (int r = 0; r < RB; ++r) acc[r] = T(0);
-      if (row < r1) {
-        const T* g = G + (long long)row * s;
-        for (int c = part * 32 + lane; c < s; c += 32 * wpr) {
-          const T gv = __ldg(g + c);
-#pragma unroll
-          for (int r = 0; r < RB; ++r) acc[r] += gv * sm[r * s + c];
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < RB; ++r) acc[r] = group_sum(acc[r], 32);
-      if (wpr > 1) {
-        if (lane == 0)
-#pragma unroll
-          for (int r = 0; r < RB; ++r) red[warp * RB + r] = acc[r];
-        __syncthreads();
-        if (part == 0)
-#pragma unroll
-          for (int r = 0; r < RB; ++r) {
-            T t = T(0);
-            for (int q = 0; q < wpr; ++q) t += red[(warp + q) * RB + r];
-            acc[r] = t;
-          }
-      }
-      if (part == 0 && row < r1) {
-#pragma unroll
-        for (int r = 0; r < RB; ++r) {
-          if (lane == r && r < nr) {
-            if (row < s) {
-              puty(st, rb + r, own[row], (double)acc[r]);
-            } else {
-              const int t = row - s;
-              const double cu = gather_updates<CG>(B, st, rb + r, cptr[row], cptr[row + 1]);
-              putw(st, rb + r, wo + t, cu + (double)acc[r]);
-            }
-          }
-        }
-      }
-      if (wpr > 1) __syncthreads();
-    }
-    __syncthreads();
-  }
-}
-
-// Forward sweep, thin node (s <= kThinCols): the node's Gf is stored
-// column-major, so lane `row` reads Gf[c][row] for c = 0..s-1: consecutive
-// lanes read consecutive addresses and every lane has s independent loads in
-// flight; no cross-lane reduction.  A warp item covers rows [r0, r1).
-template <typename T, int RB, typename SV, bool CG = false>
-__device__ void fwd_thin(const BankView& B, const SV& S, int4 it, T* sm, int chunk) {
-  const int j = it.x, r0 = it.y, r1 = it.z;
-  const int s = B.s[j], m = B.m[j], f = s + m;
-  const auto& st = S.set[B.node_set[j]];
-  const int* own = B.own_idx + B.own_off[j];
-  const int* cptr = B.cmap_ptr + B.cm_off[j];
-  const T* G = static_cast<const T*>(B.G) + B.goff[j];
-  const int wo = B.w_off[j];
-  const int lane = threadIdx.x & 31;
-  {
-    // one chunk of RB right-hand sides (blockIdx.y in the level kernels)
-    const int rb = chunk * RB;
-    if (rb >= st.nrhs) return;
-    const int nr = min(RB, st.nrhs - rb);
-    for (int p = lane; p < s; p += 32) {
-      const int gd = own[p];
-      const int c0 = cptr[p], c1 = cptr[p + 1];
-#pragma unroll
-      for (int r = 0; r < RB; ++r) {
-        double v = 0.0;
-        if (r < nr) v = getb(st, rb + r, gd) - gather_updates<CG>(B, st, rb + r, c0, c1);
-        sm[p * RB + r] = (T)v;
-      }
-    }
-    __syncwarp();
-    for (int row = r0 + lane; row < r1; row += 32) {
-      T acc[RB];
-#pragma unroll
-      for (int r = 0; r < RB; ++r) acc[r] = T(0);
-      const T* g = G + row;
-#pragma unroll 4
-      for (int c = 0; c < s; ++c) {
-        const T gv = __ldg(g + (long long)c * f);
-        T dv[RB];
-        load_rhs<T, RB>(sm + c * RB, dv);
-#pragma unroll
-        for (int r = 0; r < RB; ++r) acc[r] += gv * dv[r];
-      }
-      if (row < s) {
-#pragma unroll
-        for (int r = 0; r < RB; ++r)
-          if (r < nr) puty(st, rb + r, own[row], (double)acc[r]);
-      } else {
-        const int c0 = cptr[row], c1 = cptr[row + 1];
-#pragma unroll
-        for (int r = 0; r < RB; ++r)
-          if (r < nr) putw(st, rb + r, wo + row - s, gather_updates<CG>(B, st, rb + r, c0, c1) + (double)acc[r]);
-      }
-    }
-    __syncwarp();
-  }
-}
-
-// Backward sweep, large node: rows [r0, r1) of Hb * [y_own ; x_upd].
-template <typename T, int RB, typename SV, bool CG = false>
-__device__ void bwd_large(const BankView& B, const SV& S, int4 it, T* sm, int chunk) {
-  const int j = it.x, r0 = it.y, r1 = it.z;
-  const int s = B.s[j], m = B.m[j], f = s + m;
-  const auto& st = S.set[B.node_set[j]];
-  const int* own = B.own_idx + B.own_off[j];
-  const int* upd = B.upd_idx + B.upd_off[j];
-  const T* H = static_cast<const T*>(B.H) + B.hoff[j];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  {
-    // one chunk of RB right-hand sides (blockIdx.y in the level kernels)
-    const int rb = chunk * RB;
-    if (rb >= st.nrhs) return;
-    const int nr = min(RB, st.nrhs - rb);
-    for (int p = threadIdx.x; p < f; p += blockDim.x) {
-#pragma unroll
-      for (int r = 0; r < RB; ++r) {
-        double v = 0.0;
-        if (r < nr) v = (p < s) ? gety(st, rb + r, own[p]) : (CG ? getx_cg(st, rb + r, upd[p - s]) : getx(st, rb + r, upd[p - s]));
-        sm[r * f + p] = (T)v;
-      }
-    }
-    __syncthreads();
-    const int nrows = r1 - r0;
-    const int wpr = nrows <= 1 ? 8 : (nrows <= 2 ? 4 : (nrows <= 4 ? 2 : 1));
-    T* red = sm + (size_t)f * RB;
-    for (int rbase = r0; rbase < r1; rbase += nw / wpr) {
-      const int row = rbase + warp / wpr, part = warp % wpr;
-      T acc[RB];
-#pragma unroll
-      for (int r = 0; r < RB; ++r) acc[r] = T(0);
-      if (row < r1) {
-        const T* h = H + (long long)row * f;
-        for (int c = part * 32 + lane; c < f; c += 32 * wpr) {
-          const T hv = __ldg(h + c);
-#pragma unroll
-          for (int r = 0; r < RB; ++r) acc[r] += hv * sm[r * f + c];
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < RB; ++r) acc[r] = group_sum(acc[r], 32);
-      if (wpr > 1) {
-        if (lane == 0)
-#pragma unroll
-          for (int r = 0; r < RB; ++r) red[warp * RB + r] = acc[r];
-        __syncthreads();
-        if (part == 0)
-#pragma unroll
-          for (int r = 0; r < RB; ++r) {
-            T t = T(0);
-            for (int q = 0; q < wpr; ++q) t += red[(warp + q) * RB + r];
-            acc[r] = t;
-          }
-      }
-      if (part == 0 && row < r1) {
-#pragma unroll
-        for (int r = 0; r < RB; ++r)
-          if (lane == r && r < nr) putx(st, rb + r, own[row], (double)acc[r]);
-      }
-      if (wpr > 1) __syncthreads();
-    }
-    __syncthreads();
-  }
-}
-
-// Backward sweep, thin node (s + m <= kThinCols): Hb stored column-major.
-template <typename T, int RB, typename SV, bool CG = false>
-__device__ void bwd_thin(const BankView& B, const SV& S, int4 it, T* sm, int chunk) {
-  const int j = it.x, r0 = it.y, r1 = it.z;
-  const int s = B.s[j], m = B.m[j], f = s + m;
-  const auto& st = S.set[B.node_set[j]];
-  const int* own = B.own_idx + B.own_off[j];
-  const int* upd = B.upd_idx + B.upd_off[j];
-  const T* H = static_cast<const T*>(B.H) + B.hoff[j];
-  const int lane = threadIdx.x & 31;
-  {
-    // one chunk of RB right-hand sides (blockIdx.y in the level kernels)
-    const int rb = chunk * RB;
-    if (rb >= st.nrhs) return;
-    const int nr = min(RB, st.nrhs - rb);
-    for (int p = lane; p < f; p += 32) {
-#pragma unroll
-      for (int r = 0; r < RB; ++r) {
-        double v = 0.0;
-        if (r < nr) v = (p < s) ? gety(st, rb + r, own[p]) : (CG ? getx_cg(st, rb + r, upd[p - s]) : getx(st, rb + r, upd[p - s]));
-        sm[p * RB + r] = (T)v;
-      }
-    }
-    __syncwarp();
-    for (int row = r0 + lane; row < r1; row += 32) {
-      T acc[RB];
-#pragma unroll
-      for (int r = 0; r < RB; ++r) acc[r] = T(0);
-      const T* h = H + row;
-#pragma unroll 4
-      for (int c = 0; c < f; ++c) {
-        const T hv = __ldg(h + (long long)c * s);
-        T dv[RB];
-        load_rhs<T, RB>(sm + c * RB, dv);
-#pragma unroll
-        for (int r = 0; r < RB; ++r) acc[r] += hv * dv[r];
-      }
-#pragma unroll
-      for (int r = 0; r < RB; ++r)
-        if (r < nr) putx(st, rb + r, own[row], (double)acc[r]);
-    }
-    __syncwarp();
-  }
-}
-
-template <typename T, int RB, typename SV>
-__global__ void __launch_bounds__(kSolveThreads)
-    k_forward(BankView B, SV S, const int4* __restrict__ items, int n_large,
-              const int4* __restrict__ thin, int n_thin) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* sm = reinterpret_cast<T*>(smem_raw);
-  pdl_trigger();  // the next level may start launching once every CTA here has started
-  pdl_wait();     // every access below may read the previous level's results
-  if ((int)blockIdx.x < n_large) {
-    fwd_large<T, RB, SV>(B, S, items[blockIdx.x], sm, (int)blockIdx.y);
-  } else {
-    const int wib = threadIdx.x >> 5;
-    const int idx = ((int)blockIdx.x - n_large) * (kSolveThreads / 32) + wib;
-    if (idx < n_thin) fwd_thin<T, RB, SV>(B, S, thin[idx], sm + wib * kThinCols * RB, (int)blockIdx.y);
-  }
-}
-
-template <typename T, int RB, typename SV>
-__global__ void __launch_bounds__(kSolveThreads)
-    k_backward(BankView B, SV S, const int4* __restrict__ items, int n_large,
-               const int4* __restrict__ thin, int n_thin) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* sm = reinterpret_cast<T*>(smem_raw);
-  pdl_trigger();
-  pdl_wait();
-  if ((int)blockIdx.x < n_large) {
-    bwd_large<T, RB, SV>(B, S, items[blockIdx.x], sm, (int)blockIdx.y);
-  } else {
-    const int wib = threadIdx.x >> 5;
-    const int idx = ((int)blockIdx.x - n_large) * (kSolveThreads / 32) + wib;
-    if (idx < n_thin) bwd_thin<T, RB, SV>(B, S, thin[idx], sm + wib * kThinCols * RB, (int)blockIdx.y);
-  }
-}
-
-template <typename T, int RB, typename SV>
-void launch_level(bool forward, const BankView& B, const SV& S, const LevelPlan& L,
-                  int max_nrhs, cudaStream_t st) {
-  const int warps = kSolveThreads / 32;
-  const int nblk = L.n_large + (L.n_thin + warps - 1) / warps;
-  if (nblk == 0) return;
-  size_t sm_large = ((size_t)L.max_cols + kSolveThreads / 32) * RB * sizeof(T);
-  size_t sm_thin = L.n_thin ? (size_t)warps * kThinCols * RB * sizeof(T) : 0;
-  size_t smem = std::max(sm_large, sm_thin);
-  const dim3 grid(nblk, (max_nrhs + RB - 1) / RB);
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(kSolveThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (forward)
-    PECS_CUDA(cudaLaunchKernelEx(&cfg, k_forward<T, RB, SV>, B, S, (const int4*)L.items.p, L.n_large,
-                                 (const int4*)L.thin.p, L.n_thin));
-  else
-    PECS_CUDA(cudaLaunchKernelEx(&cfg, k_backward<T, RB, SV>, B, S, (const int4*)L.items.p, L.n_large,
-                                 (const int4*)L.thin.p, L.n_thin));
-}
-
-// The output rows of one item (RHS chunk `chunk`) set to NaN by threads
-// t0 = 0 .. nt-1: a flow item whose wait ran out, so that the solve's results
-// are flagged non-finite.
-template <int RB, bool FWD, typename SV>
-__device__ void poison_rows(const BankView& B, const SV& S, int4 it, int chunk, int t0, int nt) {
-  const int j = it.x, r0 = it.y, r1 = it.z;
-  const int s = B.s[j];
-  const auto& st = S.set[B.node_set[j]];
-  const int* own = B.own_idx + B.own_off[j];
-  const int rb = chunk * RB;
-  const double nan = __longlong_as_double(0x7ff8000000000000ll);
-  for (int e = t0; e < (r1 - r0) * RB; e += nt) {
-    const int row = r0 + e / RB, r = rb + e % RB;
-    if (r >= st.nrhs) continue;
-    if (!FWD)
-      putx(st, r, own[row], nan);
-    else if (row < s)
-      puty(st, r, own[row], nan);
-    else
-      putw(st, r, B.w_off[j] + row - s, nan);
-  }
-}
-
-// Flow sweep of the few-right-hand-side path: one persistent launch per
-// direction over the level plans' items -- wide-node row chunks (kind 0, a
-// CTA) and groups of up to eight thin-node row chunks (kind 1, a warp each)
-// -- in topological order, with the panel flow sweep's tickets, per-node
-// counters, bounded waits, deferred release signals and reset of the other
-// direction's counters (see k_panel_flow).  Vectors written inside the
-// launch are read with ld.global.cg: their rows (8 or 16 bytes per dof)
-// share cache lines.
-struct RowsFlowView {
-  const int4* entries;  // (kind, first item, item count, RHS chunk)
-  const int4* items;    // (node, row0, row1, 0)
-  const int4* sync;     // (wait counter or -1, target, signal counter or -1, 0)
-  int* ctr;
-  int* other_ctr;
-  int n_ctr;
-  int* queue;
-  int* other_queue;
-  int* err;
-  int n_entries;
-};
-
-template <typename T, int RB, bool FWD, typename SV>
-__global__ void __launch_bounds__(kSolveThreads)
-    k_rows_flow(BankView B, SV S, RowsFlowView F) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* sm = reinterpret_cast<T*>(smem_raw);
-  __shared__ int s_ticket, s_ok;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int i = blockIdx.x * kSolveThreads + tid; i < F.n_ctr; i += gridDim.x * kSolveThreads) F.other_ctr[i] = 0;
-  if (blockIdx.x == 0 && tid == 0) *F.other_queue = 0;
-  int pending = -1;
-  if (tid == 0) s_ticket = atomicAdd(F.queue, 1);
-  for (;;) {
-    __syncthreads();
-    const int t = s_ticket;
-    if (lane == 0 && pending >= 0) red_release_gpu(F.ctr + pending, 1);
-    pending = -1;
-    __syncthreads();
-    if (t >= F.n_entries) break;
-    if (tid == 0) s_ticket = atomicAdd(F.queue, 1);
-    const int4 e = F.entries[t];
-    if (e.x == 0) {
-      const int4 sy = F.sync[e.y];
-      if (tid == 0) s_ok = sy.x < 0 || flow_wait(F.ctr + sy.x, sy.y, F.err);
-      __syncthreads();
-      if (s_ok) {
-        if (FWD)
-          fwd_large<T, RB, SV, true>(B, S, F.items[e.y], sm, e.w);
-        else
-          bwd_large<T, RB, SV, true>(B, S, F.items[e.y], sm, e.w);
-      } else {
-        poison_rows<RB, FWD, SV>(B, S, F.items[e.y], e.w, tid, kSolveThreads);
-      }
-      if (tid == 0) pending = sy.z;
-    } else if (warp < e.z) {
-      const int4 sy = F.sync[e.y + warp];
-      int ok = 1;
-      if (lane == 0) ok = sy.x < 0 || flow_wait(F.ctr + sy.x, sy.y, F.err);
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (ok) {
-        T* wsm = sm + warp * kThinCols * RB;
-        if (FWD)
-          fwd_thin<T, RB, SV, true>(B, S, F.items[e.y + warp], wsm, e.w);
-        else
-          bwd_thin<T, RB, SV, true>(B, S, F.items[e.y + warp], wsm, e.w);
-      } else {
-        poison_rows<RB, FWD, SV>(B, S, F.items[e.y + warp], e.w, lane, 32);
-      }
-      __syncwarp();
-      if (lane == 0) pending = sy.z;
-    }
-  }
-}
-
-template <typename T, int RB>
-void set_smem_limit(size_t bytes) {
-  PECS_CUDA(cudaFuncSetAttribute(k_forward<T, RB, SetsView>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  PECS_CUDA(cudaFuncSetAttribute(k_backward<T, RB, SetsView>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  PECS_CUDA(cudaFuncSetAttribute(k_forward<T, RB, IlSetsView>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  PECS_CUDA(cudaFuncSetAttribute(k_backward<T, RB, IlSetsView>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-}
-
-template <typename T, typename SV>
-void launch_rb(int rb, bool forward, const BankView& B, const SV& S, const LevelPlan& L,
-               int max_nrhs, cudaStream_t st) {
-  switch (rb) {
-    case 1: launch_level<T, 1, SV>(forward, B, S, L, max_nrhs, st); break;
-    case 2: launch_level<T, 2, SV>(forward, B, S, L, max_nrhs, st); break;
-    case 4: launch_level<T, 4, SV>(forward, B, S, L, max_nrhs, st); break;
-    case 8: launch_level<T, 8, SV>(forward, B, S, L, max_nrhs, st); break;
-    default: launch_level<T, 16, SV>(forward, B, S, L, max_nrhs, st); break;
-  }
-}
-
 
 // ---- panel path --------------------------------------------------------------
 constexpr int kPanelKcF32 = 128;  // staged columns per chunk, FP32 blocks
@@ -1598,7 +1049,7 @@ BankView FactorBank::view() const {
 }
 
 int FactorBank::kernel_launches_per_solve() const {
-  if (rows_flow_on_) return 2;
+  if (!panel_) return rows_.launches_per_solve(max_nrhs_);
   if (flow_sel_ >= 0) {
     const int top = flow_cfg_[flow_sel_].top;
     int n = 2;
@@ -1609,8 +1060,6 @@ int FactorBank::kernel_launches_per_solve() const {
   int n = 0;
   for (auto& l : pfwd_) n += l.tiles[0].n_items > 0;
   for (auto& l : pbwd_) n += l.tiles[0].n_items > 0;
-  for (auto& l : fwd_) n += (l.n_large + l.n_thin) > 0;
-  for (auto& l : bwd_) n += (l.n_large + l.n_thin) > 0;
   return n;
 }
 
@@ -1628,6 +1077,14 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
   if (prec_ == PECS_PREC_FP64) tune_.chunk = std::min(tune_.chunk, kPanelKcF64);
   if (tune_.min_ctas == 0) tune_.min_ctas = kTargetCtas;
   n_sets_ = (int)factors.size();
+  max_nrhs_ = max_nrhs;
+  if (!panel) {
+    rows_.build(factors, precision, max_nrhs);
+    entries_ = rows_.entries();
+    bytes_ = rows_.bytes();
+    for (int si = 0; si < n_sets_; ++si) set_wtotal_[si] = rows_.set_wtotal(si);
+    return;
+  }
   std::vector<int> hs, hm, own_off, upd_off, w_off, cm_off, own_idx, upd_idx, cmap_ptr, cmap_idx,
       node_set;
   std::vector<long long> goff, hoff;
@@ -1666,23 +1123,14 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
       goff.push_back(go);
       hoff.push_back(ho);
       {
-        // thin blocks (few columns) are stored column-major for thread-per-row
-        // application; wide blocks row-major for warp-per-row application
+        // every block column-major
         const int s_ = nd.s, f_ = nd.s + nd.m;
         const std::vector<double>& g = F.Gf[j];  // f_ x s_ row-major
-        if (panel || s_ <= kThinCols) {
-          for (int c = 0; c < s_; ++c)
-            for (int r = 0; r < f_; ++r) G.push_back(g[(size_t)r * s_ + c]);
-        } else {
-          G.insert(G.end(), g.begin(), g.end());
-        }
+        for (int c = 0; c < s_; ++c)
+          for (int r = 0; r < f_; ++r) G.push_back(g[(size_t)r * s_ + c]);
         const std::vector<double>& h = F.Hb[j];  // s_ x f_ row-major
-        if (panel || f_ <= kThinCols) {
-          for (int c = 0; c < f_; ++c)
-            for (int r = 0; r < s_; ++r) H.push_back(h[(size_t)r * f_ + c]);
-        } else {
-          H.insert(H.end(), h.begin(), h.end());
-        }
+        for (int c = 0; c < f_; ++c)
+          for (int r = 0; r < s_; ++r) H.push_back(h[(size_t)r * f_ + c]);
       }
       go += (long long)F.Gf[j].size();
       ho += (long long)F.Hb[j].size();
@@ -1738,58 +1186,7 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
     H32_.upload(h32);
     bytes_ = (long long)(G.size() + H.size()) * 4;
   }
-  // level plans: uniform work units so a level's time is not set by one long
-  // item.  Thin nodes (cols <= kThinCols): warp items of <= kThinRows rows.
-  // Wide nodes: CTA items of <= kWideRows rows (kWideRows/8 rows per warp).
-  std::vector<std::vector<int4>> keep_items[2], keep_thin[2];  // host copies for the flow plans
-  auto make = [&](const std::vector<LevelNodes>& lv, bool forward, std::vector<LevelPlan>& out) {
-    out.clear();
-    out.resize(lv.size());
-    keep_items[forward ? 0 : 1].assign(lv.size(), {});
-    keep_thin[forward ? 0 : 1].assign(lv.size(), {});
-    for (size_t l = 0; l < lv.size(); ++l) {
-      std::vector<int4> items, thin;
-      int max_cols = 0;
-      for (int g : lv[l].nodes) {
-        const int s = hs[g], m = hm[g], f = s + m;
-        const int cols = forward ? s : f;
-        const int rows = forward ? f : s;
-        if (cols <= kThinCols) {
-          for (int r0 = 0; r0 < rows; r0 += kThinRows)
-            thin.push_back(make_int4(g, r0, std::min(rows, r0 + kThinRows), 0));
-        } else {
-          max_cols = std::max(max_cols, cols);
-        }
-      }
-      // wide nodes: 8 rows per CTA item (one per warp), fewer when the level
-      // would not give the GPU enough CTAs -- down to one row whose columns are
-      // split over the CTA's eight warps
-      long long wide_rows = 0;
-      for (int g : lv[l].nodes) {
-        const int s = hs[g], m = hm[g];
-        const int cols = forward ? s : s + m;
-        if (cols > kThinCols) wide_rows += forward ? s + m : s;
-      }
-      int per = kWideRows;
-      while (per > 1 && wide_rows / per < 2 * kTargetCtas) per /= 2;
-      for (int g : lv[l].nodes) {
-        const int s = hs[g], m = hm[g], f = s + m;
-        const int cols = forward ? s : f;
-        const int rows = forward ? f : s;
-        if (cols <= kThinCols) continue;
-        for (int r0 = 0; r0 < rows; r0 += per)
-          items.push_back(make_int4(g, r0, std::min(rows, r0 + per), 0));
-      }
-      out[l].n_large = (int)items.size();
-      out[l].n_thin = (int)thin.size();
-      out[l].max_cols = max_cols;
-      out[l].items.upload(items);
-      out[l].thin.upload(thin);
-      keep_items[forward ? 0 : 1][l] = items;
-      keep_thin[forward ? 0 : 1][l] = thin;
-    }
-  };
-  if (panel) {
+  {
     // panel items: a node's rows in tiles of ri <= cap rows, for caps 32, 16,
     // 8 and 4 (levels that would not fill the GPU use shorter tiles: more
     // CTAs, column parts per warp)
@@ -1943,8 +1340,6 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
     };
     make_panel(fl, true, pfwd_);
     make_panel(bl, false, pbwd_);
-    fwd_.clear();
-    bwd_.clear();
     if (prec_ == PECS_PREC_FP64)
       set_panel_smem_limit<double, IlSetsView>();
     else
@@ -2023,209 +1418,30 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
         }
       }
     }
-    return;
   }
-  make(fl, true, fwd_);
-  make(bl, false, bwd_);
-  // flow plans over the same items: per node the number of its items (its
-  // signals), waits on the children's (forward) or the parent's (backward)
-  {
-    const int n_nodes = (int)hs.size();
-    n_nodes_ = n_nodes;
-    std::vector<int> parent(n_nodes, -1);
-    int b0 = 0;
-    for (int fi = 0; fi < n_sets_; ++fi) {
-      const MfFactor& F = *factors[fi];
-      for (int j = 0; j < (int)F.nodes.size(); ++j)
-        for (int c : F.nodes[j].children) parent[b0 + c] = b0 + j;
-      b0 += (int)F.nodes.size();
-    }
-    flow_state_.alloc(2 * (size_t)n_nodes + 3);
-    flow_state_.zero();
-    rows_flow_on_ = false;
-    stall_node_ = -1;
-    for (int g = 0; g < (int)factors[0]->nodes.size() && stall_node_ < 0; ++g)
-      if (parent[g] < 0 && !factors[0]->nodes[g].children.empty()) stall_node_ = g;
-    for (int d = 0; d < 2; ++d) {
-      std::vector<int> nsig(n_nodes, 0), kid_sig(n_nodes, 0);
-      for (size_t l = 0; l < keep_items[d].size(); ++l) {
-        for (const int4& it : keep_items[d][l]) ++nsig[it.x];
-        for (const int4& it : keep_thin[d][l]) ++nsig[it.x];
-      }
-      for (int g = 0; g < n_nodes; ++g)
-        if (parent[g] >= 0) kid_sig[parent[g]] += nsig[g];
-      std::vector<int4> items, sync, entries;
-      auto push = [&](const int4& it) {
-        const int g = it.x, pa = parent[g];
-        items.push_back(it);
-        sync.push_back(d == 0 ? make_int4(kid_sig[g] > 0 ? g : -1, kid_sig[g], pa, 0)
-                              : make_int4(pa, pa >= 0 ? nsig[pa] : 0, g, 0));
-      };
-      for (size_t l = 0; l < keep_items[d].size(); ++l) {
-        for (const int4& it : keep_items[d][l]) {
-          entries.push_back(make_int4(0, (int)items.size(), 1, 0));
-          push(it);
-        }
-        const std::vector<int4>& th = keep_thin[d][l];
-        for (size_t i = 0; i < th.size(); i += kSolveThreads / 32) {
-          const int n = (int)std::min<size_t>(kSolveThreads / 32, th.size() - i);
-          entries.push_back(make_int4(1, (int)items.size(), n, 0));
-          for (int k = 0; k < n; ++k) push(th[i + k]);
-        }
-      }
-      RowsFlowPlan& P = rows_flow_plan_[d];
-      P.n_entries = (int)entries.size();
-      P.entries.upload(entries);
-      P.items.upload(items);
-      P.sync.upload(sync);
-    }
-  }
-  max_cols_ = 0;
-  for (auto& l : fwd_) max_cols_ = std::max(max_cols_, l.max_cols);
-  for (auto& l : bwd_) max_cols_ = std::max(max_cols_, l.max_cols);
-  const size_t esz = prec_ == PECS_PREC_FP64 ? 8 : 4;
-  const size_t small_need = (size_t)(kSolveThreads / 32) * kThinCols * esz;
-  max_rb_ = 16;
-  while (max_rb_ > 1 &&
-         std::max((size_t)max_cols_ + kSolveThreads / 32, small_need / esz) * max_rb_ * esz > kSmemCap)
-    max_rb_ /= 2;
-  if ((size_t)max_cols_ * esz > kSmemCap) throw PecsError(PECS_E_ARG, "front too large for shared memory");
-  const size_t lim = kSmemCap;
-  if (prec_ == PECS_PREC_FP64) {
-    set_smem_limit<double, 1>(lim);
-    set_smem_limit<double, 2>(lim);
-    set_smem_limit<double, 4>(lim);
-    set_smem_limit<double, 8>(lim);
-    set_smem_limit<double, 16>(lim);
-  } else {
-    set_smem_limit<float, 1>(lim);
-    set_smem_limit<float, 2>(lim);
-    set_smem_limit<float, 4>(lim);
-    set_smem_limit<float, 8>(lim);
-    set_smem_limit<float, 16>(lim);
-  }
-}
-
-int FactorBank::solve_rb(int max_nrhs) const {
-  int rb = max_nrhs <= 1 ? 1 : (max_nrhs <= 2 ? 2 : (max_nrhs <= 4 ? 4 : (max_nrhs <= 8 ? 8 : 16)));
-  if (prec_ == PECS_PREC_FP64) rb = std::min(rb, 8);  // FP64: register budget
-  return std::min(rb, max_rb_);
-}
-
-template <typename T, int RB, typename SV>
-void launch_rows_flow(const BankView& B, const SV& S, const RowsFlowView& Ff, const RowsFlowView& Fb,
-                      size_t smem, cudaStream_t st) {
-  const void* fns[2] = {(const void*)k_rows_flow<T, RB, true, SV>, (const void*)k_rows_flow<T, RB, false, SV>};
-  int dev = 0, n_sm = 0;
-  PECS_CUDA(cudaGetDevice(&dev));
-  PECS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
-  for (int d = 0; d < 2; ++d) {
-    PECS_CUDA(cudaFuncSetAttribute(fns[d], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap));
-    int per_sm = 0;
-    PECS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fns[d], kSolveThreads, smem));
-    const RowsFlowView& F = d == 0 ? Ff : Fb;
-    const int grid = std::max(1, std::min(F.n_entries, std::max(1, per_sm) * n_sm));
-    if (d == 0)
-      k_rows_flow<T, RB, true, SV><<<grid, kSolveThreads, smem, st>>>(B, S, F);
-    else
-      k_rows_flow<T, RB, false, SV><<<grid, kSolveThreads, smem, st>>>(B, S, F);
-    PECS_CUDA(cudaGetLastError());
-  }
-}
-
-template <typename SV>
-void FactorBank::solve_rows_flow(const SV& sets, int max_nrhs, cudaStream_t st) const {
-  const BankView B = view();
-  const int rb = solve_rb(max_nrhs);
-  const size_t esz = prec_ == PECS_PREC_FP64 ? 8 : 4;
-  const size_t smem = std::max(((size_t)max_cols_ + kSolveThreads / 32) * rb * esz,
-                               (size_t)(kSolveThreads / 32) * kThinCols * rb * esz);
-  int* base = flow_state_.p;
-  int* ctr[2] = {base, base + n_nodes_};
-  int* queue[2] = {base + 2 * (size_t)n_nodes_, base + 2 * (size_t)n_nodes_ + 1};
-  int* err = base + 2 * (size_t)n_nodes_ + 2;
-  RowsFlowView F[2];
-  for (int d = 0; d < 2; ++d) {
-    const RowsFlowPlan& P = rows_flow_plan_[d];
-    F[d] = RowsFlowView{P.entries.p, P.items.p, P.sync.p, ctr[d], ctr[1 - d], n_nodes_,
-                        queue[d],    queue[1 - d], err,   P.n_entries};
-  }
-  auto go = [&](auto tag) {
-    using T = decltype(tag);
-    switch (rb) {
-      case 1: launch_rows_flow<T, 1, SV>(B, sets, F[0], F[1], smem, st); break;
-      case 2: launch_rows_flow<T, 2, SV>(B, sets, F[0], F[1], smem, st); break;
-      case 4: launch_rows_flow<T, 4, SV>(B, sets, F[0], F[1], smem, st); break;
-      case 8: launch_rows_flow<T, 8, SV>(B, sets, F[0], F[1], smem, st); break;
-      default: launch_rows_flow<T, 16, SV>(B, sets, F[0], F[1], smem, st); break;
-    }
-  };
-  if (prec_ == PECS_PREC_FP64)
-    go(double{});
-  else
-    go(float{});
 }
 
 void FactorBank::tune_rows_flow(const IlSetsView& sets, int max_nrhs, cudaStream_t st, int flow_mode, int reps) {
-  rows_flow_on_ = false;
-  if (panel_ || flow_mode < 0 || max_nrhs > solve_rb(max_nrhs) || rows_flow_plan_[0].n_entries == 0) return;
-  if (flow_mode > 0) {
-    rows_flow_on_ = true;
-    return;
-  }
-  cudaEvent_t e0, e1;
-  PECS_CUDA(cudaEventCreate(&e0));
-  PECS_CUDA(cudaEventCreate(&e1));
-  auto time = [&](bool flow) {
-    rows_flow_on_ = flow;
-    solve(sets, max_nrhs, st);  // warm-up
-    float best = 1e30f;
-    for (int r = 0; r < reps; ++r) {
-      PECS_CUDA(cudaEventRecord(e0, st));
-      solve(sets, max_nrhs, st);
-      PECS_CUDA(cudaEventRecord(e1, st));
-      PECS_CUDA(cudaEventSynchronize(e1));
-      float ms = 0.f;
-      PECS_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-      best = std::min(best, ms);
-    }
-    return best;
-  };
-  const float lev = time(false), flo = time(true);
-  if (flow_error() != 0) throw PecsError(PECS_E_CUDA, "flow sweep: a wait for a node's inputs ran out");
-  if (std::getenv("PECS_TUNE_LOG"))
-    std::fprintf(stderr, "rows flow: %.4f ms (levels %.4f ms)\n", flo, lev);
-  rows_flow_on_ = flo < lev;
-  tuned_ms_ = std::min(flo, lev);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
+  if (!panel_) rows_.tune_flow(row_sets(sets), max_nrhs, st, flow_mode, reps);
 }
 
-template <typename SV>
-void FactorBank::solve_impl(const SV& sets, int max_nrhs, cudaStream_t st) const {
-  if (rows_flow_on_ && max_nrhs <= solve_rb(max_nrhs)) {
-    solve_rows_flow(sets, max_nrhs, st);
-    return;
+RowSets FactorBank::row_sets(const IlSetsView& sets) const {
+  RowSets v;
+  for (int si = 0; si < n_sets_; ++si) {
+    const IlSetView& a = sets.set[si];
+    RowSet& r = v.set[si];
+    r.nrhs = r.sd = a.nrhs;
+    r.n = rows_.dofs(si);
+    r.sr = 1;
+    r.b = a.b, r.x = a.x, r.y = a.y, r.w = a.w;
+    r.d = a.x;  // free until the backward sweep writes the solutions
   }
-  const BankView B = view();
-  const int rb = solve_rb(max_nrhs);
-  for (const LevelPlan& L : fwd_) {
-    if (prec_ == PECS_PREC_FP64)
-      launch_rb<double, SV>(rb, true, B, sets, L, max_nrhs, st);
-    else
-      launch_rb<float, SV>(rb, true, B, sets, L, max_nrhs, st);
-  }
-  for (const LevelPlan& L : bwd_) {
-    if (prec_ == PECS_PREC_FP64)
-      launch_rb<double, SV>(rb, false, B, sets, L, max_nrhs, st);
-    else
-      launch_rb<float, SV>(rb, false, B, sets, L, max_nrhs, st);
-  }
+  return v;
 }
 
-void FactorBank::solve(const SetsView& sets, int max_nrhs, cudaStream_t st) const {
+void FactorBank::solve(const RowSets& sets, int max_nrhs, cudaStream_t st) const {
   if (panel_) throw PecsError(PECS_E_STATE, "panel factor bank needs the interleaved layout");
-  solve_impl(sets, max_nrhs, st);
+  rows_.solve(sets, max_nrhs, st);
 }
 
 void FactorBank::solve(const IlSetsView& sets, int max_nrhs, cudaStream_t st) const {
@@ -2234,7 +1450,7 @@ void FactorBank::solve(const IlSetsView& sets, int max_nrhs, cudaStream_t st) co
   if (panel_)
     solve_panel(sets, max_nrhs, st);
   else
-    solve_impl(sets, max_nrhs, st);
+    rows_.solve(row_sets(sets), max_nrhs, st);
 }
 
 template <typename SVT>
@@ -2247,6 +1463,7 @@ int FactorBank::panel_rpl(const SVT& sets, int max_nrhs) const {
 }
 
 int FactorBank::flow_error(bool clear) const {
+  if (!panel_) return rows_.flow_error(clear);
   if (flow_state_.n == 0) return 0;
   int e = 0;
   int* p = flow_state_.p + 2 * (size_t)n_nodes_ + 2;
@@ -2256,6 +1473,7 @@ int FactorBank::flow_error(bool clear) const {
 }
 
 void FactorBank::debug_arm_flow_stall() const {
+  if (!panel_) return rows_.debug_arm_flow_stall();
   if (flow_state_.n == 0 || stall_node_ < 0) throw PecsError(PECS_E_STATE, "no flow sweep to stall");
   PECS_CUDA(cudaDeviceSynchronize());
   const int v = -(1 << 30);

@@ -6,11 +6,9 @@
 // factor (e.g. electrons and holes of every instance when their mobilities
 // are equal), so that every stored factor entry read from HBM is applied to
 // all of them.  One kernel launch processes one tree level of every factor in
-// the bank: wide nodes are split into row chunks handled by a CTA each
-// (warp per row, coalesced row-major reads, warp-shuffle reduction); thin
-// nodes (few columns) are stored column-major and applied thread-per-row,
-// in warp-sized row chunks.  A bank built for many right-hand sides per set
-// ("panel" banks) stores every block column-major and applies each node as a
+// the bank.  Banks with few right-hand sides per set apply row tiles of the blocks
+// (rows.cuh); a bank built for many right-hand sides per set ("panel" banks)
+// stores every block column-major and applies each node as a
 // small dense GEMM: a CTA stages a chunk of columns of the right-hand sides
 // (interleaved layout: a dof's values are contiguous) and of the block in
 // shared memory, each warp accumulates a 4-row x (32 * RPL)-RHS register tile
@@ -22,16 +20,13 @@
 
 #include "common.hpp"
 #include "mf.hpp"
+#include "rows.cuh"
 
 namespace pecs {
 
 constexpr int kMaxSets = 4;
-constexpr int kThinCols = 128;   // nodes with at most this many columns: thread per row
-constexpr int kThinRows = 32;    // rows per warp item of a thin node (one per lane)
-constexpr int kWideRows = 8;     // rows per CTA item of a wide node (one per warp)
 constexpr int kTargetCtas = 152; // SMs of a GB300: levels with fewer wide items split rows
 constexpr int kSolveThreads = 256;
-constexpr size_t kSmemCap = 200 * 1024;  // dynamic shared memory budget per CTA
 constexpr int kPanelMinRhs = 32;  // right-hand sides per set from which banks use the panel kernels
 
 struct BankView {  // device pointers, passed by value to kernels
@@ -50,18 +45,6 @@ struct BankView {  // device pointers, passed by value to kernels
   const int* node_set;
   const void* G;
   const void* H;
-};
-
-struct SetView {
-  int nrhs;
-  double* const* b;  // right-hand sides (read)
-  double* const* y;  // forward result slots
-  double* const* w;  // update-vector workspace (set_wtotal(set) doubles each)
-  double* const* x;  // solutions (written)
-};
-
-struct SetsView {
-  SetView set[kMaxSets];
 };
 
 // Interleaved layout: all right-hand sides of a set in one buffer, element
@@ -193,20 +176,6 @@ struct FlowPlanHost {
 FlowPlanHost plan_flow(const FlowNodes& nd, bool forward, int top, int rpl, int max_nrhs, int kc_max, int esz,
                        int n_sm);
 
-// The flow sweep of the few-right-hand-side path (one direction): the level
-// plans' wide and thin items in topological order (solve.cu, k_rows_flow).
-struct RowsFlowPlan {
-  int n_entries = 0;
-  DBuf<int4> entries, items, sync;
-};
-
-struct LevelPlan {
-  int n_large = 0, n_thin = 0;
-  DBuf<int4> items;   // wide nodes: (node, row0, row1, 0), one CTA each
-  DBuf<int4> thin;    // thin nodes: (node, row0, row1, 0), one warp each
-  int max_cols = 0;   // staged columns per large item
-};
-
 struct PanelTuning {
   int chunk = 0;     // staged block columns per chunk (0: 128 FP32, 64 FP64)
   int min_ctas = 0;  // CTAs a level must reach before shorter tiles are used (0: one per SM)
@@ -222,15 +191,13 @@ class FactorBank {
   void build(const std::vector<const MfFactor*>& factors, int precision, bool panel = false,
              PanelTuning tuning = PanelTuning(), int max_nrhs = 0);
   // y = forward(b), x = backward(y); w is workspace.  All sets must be bound.
-  void solve(const SetsView& sets, int max_nrhs, cudaStream_t st) const;
+  void solve(const RowSets& sets, int max_nrhs, cudaStream_t st) const;  // few right-hand sides
   void solve(const IlSetsView& sets, int max_nrhs, cudaStream_t st) const;
   void solve(const IlSetsViewF& sets, int max_nrhs, cudaStream_t st) const;
   int set_wtotal(int set) const { return set_wtotal_[set]; }
   int precision() const { return prec_; }
   long long entries() const { return entries_; }
   long long bytes() const { return bytes_; }
-  int n_fwd_levels() const { return (int)fwd_.size(); }
-  int n_bwd_levels() const { return (int)bwd_.size(); }
   int kernel_launches_per_solve() const;
   bool panel() const { return panel_; }
   // Panel banks: choose each level's tiling option by timing whole sweeps on
@@ -244,17 +211,17 @@ class FactorBank {
   // these sets (a few sweeps each; outputs are garbage afterwards) and keep
   // the faster (flow_mode 0), the flow sweep (1) or the levels (-1).
   void tune_rows_flow(const IlSetsView& sets, int max_nrhs, cudaStream_t st, int flow_mode = 0, int reps = 3);
-  bool rows_flow() const { return rows_flow_on_; }
+  bool rows_flow() const { return !panel_ && rows_.flow_on(); }
   // Untuned banks: the flow sweep with the most right-hand sides per lane that
   // applies to these sets (the level sweep if none does).
   void force_flow(const IlSetsViewF& sets, int max_nrhs);
   void force_flow(const IlSetsView& sets, int max_nrhs);
-  double tuned_ms() const { return tuned_ms_; }
+  double tuned_ms() const { return panel_ ? tuned_ms_ : rows_.tuned_ms(); }
   // Panel banks: right-hand sides per lane of the flow sweep in use (0: every
   // level its own launch), and the tree levels it covers from the root side.
   int flow_rpl() const { return flow_sel_ < 0 ? 0 : flow_cfg_[flow_sel_].rpl; }
   int flow_top() const {
-    return rows_flow_on_ ? (int)fwd_.size() : (flow_sel_ < 0 ? 0 : flow_cfg_[flow_sel_].top);
+    return rows_flow() ? rows_.n_levels() : (flow_sel_ < 0 ? 0 : flow_cfg_[flow_sel_].top);
   }
   // 1 if a flow sweep's wait ran out since the bank was built or the flag was
   // last cleared (that sweep's results were written as NaN); synchronises
@@ -271,7 +238,7 @@ class FactorBank {
 
  private:
   int prec_ = PECS_PREC_FP64;
-  int n_sets_ = 0;
+  int n_sets_ = 0, max_nrhs_ = 0;
   int set_wtotal_[kMaxSets] = {0, 0, 0, 0};
   long long entries_ = 0, bytes_ = 0;
   DBuf<int> s_, m_, own_off_, upd_off_, w_off_, cm_off_, own_idx_, upd_idx_, cmap_ptr_, cmap_idx_,
@@ -279,12 +246,10 @@ class FactorBank {
   DBuf<long long> goff_, hoff_;
   DBuf<double> G64_, H64_;
   DBuf<float> G32_, H32_;
-  std::vector<LevelPlan> fwd_, bwd_;
   std::vector<PanelPlan> pfwd_, pbwd_;
   bool panel_ = false;
   PanelTuning tune_;
   int parts_ld_ = 32;  // split-K scratch: right-hand sides per partial row
-  int max_cols_ = 0, max_rb_ = 8;
   template <typename SVT>
   void solve_panel(const SVT& sets, int max_nrhs, cudaStream_t st) const;
   template <typename SVT>
@@ -306,19 +271,14 @@ class FactorBank {
   DBuf<int> flow_state_;  // [2][nodes] counters, 2 tickets, error flag
   int n_nodes_ = 0;
   int stall_node_ = -1;  // the first factor's root (debug_arm_flow_stall)
-  RowsFlowPlan rows_flow_plan_[2];
-  bool rows_flow_on_ = false;
-  int solve_rb(int max_nrhs) const;
-  template <typename SV>
-  void solve_rows_flow(const SV& sets, int max_nrhs, cudaStream_t st) const;
+  RowsSweep rows_;       // banks with few right-hand sides per set (not panel_)
+  RowSets row_sets(const IlSetsView& sets) const;
   void release_unused_flow();
   template <typename SVT>
   bool flow_ok(const SVT& sets, int max_nrhs, int cfg) const;
   template <typename SVT>
   void solve_flow(const SVT& sets, int max_nrhs, int cfg, cudaStream_t st) const;
   BankView view() const;
-  template <typename SV>
-  void solve_impl(const SV& sets, int max_nrhs, cudaStream_t st) const;
 };
 
 }  // namespace pecs
