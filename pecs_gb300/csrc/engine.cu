@@ -68,105 +68,131 @@ struct CsrDfSet {
 };
 
 // ---- interleaved [dof][rhs] buffers of the batched solves --------------------
-// dst[d * R + k] = src_k[d]   (32 x 32 tiles through shared memory); dst32,
-// when given, receives the same values rounded to float (the right-hand sides
-// of the FP32 sweeps)
-__global__ void k_gather_il(const double* const* __restrict__ src, double* __restrict__ dst,
-                            float* __restrict__ dst32, int n, int R) {
+// The element-wise kernels around the sweeps take every set of a bank in one
+// launch (the last grid dimension; grids are sized for the largest set).
+struct ElemSet {
+  int n = 0, R = 0;
+  const double* const* src = nullptr;  // per column: right-hand side
+  const double* const* old = nullptr;  // per column: previous state
+  double* const* dst = nullptr;        // per column: state written
+  double *B = nullptr, *X = nullptr, *D = nullptr, *Rr = nullptr;
+  float *B32 = nullptr, *X32 = nullptr, *D32 = nullptr, *Rr32 = nullptr;
+  float2* Xs = nullptr;
+  CsrDev A{};
+  CsrDf Adf{};
+};
+struct ElemSets {
+  ElemSet s[kMaxSets];
+};
+
+// B[d * R + k] = src_k[d]   (32 x 32 tiles through shared memory); B32, when
+// present, receives the same values rounded to float (the right-hand sides of the
+// FP32 sweeps)
+__global__ void k_gather_il(ElemSets E) {
+  const ElemSet& S = E.s[blockIdx.z];
   __shared__ double t[32][33];
-  const int d0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+  const int n = S.n, R = S.R, d0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+  if (d0 >= n || k0 >= R) return;
   for (int kk = threadIdx.y; kk < 32; kk += blockDim.y) {
     const int k = k0 + kk, d = d0 + threadIdx.x;
-    t[kk][threadIdx.x] = (k < R && d < n) ? src[k][d] : 0.0;
+    t[kk][threadIdx.x] = (k < R && d < n) ? S.src[k][d] : 0.0;
   }
   __syncthreads();
   for (int dd = threadIdx.y; dd < 32; dd += blockDim.y) {
     const int d = d0 + dd, k = k0 + threadIdx.x;
     if (d < n && k < R) {
       const double v = t[threadIdx.x][dd];
-      dst[(size_t)d * R + k] = v;
-      if (dst32) dst32[(size_t)d * R + k] = (float)v;
+      S.B[(size_t)d * R + k] = v;
+      if (S.B32) S.B32[(size_t)d * R + k] = (float)v;
     }
   }
 }
 
-// dst_k[d] = src[d * R + k]
+// What a solve writes to the state: dst_k[d] = one of these at d * R + k.  The last
+// refinement's correction is added here instead of in a pass of its own.
+enum class Out { X, X32, XPlusD, XPlusD32, X32PlusD32 };
+
+template <Out O>
+__device__ __forceinline__ double out_value(const ElemSet& S, size_t o) {
+  if constexpr (O == Out::X) return S.X[o];
+  if constexpr (O == Out::X32) return (double)S.X32[o];
+  if constexpr (O == Out::XPlusD) return S.X[o] + S.D[o];
+  if constexpr (O == Out::XPlusD32) return S.X[o] + (double)S.D32[o];
+  return f2d_exact(S.X32[o]) + f2d_exact(S.D32[o]);
+}
+
 // mask (optional): only columns of instances k / nf with mask[k / nf] != 0
-template <typename V>
-__global__ void k_scatter_il(const V* __restrict__ src, double* const* __restrict__ dst, int n,
-                             int R, const int* __restrict__ mask, int nf) {
+template <Out O>
+__global__ void k_scatter_il(ElemSets E, const int* __restrict__ mask, int n_inst) {
+  const ElemSet& S = E.s[blockIdx.z];
   __shared__ double t[32][33];
-  const int d0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+  const int n = S.n, R = S.R, d0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+  if (d0 >= n || k0 >= R) return;
+  const int nf = R / n_inst;
   for (int dd = threadIdx.y; dd < 32; dd += blockDim.y) {
     const int d = d0 + dd, k = k0 + threadIdx.x;
-    t[dd][threadIdx.x] = (d < n && k < R) ? (double)src[(size_t)d * R + k] : 0.0;
+    t[dd][threadIdx.x] = (d < n && k < R) ? out_value<O>(S, (size_t)d * R + k) : 0.0;
   }
   __syncthreads();
   for (int kk = threadIdx.y; kk < 32; kk += blockDim.y) {
     const int k = k0 + kk, d = d0 + threadIdx.x;
-    if (k < R && d < n && (!mask || mask[k / nf])) dst[k][d] = t[threadIdx.x][kk];
+    if (k < R && d < n && (!mask || mask[k / nf])) S.dst[k][d] = t[threadIdx.x][kk];
   }
 }
 
-__global__ void k_split_il(const double* __restrict__ x, float2* __restrict__ xs, size_t n) {
+// Xs = X as FP32 pairs
+__global__ void k_split_il(ElemSets E) {
+  const ElemSet& S = E.s[blockIdx.y];
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double a = x[i];
+  if (i >= (size_t)S.n * S.R) return;
+  const double a = S.X[i];
   const float hi = __double2float_rn(a);
-  xs[i] = make_float2(hi, __double2float_rn(a - (double)hi));
+  S.Xs[i] = make_float2(hi, __double2float_rn(a - (double)hi));
 }
 
-template <typename V>
-__global__ void k_axpy_il(double* __restrict__ x, const V* __restrict__ d, size_t n) {
+// between refinements: X += D (the correction's type), X = X32 + D32, X = X32
+enum class Upd { AddD, AddD32, Sum32, Widen };
+
+template <Upd U>
+__global__ void k_update_il(ElemSets E) {
+  const ElemSet& S = E.s[blockIdx.y];
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i < n) x[i] += (double)d[i];
+  if (i >= (size_t)S.n * S.R) return;
+  if constexpr (U == Upd::AddD) S.X[i] += S.D[i];
+  if constexpr (U == Upd::AddD32) S.X[i] += (double)S.D32[i];
+  if constexpr (U == Upd::Sum32) S.X[i] = (double)S.X32[i] + (double)S.D32[i];
+  if constexpr (U == Upd::Widen) S.X[i] = (double)S.X32[i];
 }
 
-// dst_k[d] = (double) x32[d * R + k] + (double) d32[d * R + k]: the refined
-// solution of an FP32 sweep and its one correction, written to the state
-__global__ void k_scatter_sum_il(const float* __restrict__ x32, const float* __restrict__ d32,
-                                 double* const* __restrict__ dst, int n, int R,
-                                 const int* __restrict__ mask, int nf) {
-  __shared__ double t[32][33];
-  const int d0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
-  for (int dd = threadIdx.y; dd < 32; dd += blockDim.y) {
-    const int d = d0 + dd, k = k0 + threadIdx.x;
-    const size_t o = (size_t)d * R + k;
-    t[dd][threadIdx.x] = (d < n && k < R) ? f2d_exact(x32[o]) + f2d_exact(d32[o]) : 0.0;
-  }
-  __syncthreads();
-  for (int kk = threadIdx.y; kk < 32; kk += blockDim.y) {
-    const int k = k0 + kk, d = d0 + threadIdx.x;
-    if (k < R && d < n && (!mask || mask[k / nf])) dst[k][d] = t[threadIdx.x][kk];
-  }
-}
-
-// dst[d * R + k] = src[k][d] as an FP32 pair (the previous step's solution,
+// Xs[d * R + k] = old_k[d] as an FP32 pair (the previous step's solution,
 // interleaved for the residual of an increment solve)
-__global__ void k_gather_pairs_il(const double* const* __restrict__ src, float2* __restrict__ dst, int n, int R) {
+__global__ void k_gather_pairs_il(ElemSets E) {
+  const ElemSet& S = E.s[blockIdx.z];
   __shared__ double t[32][33];
-  const int d0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+  const int n = S.n, R = S.R, d0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+  if (d0 >= n || k0 >= R) return;
   for (int kk = threadIdx.y; kk < 32; kk += blockDim.y) {
     const int k = k0 + kk, d = d0 + threadIdx.x;
-    t[kk][threadIdx.x] = (k < R && d < n) ? src[k][d] : 0.0;
+    t[kk][threadIdx.x] = (k < R && d < n) ? S.old[k][d] : 0.0;
   }
   __syncthreads();
   for (int dd = threadIdx.y; dd < 32; dd += blockDim.y) {
     const int d = d0 + dd, k = k0 + threadIdx.x;
-    if (d < n && k < R) dst[(size_t)d * R + k] = d2ff(t[threadIdx.x][dd]);
+    if (d < n && k < R) S.Xs[(size_t)d * R + k] = d2ff(t[threadIdx.x][dd]);
   }
 }
 
-// dst_k[d] = old_k[d] + (double) d32[d * R + k]: the previous step's solution
-// plus the increment an increment solve found
-__global__ void k_scatter_delta_il(const float* __restrict__ d32, const double* const* __restrict__ old,
-                                   double* const* __restrict__ dst, int n, int R, const int* __restrict__ mask,
-                                   int nf) {
+// dst_k[d] = old_k[d] + D32[d * R + k]: the previous step's solution plus the
+// increment an increment solve found
+__global__ void k_scatter_delta_il(ElemSets E, const int* __restrict__ mask, int n_inst) {
+  const ElemSet& S = E.s[blockIdx.z];
   __shared__ float t[32][33];
-  const int d0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+  const int n = S.n, R = S.R, d0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+  if (d0 >= n || k0 >= R) return;
+  const int nf = R / n_inst;
   for (int dd = threadIdx.y; dd < 32; dd += blockDim.y) {
     const int d = d0 + dd, k = k0 + threadIdx.x;
-    t[dd][threadIdx.x] = (d < n && k < R) ? d32[(size_t)d * R + k] : 0.f;
+    t[dd][threadIdx.x] = (d < n && k < R) ? S.D32[(size_t)d * R + k] : 0.f;
   }
   __syncthreads();
   for (int kk = threadIdx.y; kk < 32; kk += blockDim.y) {
@@ -174,24 +200,24 @@ __global__ void k_scatter_delta_il(const float* __restrict__ d32, const double* 
     // FP32-pair sum converted with integer operations (FP64 additions are
     // the scarce resource on GB300): the state keeps ~47 bits of the update
     if (k < R && d < n && (!mask || mask[k / nf]))
-      dst[k][d] = ff2d_i32(ff_add(d2ff(old[k][d]), t[threadIdx.x][kk]));
+      S.dst[k][d] = ff2d_i32(ff_add(d2ff(S.old[k][d]), t[threadIdx.x][kk]));
   }
 }
 
-// x = (double) x32 + (double) d32
-__global__ void k_sum_il(const float* __restrict__ x32, const float* __restrict__ d32,
-                         double* __restrict__ x, size_t n) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i < n) x[i] = (double)x32[i] + (double)d32[i];
+// r = b - A x for R right-hand sides sharing A, a thread per (row, right-hand
+// side), right-hand sides fastest: matrix entries are broadcast within a row's
+// threads, vectors read and written contiguously, and every lane works whatever R
+// (a warp per row left 30 of 32 lanes idle at R = 2).  (row, k) of this thread:
+struct RowRhs {
+  int row, k;
+};
+__device__ __forceinline__ RowRhs row_rhs(int R) {
+  const unsigned long long e0 = (unsigned long long)blockIdx.x * blockDim.x;
+  const unsigned long long r0 = e0 / (unsigned)R;
+  const unsigned e = (unsigned)(e0 - r0 * (unsigned)R) + threadIdx.x, q = e / (unsigned)R;
+  return RowRhs{(int)(r0 + q), (int)(e - q * (unsigned)R)};
 }
 
-__global__ void k_widen_il(const float* __restrict__ x32, double* __restrict__ x, size_t n) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i < n) x[i] = (double)x32[i];
-}
-
-// r = b - A x for R right-hand sides sharing A: one warp per row, lanes over
-// right-hand sides (matrix entries broadcast, vectors read contiguously).
 // The sum runs in FP32-pair ("double-float") arithmetic: products are exact
 // through fmaf, partial sums through TwoSum, so the residual keeps ~46-bit
 // accuracy while running on the FP32 pipe.
@@ -199,6 +225,14 @@ __global__ void k_widen_il(const float* __restrict__ x32, double* __restrict__ x
 // refinement of an FP32 sweep's solution); RT the residual's storage type.
 __device__ __forceinline__ float2 as_pair(float2 v) { return v; }
 __device__ __forceinline__ float2 as_pair(float v) { return make_float2(v, 0.f); }
+template <typename X>
+__device__ __forceinline__ const X* pair_x(const ElemSet& S) {
+  if constexpr (sizeof(X) == 8) return S.Xs; else return S.X32;
+}
+template <typename RT>
+__device__ __forceinline__ RT* residual_of(const ElemSet& S) {
+  if constexpr (sizeof(RT) == 8) return S.Rr; else return S.Rr32;
+}
 
 // b - (sh + sl): for a float residual (the next sweep's input) entirely in
 // FP32 pairs, b split on the integer pipe; for a double residual in FP64
@@ -212,18 +246,20 @@ __device__ __forceinline__ RT df_residual(double b, float sh, float sl) {
   }
 }
 
-// b: interleaved right-hand sides, or (bt non-null) a table of per-RHS
-// vectors read in place (one 8-byte load per lane; saves the transposing
-// gather of an increment solve)
+// in_place: the right-hand sides are read from the per-instance vectors (one
+// 8-byte load per thread; saves the transposing gather of an increment solve)
 template <typename X, typename RT>
-__global__ void k_residual_df_il(CsrDf A, const double* __restrict__ b, const double* const* __restrict__ bt,
-                                 const X* __restrict__ xs, RT* __restrict__ r, int n, int R) {
-  const int row = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-  const int k = blockIdx.y * 32 + (threadIdx.x & 31);
-  if (row >= n || k >= R) return;
+__global__ void k_residual_df_il(ElemSets E, int in_place) {
+  const ElemSet& S = E.s[blockIdx.y];
+  const RowRhs p_ = row_rhs(S.R);
+  const int row = p_.row, k = p_.k, R = S.R;
+  if (row >= S.n) return;
+  const X* xs = pair_x<X>(S);
   float sh = 0.f, sl = 0.f;
-  for (int p = A.rp[row]; p < A.rp[row + 1]; ++p) {
-    const float2 a = A.v[p], xv = as_pair(xs[(size_t)A.ci[p] * R + k]);
+  const int p1 = S.Adf.rp[row + 1];
+#pragma unroll 4
+  for (int p = S.Adf.rp[row]; p < p1; ++p) {
+    const float2 a = S.Adf.v[p], xv = as_pair(xs[(size_t)S.Adf.ci[p] * R + k]);
     const float ph = a.x * xv.x;
     const float pe = fmaf(a.x, xv.x, -ph) + fmaf(a.x, xv.y, a.y * xv.x);
     const float t = sh + ph;
@@ -233,7 +269,7 @@ __global__ void k_residual_df_il(CsrDf A, const double* __restrict__ b, const do
     sl += e + pe;
   }
   const size_t o = (size_t)row * R + k;
-  r[o] = df_residual<RT>(bt ? bt[k][row] : b[o], sh, sl);
+  residual_of<RT>(S)[o] = df_residual<RT>(in_place ? S.src[k][row] : S.B[o], sh, sl);
 }
 
 // Four right-hand sides per lane (128 per warp, R a multiple of 4): the row's
@@ -262,17 +298,18 @@ __device__ __forceinline__ void st4(double* p, const double (&v)[4]) {
 }
 
 template <typename X, typename RT>
-__global__ void k_residual_df_il4(CsrDf A, const double* __restrict__ b, const double* const* __restrict__ bt,
-                                  const X* __restrict__ xs, RT* __restrict__ r, int n, int R) {
-  const int row = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+__global__ void k_residual_df_il4(ElemSets E, int in_place) {
+  const ElemSet& S = E.s[blockIdx.z];
+  const int row = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, R = S.R;
   const int k = blockIdx.y * 128 + (threadIdx.x & 31) * 4;
-  if (row >= n || k >= R) return;
+  if (row >= S.n || k >= R) return;
+  const X* xs = pair_x<X>(S);
   float sh[4] = {0.f, 0.f, 0.f, 0.f}, sl[4] = {0.f, 0.f, 0.f, 0.f};
-  const int p1 = A.rp[row + 1];
-  for (int p = A.rp[row]; p < p1; ++p) {
-    const float2 a = A.v[p];
+  const int p1 = S.Adf.rp[row + 1];
+  for (int p = S.Adf.rp[row]; p < p1; ++p) {
+    const float2 a = S.Adf.v[p];
     float2 xv[4];
-    ld_pairs4(xs + (size_t)A.ci[p] * R + k, xv);
+    ld_pairs4(xs + (size_t)S.Adf.ci[p] * R + k, xv);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const float ph = a.x * xv[q].x;
@@ -286,27 +323,32 @@ __global__ void k_residual_df_il4(CsrDf A, const double* __restrict__ b, const d
   }
   const size_t o = (size_t)row * R + k;
   double bb[4];
-  if (bt) {
+  if (in_place) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) bb[q] = bt[k + q][row];
+    for (int q = 0; q < 4; ++q) bb[q] = S.src[k + q][row];
   } else {
-    const double2 b0 = reinterpret_cast<const double2*>(b + o)[0], b1 = reinterpret_cast<const double2*>(b + o)[1];
+    const double2 b0 = reinterpret_cast<const double2*>(S.B + o)[0], b1 = reinterpret_cast<const double2*>(S.B + o)[1];
     bb[0] = b0.x, bb[1] = b0.y, bb[2] = b1.x, bb[3] = b1.y;
   }
   RT v[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) v[q] = df_residual<RT>(bb[q], sh[q], sl[q]);
-  st4(r + o, v);
+  st4(residual_of<RT>(S) + o, v);
 }
 
-template <typename X, typename RT>
-void launch_residual_df(const CsrDf& A, const double* b, const X* xs, RT* r, int n, int R, cudaStream_t s,
-                        const double* const* bt = nullptr) {
-  if (R % 4 == 0 && R >= 96)
-    k_residual_df_il4<X, RT><<<dim3((n + 7) / 8, (R + 127) / 128), 256, 0, s>>>(A, b, bt, xs, r, n, R);
-  else
-    k_residual_df_il<X, RT><<<dim3((n + 7) / 8, (R + 31) / 32), 256, 0, s>>>(A, b, bt, xs, r, n, R);
-  PECS_CUDA(cudaGetLastError());
+// FP64 variant (FP64 and FP32_IR modes)
+template <typename RT>
+__global__ void k_residual_il(ElemSets E) {
+  const ElemSet& S = E.s[blockIdx.y];
+  const RowRhs p_ = row_rhs(S.R);
+  const int row = p_.row, k = p_.k, R = S.R;
+  if (row >= S.n) return;
+  double acc = 0.0;
+  const int p1 = S.A.rp[row + 1];
+#pragma unroll 4
+  for (int p = S.A.rp[row]; p < p1; ++p) acc += S.A.v[p] * S.X[(size_t)S.A.ci[p] * R + k];
+  const size_t o = (size_t)row * R + k;
+  residual_of<RT>(S)[o] = (RT)(S.B[o] - acc);
 }
 
 // ||b - A x||^2 and ||b||^2 of one instance-major vector pair (grid.y =
@@ -334,19 +376,6 @@ __global__ void k_residual_norms(CsrDev A, const double* __restrict__ b, const d
   }
 }
 
-// FP64 variant (FP32_IR mode)
-template <typename RT>
-__global__ void k_residual_il(CsrDev A, const double* __restrict__ b, const double* __restrict__ x,
-                              RT* __restrict__ r, int n, int R) {
-  const int row = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-  const int k = blockIdx.y * 32 + (threadIdx.x & 31);
-  if (row >= n || k >= R) return;
-  double acc = 0.0;
-  for (int p = A.rp[row]; p < A.rp[row + 1]; ++p) acc += A.v[p] * x[(size_t)A.ci[p] * R + k];
-  const size_t o = (size_t)row * R + k;
-  r[o] = (RT)(b[o] - acc);
-}
-
 constexpr int kRedThreads = 256;
 constexpr int kRedChunks = 16;
 
@@ -366,18 +395,28 @@ __global__ void k_relchange_partial(FieldPtrs NEW, FieldPtrs OLD, int n_fields,
     const double* b = OLD.u[f] + (size_t)i * nd;
     const int per = (nd + kRedChunks - 1) / kRedChunks;
     const int lo = chunk * per, hi = min(nd, lo + per);
-    for (int t = lo + threadIdx.x; t < hi; t += blockDim.x) {
-      const double x = a[t], y = b[t];
-      Acc d, xa;
-      if constexpr (sizeof(Acc) == 4) {
-        d = d2f_trunc(x - y);  // the one FP64 operation per element
-        xa = d2f_trunc(x);
-      } else {
-        d = x - y;
-        xa = x;
+    constexpr int U = 8;  // elements in flight per thread
+    for (int t0 = lo + threadIdx.x; t0 < hi; t0 += U * kRedThreads) {
+      double x[U], y[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int t = t0 + u * kRedThreads;
+        x[u] = t < hi ? a[t] : 0.0;
+        y[u] = t < hi ? b[t] : 0.0;
       }
-      d2 += d * d;
-      n2 += xa * xa;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        Acc d, xa;
+        if constexpr (sizeof(Acc) == 4) {
+          d = d2f_trunc(x[u] - y[u]);  // the one FP64 operation per element
+          xa = d2f_trunc(x[u]);
+        } else {
+          d = x[u] - y[u];
+          xa = x[u];
+        }
+        d2 += d * d;
+        n2 += xa * xa;
+      }
     }
   }
   sd[threadIdx.x] = (double)d2;
@@ -404,39 +443,45 @@ __global__ void k_converge(const double2* __restrict__ partial, int n_inst, int 
                            int* __restrict__ step_ctr, int* __restrict__ active,
                            int* __restrict__ n_active, const int* __restrict__ start, int max_steps,
                            int* __restrict__ capped) {
+  // a warp per instance; 16 lanes add one field's chunks (a serial walk over
+  // them took 17 us of every step, whatever the instances' number)
+  static_assert(kRedChunks == 16, "half a warp adds the chunks of a field");
   const int step = *step_ctr + 1;
   __shared__ int cnt;
   if (threadIdx.x == 0) cnt = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < n_inst; i += blockDim.x) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = warp; i < n_inst; i += blockDim.x >> 5) {
     double r = 0.0;
     bool finite = true;
-    for (int fld = 0; fld < n_fields; ++fld) {
-      double d2 = 0.0, n2 = 0.0;
-      for (int c = 0; c < kRedChunks; ++c) {
-        const double2 v = partial[((size_t)i * 5 + fld) * kRedChunks + c];
-        d2 += v.x;
-        n2 += v.y;
+    for (int f0 = 0; f0 < n_fields; f0 += 2) {
+      const int fld = f0 + (lane >> 4);
+      double2 v = make_double2(0.0, 0.0);
+      if (fld < n_fields) v = partial[((size_t)i * 5 + fld) * kRedChunks + (lane & 15)];
+      for (int o = 8; o > 0; o >>= 1) {
+        v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+        v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
       }
-      finite = finite && isfinite(d2) && isfinite(n2);
-      const double q = n2 > 0.0 ? sqrt(d2 / n2) : sqrt(d2);
-      r = fmax(r, q);
+      finite = finite && isfinite(v.x) && isfinite(v.y);
+      if (fld < n_fields) r = fmax(r, v.y > 0.0 ? sqrt(v.x / v.y) : sqrt(v.x));
     }
-    if (active[i]) {
-      rel[i] = finite ? r : __longlong_as_double(0x7ff8000000000000LL);
-      if (!finite) {
-        active[i] = 0;
-        conv_step[i] = -step;  // non-finite state: stopped, reported as failure
-      } else if (r <= tol) {
-        active[i] = 0;
-        conv_step[i] = step;
-      } else if (step - start[i] >= max_steps) {
-        active[i] = 0;
-        conv_step[i] = step;
-        capped[i] = 1;
-      }
+    r = fmax(r, __shfl_xor_sync(0xffffffffu, r, 16));
+    finite = __all_sync(0xffffffffu, finite);
+    if (lane != 0 || !active[i]) continue;
+    rel[i] = finite ? r : __longlong_as_double(0x7ff8000000000000LL);
+    if (!finite) {
+      active[i] = 0;
+      conv_step[i] = -step;  // non-finite state: stopped, reported as failure
+    } else if (r <= tol) {
+      active[i] = 0;
+      conv_step[i] = step;
+    } else if (step - start[i] >= max_steps) {
+      active[i] = 0;
+      conv_step[i] = step;
+      capped[i] = 1;
+    } else {
+      atomicAdd(&cnt, 1);
     }
-    if (active[i]) atomicAdd(&cnt, 1);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -591,32 +636,30 @@ struct Engine {
     if (opt.ir_max_iters > 0) return opt.ir_max_iters;
     return opt.precision == PECS_PREC_FP32_IR ? 2 : 1;
   }
-  // element-wise launches per set of one solve: gather, scatter and, per
-  // refinement sweep, the residual and its helpers (split / widen, axpy / sum)
-  int set_launches_per_solve(int which) const {
+  // element-wise launches of one solve: gather, scatter and, per refinement
+  // sweep, the residual and its helpers (split, widen, and the updates between
+  // refinements)
+  int elem_launches_per_solve(int which) const {
     const int iters = ir_iters(which);
-    const bool mixed = opt.precision == PECS_PREC_FP32_MIXED;
-    int n = 2;
+    const bool mixed = opt.precision == PECS_PREC_FP32_MIXED, f32 = il_f32(which);
+    int n = 2 + iters;
     for (int it = 0; it < iters; ++it) {
-      if (il_f32(which))
-        n += mixed ? (it == 0 ? (iters == 1 ? 1 : 2) : 3) : (it == 0 ? 3 : 2);
-      else
-        n += mixed ? 3 : 2;
+      if (mixed ? !(f32 && it == 0) : (f32 && it == 0)) ++n;  // split / widen
+      if (it + 1 < iters) ++n;                                // update
     }
     return n;
   }
   // Poisson RHS + Poisson solve
   int initialize_launches() const {
-    return 1 + bank_p.kernel_launches_per_solve() * (1 + ir_iters(1)) + il[1].n_sets * set_launches_per_solve(1);
+    return 1 + bank_p.kernel_launches_per_solve() * (1 + ir_iters(1)) + elem_launches_per_solve(1);
   }
   int launches_per_step() const {
     const int lc = bank_c.kernel_launches_per_solve(), lp = bank_p.kernel_launches_per_solve();
-    const int sc = il[0].n_sets, sp = il[1].n_sets;
     // increment solves: gather of the previous solution, residual and
-    // scatter per set, one sweep
+    // scatter, one sweep
     const bool dc = delta_solves() && il_f32(0), dp = delta_solves() && il_f32(1);
-    return 1 + (dc ? lc + 3 * sc : lc * (1 + ir_iters(0)) + sc * set_launches_per_solve(0)) + 1 +
-           (dp ? lp + 3 * sp : lp * (1 + ir_iters(1)) + sp * set_launches_per_solve(1)) + 3;
+    return 1 + (dc ? lc + 3 : lc * (1 + ir_iters(0)) + elem_launches_per_solve(0)) + 1 +
+           (dp ? lp + 3 : lp * (1 + ir_iters(1)) + elem_launches_per_solve(1)) + 3;
   }
   // algorithmic bytes of one application of a bank to all of its right-hand
   // sides: every stored factor entry once, plus the vectors (b read, y write +
@@ -756,26 +799,61 @@ struct Engine {
   bool delta_solves() const {
     return opt.increment_solves > 0 && opt.precision == PECS_PREC_FP32_MIXED;
   }
+  ElemSets elem_sets(int which, int target) const {
+    ElemSets E;
+    const IlBank& I = il[which];
+    for (int si = 0; si < I.n_sets; ++si) {
+      const IlSet& S_ = I.set[si];
+      ElemSet& e = E.s[si];
+      e.n = S_.n, e.R = S_.R;
+      e.src = S_.src.p, e.old = S_.dst[1 - target].p, e.dst = S_.dst[target].p;
+      e.B = S_.B.p, e.X = S_.X.p, e.D = S_.D.p, e.Rr = S_.Rr.p;
+      e.B32 = S_.f32 ? S_.B32.p : nullptr;
+      e.X32 = S_.X32.p, e.D32 = S_.D32.p, e.Rr32 = S_.Rr32.p, e.Xs = S_.Xs.p;
+      e.A = csr.m[S_.mat];
+      e.Adf = csr_df.m[S_.mat];
+    }
+    return E;
+  }
+  // grids over all sets of a bank: 32 x 32 tiles, or a thread per element
+  dim3 tile_grid(int which) const {
+    const IlBank& I = il[which];
+    int n = 0;
+    for (int si = 0; si < I.n_sets; ++si) n = std::max(n, I.set[si].n);
+    return dim3((n + 31) / 32, (I.max_R + 31) / 32, I.n_sets);
+  }
+  dim3 elem_grid(int which) const {
+    const IlBank& I = il[which];
+    size_t m = 0;
+    for (int si = 0; si < I.n_sets; ++si) m = std::max(m, (size_t)I.set[si].n * I.set[si].R);
+    return dim3((unsigned)((m + 255) / 256), I.n_sets);
+  }
+  template <typename X, typename RT>
+  void launch_residual_df(int which, const ElemSets& E, bool in_place, cudaStream_t s) const {
+    const IlBank& I = il[which];
+    bool four = true;
+    int n = 0;
+    for (int si = 0; si < I.n_sets; ++si) {
+      four = four && I.set[si].R % 4 == 0 && I.set[si].R >= 96;
+      n = std::max(n, I.set[si].n);
+    }
+    if (four)
+      k_residual_df_il4<X, RT><<<dim3((n + 7) / 8, (I.max_R + 127) / 128, I.n_sets), 256, 0, s>>>(E, in_place);
+    else
+      k_residual_df_il<X, RT><<<elem_grid(which), 256, 0, s>>>(E, in_place);
+    PECS_CUDA(cudaGetLastError());
+  }
+
   void solve_bank_delta(const FactorBank& bank, int which, int target, cudaStream_t s) {
-    IlBank& I = il[which];
-    const dim3 tb(32, 8);
-    for (int si = 0; si < I.n_sets; ++si) {
-      IlSet& S_ = I.set[si];
-      const dim3 g((S_.n + 31) / 32, (S_.R + 31) / 32);
-      k_gather_pairs_il<<<g, tb, 0, s>>>(S_.dst[1 - target].p, S_.Xs.p, S_.n, S_.R);
-      PECS_CUDA(cudaGetLastError());
-      // the right-hand sides are read in place from the per-instance vectors
-      launch_residual_df(csr_df.m[S_.mat], (const double*)nullptr, S_.Xs.p, S_.Rr32.p, S_.n, S_.R, s,
-                         (const double* const*)S_.src.p);
-    }
+    const ElemSets E = elem_sets(which, target);
+    const dim3 tb(32, 8), tg = tile_grid(which);
+    k_gather_pairs_il<<<tg, tb, 0, s>>>(E);
+    PECS_CUDA(cudaGetLastError());
+    // the right-hand sides are read in place from the per-instance vectors
+    launch_residual_df<float2, float>(which, E, true, s);
     bank_sweep(bank, which, true, s);
-    for (int si = 0; si < I.n_sets; ++si) {
-      IlSet& S_ = I.set[si];
-      const dim3 g((S_.n + 31) / 32, (S_.R + 31) / 32);
-      k_scatter_delta_il<<<g, tb, 0, s>>>(S_.D32.p, S_.dst[1 - target].p, S_.dst[target].p, S_.n, S_.R,
-                                          scatter_mask, S_.R / n_inst);
-      PECS_CUDA(cudaGetLastError());
-    }
+    k_scatter_delta_il<<<tg, tb, 0, s>>>(E, scatter_mask, n_inst);
+    PECS_CUDA(cudaGetLastError());
   }
 
   void solve_bank_il(const FactorBank& bank, int which, int target, cudaStream_t s, bool delta = false) {
@@ -783,76 +861,59 @@ struct Engine {
       solve_bank_delta(bank, which, target, s);
       return;
     }
-    IlBank& I = il[which];
-    const dim3 tb(32, 8);
+    const ElemSets E = elem_sets(which, target);
+    const dim3 tb(32, 8), tg = tile_grid(which), eg = elem_grid(which);
     const bool f32 = il_f32(which);
     const bool mixed = opt.precision == PECS_PREC_FP32_MIXED;
-    for (int si = 0; si < I.n_sets; ++si) {
-      IlSet& S_ = I.set[si];
-      k_gather_il<<<dim3((S_.n + 31) / 32, (S_.R + 31) / 32), tb, 0, s>>>(
-          S_.src.p, S_.B.p, f32 ? S_.B32.p : nullptr, S_.n, S_.R);
-      PECS_CUDA(cudaGetLastError());
-    }
+    k_gather_il<<<tg, tb, 0, s>>>(E);
+    PECS_CUDA(cudaGetLastError());
     bank_sweep(bank, which, false, s);
     const int iters = ir_iters(which);
-    auto egrid = [](size_t nR) { return (unsigned)((nR + 255) / 256); };
     for (int it = 0; it < iters; ++it) {
-      for (int si = 0; si < I.n_sets; ++si) {
-        IlSet& S_ = I.set[si];
-        const size_t nR = (size_t)S_.n * S_.R;
-        const dim3 rg((S_.n + 7) / 8, (S_.R + 31) / 32);
-        if (f32) {
-          // FP32 sweep vectors: the residual is stored in float for the next sweep
-          if (mixed && it == 0) {
-            launch_residual_df(csr_df.m[S_.mat], S_.B.p, S_.X32.p, S_.Rr32.p, S_.n, S_.R, s);
-          } else if (mixed) {
-            k_split_il<<<egrid(nR), 256, 0, s>>>(S_.X.p, S_.Xs.p, nR);
-            PECS_CUDA(cudaGetLastError());
-            launch_residual_df(csr_df.m[S_.mat], S_.B.p, S_.Xs.p, S_.Rr32.p, S_.n, S_.R, s);
-          } else {
-            if (it == 0) {
-              k_widen_il<<<egrid(nR), 256, 0, s>>>(S_.X32.p, S_.X.p, nR);
-              PECS_CUDA(cudaGetLastError());
-            }
-            k_residual_il<float><<<rg, 256, 0, s>>>(csr.m[S_.mat], S_.B.p, S_.X.p, S_.Rr32.p, S_.n, S_.R);
-          }
+      if (f32) {
+        // FP32 sweep vectors: the residual is stored in float for the next sweep
+        if (mixed && it == 0) {
+          launch_residual_df<float, float>(which, E, false, s);
         } else if (mixed) {
-          k_split_il<<<egrid(nR), 256, 0, s>>>(S_.X.p, S_.Xs.p, nR);
+          k_split_il<<<eg, 256, 0, s>>>(E);
           PECS_CUDA(cudaGetLastError());
-          launch_residual_df(csr_df.m[S_.mat], S_.B.p, S_.Xs.p, S_.Rr.p, S_.n, S_.R, s);
+          launch_residual_df<float2, float>(which, E, false, s);
         } else {
-          k_residual_il<double><<<rg, 256, 0, s>>>(csr.m[S_.mat], S_.B.p, S_.X.p, S_.Rr.p, S_.n, S_.R);
+          if (it == 0) {
+            k_update_il<Upd::Widen><<<eg, 256, 0, s>>>(E);
+            PECS_CUDA(cudaGetLastError());
+          }
+          k_residual_il<float><<<eg, 256, 0, s>>>(E);
         }
+      } else if (mixed) {
+        k_split_il<<<eg, 256, 0, s>>>(E);
         PECS_CUDA(cudaGetLastError());
+        launch_residual_df<float2, double>(which, E, false, s);
+      } else {
+        k_residual_il<double><<<eg, 256, 0, s>>>(E);
       }
+      PECS_CUDA(cudaGetLastError());
       bank_sweep(bank, which, true, s);
-      for (int si = 0; si < I.n_sets; ++si) {
-        IlSet& S_ = I.set[si];
-        const size_t nR = (size_t)S_.n * S_.R;
-        if (f32 && mixed && it == 0 && iters == 1)
-          continue;  // the scatter adds the correction
-        if (f32 && mixed && it == 0)
-          k_sum_il<<<egrid(nR), 256, 0, s>>>(S_.X32.p, S_.D32.p, S_.X.p, nR);
-        else if (f32)
-          k_axpy_il<float><<<egrid(nR), 256, 0, s>>>(S_.X.p, S_.D32.p, nR);
-        else
-          k_axpy_il<double><<<egrid(nR), 256, 0, s>>>(S_.X.p, S_.D.p, nR);
-        PECS_CUDA(cudaGetLastError());
-      }
-    }
-    for (int si = 0; si < I.n_sets; ++si) {
-      IlSet& S_ = I.set[si];
-      const dim3 sg((S_.n + 31) / 32, (S_.R + 31) / 32);
-      const int nf = S_.R / n_inst;  // columns per instance
-      if (f32 && iters == 0)
-        k_scatter_il<float><<<sg, tb, 0, s>>>(S_.X32.p, S_.dst[target].p, S_.n, S_.R, scatter_mask, nf);
-      else if (f32 && mixed && iters == 1)
-        k_scatter_sum_il<<<sg, tb, 0, s>>>(S_.X32.p, S_.D32.p, S_.dst[target].p, S_.n, S_.R, scatter_mask,
-                                           nf);
+      if (it + 1 == iters) break;  // the scatter adds the last correction
+      if (f32 && mixed && it == 0)
+        k_update_il<Upd::Sum32><<<eg, 256, 0, s>>>(E);
+      else if (f32)
+        k_update_il<Upd::AddD32><<<eg, 256, 0, s>>>(E);
       else
-        k_scatter_il<double><<<sg, tb, 0, s>>>(S_.X.p, S_.dst[target].p, S_.n, S_.R, scatter_mask, nf);
+        k_update_il<Upd::AddD><<<eg, 256, 0, s>>>(E);
       PECS_CUDA(cudaGetLastError());
     }
+    if (f32 && iters == 0)
+      k_scatter_il<Out::X32><<<tg, tb, 0, s>>>(E, scatter_mask, n_inst);
+    else if (f32 && mixed && iters == 1)
+      k_scatter_il<Out::X32PlusD32><<<tg, tb, 0, s>>>(E, scatter_mask, n_inst);
+    else if (f32)
+      k_scatter_il<Out::XPlusD32><<<tg, tb, 0, s>>>(E, scatter_mask, n_inst);
+    else if (iters == 0)
+      k_scatter_il<Out::X><<<tg, tb, 0, s>>>(E, scatter_mask, n_inst);
+    else
+      k_scatter_il<Out::XPlusD><<<tg, tb, 0, s>>>(E, scatter_mask, n_inst);
+    PECS_CUDA(cudaGetLastError());
   }
 
   std::vector<std::vector<int>> carrier_set_fields() const {
@@ -1325,10 +1386,10 @@ struct Engine {
       k_relchange_partial<double><<<dim3(kRedChunks, 5, n_inst), kRedThreads, 0, s>>>(NEW, OLD, n_fields,
                                                                                      partial.p);
     PECS_CUDA(cudaGetLastError());
-    k_converge<<<1, 256, 0, s>>>(partial.p, n_inst, n_fields, tol, conv_step.p, rel.p, step_ctr.p,
+    k_converge<<<1, 1024, 0, s>>>(partial.p, n_inst, n_fields, tol, conv_step.p, rel.p, step_ctr.p,
                                  active.p, n_active.p, start_step.p, step_cap, capped.p);
     PECS_CUDA(cudaGetLastError());
-    k_snapshot<<<dim3(32, 5, n_inst), 256, 0, s>>>(NEW, snap_ptrs.p, conv_step.p, step_ctr.p, 5);
+    k_snapshot<<<dim3(8, 5, n_inst), 256, 0, s>>>(NEW, snap_ptrs.p, conv_step.p, step_ctr.p, 5);
     PECS_CUDA(cudaGetLastError());
   }
 
