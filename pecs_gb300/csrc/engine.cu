@@ -573,12 +573,7 @@ struct Engine {
   DBuf<double> A_v[5];
   CsrSet csr{};
   // tables and regions
-  DBuf<double> t_phi, t_qw, t_fphi, t_fw, t_psix, t_psiy, t_phiP, t_mref;
-  DBuf<float> tf_phi, tf_qw, tf_fphi, tf_fw, tf_psix, tf_psiy;
-  DBuf<double> t_drift_x, t_drift_y;
-  DBuf<float2> t_drift_x_ff, t_drift_y_ff, t_mref_ff;
-  DBuf<int> t_drift_cx, t_drift_cy;
-  DBuf<double> t_charge;
+  DBuf<double> t_fphi, t_fw, t_charge;
   Tables T{};
   DBuf<double2> h_[2], ph_[2];
   DBuf<int4> bid_[2];
@@ -1145,79 +1140,84 @@ struct Engine {
   void upload_tables() {
     const CarrierTables& ct = S->ct;
     const PoissonTables& pt = S->pt;
-    t_phi.upload(ct.phi);
-    t_qw.upload(ct.qw);
     t_fphi.upload(ct.fphi);
     t_fw.upload(ct.fw);
-    t_psix.upload(pt.psi_x);
-    t_psiy.upload(pt.psi_y);
-    t_phiP.upload(pt.phi);
-    std::vector<double> mref(ct.n1 * ct.n1, 0.0);
-    for (int a = 0; a < ct.n1; ++a)
-      for (int b = 0; b < ct.n1; ++b)
-        for (int q = 0; q < ct.Q; ++q) mref[a * ct.n1 + b] += ct.phi[a * ct.Q + q] * ct.phi[b * ct.Q + q] * ct.qw[q];
-    t_mref.upload(mref);
-    auto f32 = [](const std::vector<double>& v) { return std::vector<float>(v.begin(), v.end()); };
-    tf_phi.upload(f32(ct.phi));
-    tf_qw.upload(f32(ct.qw));
-    tf_fphi.upload(f32(ct.fphi));
-    tf_fw.upload(f32(ct.fw));
-    tf_psix.upload(f32(pt.psi_x));
-    tf_psiy.upload(f32(pt.psi_y));
-    // drift tensors sum_q phi_a phi_b psi_c w_q over the RT functions with a
-    // non-zero x (y) component; on rectangles each RT function has one
-    // component only, nrt/2 of each
-    const int n1 = ct.n1, Q = ct.Q, nrt = pt.n_rt, NC = nrt / 2;
-    std::vector<int> cx, cy;
-    for (int c = 0; c < nrt; ++c) {
-      bool nx = false, ny = false;
-      for (int q = 0; q < Q; ++q) {
-        nx = nx || pt.psi_x[c * Q + q] != 0.0;
-        ny = ny || pt.psi_y[c * Q + q] != 0.0;
-      }
-      if (nx && ny) throw PecsError(PECS_E_STATE, "RT function with two components");
-      if (nx) cx.push_back(c);
-      if (ny) cy.push_back(c);
-    }
-    if ((int)cx.size() != NC || (int)cy.size() != NC)
-      throw PecsError(PECS_E_STATE, "RT functions not split evenly by component");
-    std::vector<double> dx((size_t)n1 * n1 * NC, 0.0), dy((size_t)n1 * n1 * NC, 0.0);
-    for (int a = 0; a < n1; ++a)
-      for (int b = 0; b < n1; ++b)
-        for (int j = 0; j < NC; ++j)
-          for (int q = 0; q < Q; ++q) {
-            const double pw = ct.phi[a * Q + q] * ct.phi[b * Q + q] * ct.qw[q];
-            dx[((size_t)a * n1 + b) * NC + j] += pw * pt.psi_x[cx[j] * Q + q];
-            dy[((size_t)a * n1 + b) * NC + j] += pw * pt.psi_y[cy[j] * Q + q];
-          }
-    t_drift_x.upload(dx);
-    t_drift_y.upload(dy);
-    t_drift_cx.upload(cx);
-    t_drift_cy.upload(cy);
     // Poisson charge matrix sum_q phiP_a phi_b w_q
-    const int nphi = pt.n_phi;
+    const int nphi = pt.n_phi, n1 = ct.n1, Q = ct.Q;
     std::vector<double> chg((size_t)nphi * n1, 0.0);
     for (int a = 0; a < nphi; ++a)
       for (int b = 0; b < n1; ++b)
         for (int q = 0; q < Q; ++q) chg[(size_t)a * n1 + b] += pt.phi[a * Q + q] * ct.phi[b * Q + q] * ct.qw[q];
     t_charge.upload(chg);
-    // FP32 pairs (hi rounded to nearest, lo the rounded remainder) for the
-    // mixed path
-    auto ff = [](const std::vector<double>& v) {
-      std::vector<float2> o(v.size());
-      for (size_t k = 0; k < v.size(); ++k) {
-        const float hi = (float)v[k];
-        o[k] = make_float2(hi, (float)(v[k] - (double)hi));
-      }
-      return o;
+    T = Tables{t_fphi.p, t_fw.p, t_charge.p};
+    with_element([&](auto kk, auto kp, auto tq) {
+      const auto t = tab_1d<decltype(kk)::value, decltype(kp)::value, decltype(tq)>();
+      tab_.resize(sizeof(t));
+      std::memcpy(tab_.data(), &t, sizeof(t));
+    });
+  }
+  std::vector<unsigned char> tab_;  // the Tab1D of this element and precision
+
+  // calls f(LDG degree, Poisson table degree, quadrature type): the reference's
+  // RT_{k-1} x DGQ_{k-1} pairing has KP = k, the configurations' RT_k x DGQ_k KP = k + 1
+  template <typename Fn>
+  void with_element(Fn f) const {
+    using I1 = std::integral_constant<int, 1>;
+    using I2 = std::integral_constant<int, 2>;
+    using I3 = std::integral_constant<int, 3>;
+    const int kp = S->pt.k;
+    auto go = [&](auto kk, auto kp_) {
+      opt.precision == PECS_PREC_FP32_MIXED ? f(kk, kp_, float()) : f(kk, kp_, double());
     };
-    t_drift_x_ff.upload(ff(dx));
-    t_drift_y_ff.upload(ff(dy));
-    t_mref_ff.upload(ff(mref));
-    T = Tables{t_phi.p,  t_qw.p,  t_fphi.p,  t_fw.p,   t_psix.p,  t_psiy.p, t_phiP.p,
-               t_mref.p, tf_phi.p, tf_qw.p, tf_fphi.p, tf_fw.p, tf_psix.p, tf_psiy.p,
-               t_drift_x.p, t_drift_y.p, t_drift_cx.p, t_drift_cy.p, t_charge.p,
-               t_drift_x_ff.p, t_drift_y_ff.p, t_mref_ff.p};
+    if (S->k == 1)
+      kp == 1 ? go(I1{}, I1{}) : go(I1{}, I2{});
+    else
+      kp == 2 ? go(I2{}, I2{}) : go(I2{}, I3{});
+  }
+
+  // the carrier element's one-dimensional tables (rhs_kernels.cuh); pairs: high part
+  // rounded to nearest, low part the rounded remainder
+  template <int K, int KP, typename Tq>
+  auto tab_1d() const {
+    using V = typename std::conditional<sizeof(Tq) == 4, float2, double>::type;
+    using Tab = Tab1D<K, KP, V, Tq>;
+    auto put = [](double x, V& v) {
+      if constexpr (sizeof(Tq) == 4) {
+        const float hi = (float)x;
+        v = make_float2(hi, (float)(x - (double)hi));
+      } else {
+        v = x;
+      }
+    };
+    const CarrierTables& ct = S->ct;
+    std::vector<double> nn(KP + 1), tn(KP);
+    for (int i = 0; i <= KP; ++i) nn[i] = double(i) / KP;
+    for (int i = 0; i < KP; ++i) tn[i] = (i + 0.5) / KP;
+    double mass[Tab::m][Tab::m] = {}, X[Tab::m][Tab::m][KP + 1] = {}, Y[Tab::m][Tab::m][KP] = {};
+    Tab t{};
+    for (int q = 0; q < Tab::nq; ++q) {
+      std::vector<double> l, xi, eta, der;
+      lagrange1d(dgq_nodes(K), ct.fq[q], l, der);
+      lagrange1d(nn, ct.fq[q], xi, der);
+      lagrange1d(tn, ct.fq[q], eta, der);
+      t.w[q] = (Tq)ct.fw[q];
+      for (int a = 0; a < Tab::m; ++a) {
+        t.L[q][a] = (Tq)l[a];
+        for (int b = 0; b < Tab::m; ++b) {
+          const double ab = l[a] * l[b] * ct.fw[q];
+          mass[a][b] += ab;
+          for (int j = 0; j <= KP; ++j) X[a][b][j] += ab * xi[j];
+          for (int j = 0; j < KP; ++j) Y[a][b][j] += ab * eta[j];
+        }
+      }
+    }
+    for (int a = 0; a < Tab::m; ++a)
+      for (int b = 0; b < Tab::m; ++b) {
+        put(mass[a][b], t.mass[a][b]);
+        for (int j = 0; j <= KP; ++j) put(X[a][b][j], t.X[a][b][j]);
+        for (int j = 0; j < KP; ++j) put(Y[a][b][j], t.Y[a][b][j]);
+      }
+    return t;
   }
 
   void upload_regions() {
@@ -1302,27 +1302,15 @@ struct Engine {
     const int nif = (int)S->iface_semi.size();
     const double* sne = S->has_schottky ? sch_ne.p : nullptr;
     const double* spe = S->has_schottky ? sch_pe.p : nullptr;
-    const bool mixed = opt.precision == PECS_PREC_FP32_MIXED;
     const int nreg = full ? 2 : 1;
-    // (LDG degree, Poisson table degree): the reference's RT_{k-1} x DGQ_{k-1}
-    // pairing has KP = k, the configurations' RT_k x DGQ_k KP = k + 1
-    auto go = [&](auto kk, auto kp) {
+    with_element([&](auto kk, auto kp, auto tq) {
       constexpr int K = decltype(kk)::value, KP = decltype(kp)::value;
-      if (mixed)
-        k_carrier_rhs<K, KP, float><<<grid, 128, 0, s>>>(T, R[0], R[1], nreg, F, inst.p, iface_ne.p,
-                                                         iface_pe.p, nif, sne, spe, act);
-      else
-        k_carrier_rhs<K, KP, double><<<grid, 128, 0, s>>>(T, R[0], R[1], nreg, F, inst.p, iface_ne.p,
-                                                          iface_pe.p, nif, sne, spe, act);
-    };
-    using I1 = std::integral_constant<int, 1>;
-    using I2 = std::integral_constant<int, 2>;
-    using I3 = std::integral_constant<int, 3>;
-    const int kp = S->pt.k;
-    if (S->k == 1)
-      kp == 1 ? go(I1{}, I1{}) : go(I1{}, I2{});
-    else
-      kp == 2 ? go(I2{}, I2{}) : go(I2{}, I3{});
+      using Tq = decltype(tq);
+      decltype(tab_1d<K, KP, Tq>()) t;
+      std::memcpy(&t, tab_.data(), sizeof(t));
+      k_carrier_rhs<K, KP, Tq><<<grid, 128, 0, s>>>(t, R[0], R[1], nreg, F, inst.p, iface_ne.p, iface_pe.p, nif, sne,
+                                                    spe, act);
+    });
     PECS_CUDA(cudaGetLastError());
   }
 

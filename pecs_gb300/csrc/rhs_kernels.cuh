@@ -23,26 +23,25 @@
 namespace pecs {
 
 struct Tables {
-  const double* phi;   // n1*Q   carrier basis at cell qp
-  const double* qw;    // Q
-  const double* fphi;  // 4*n1*nq face values
-  const double* fw;    // nq
-  const double* psix;  // nrt*Q  RT basis x-component at cell qp
-  const double* psiy;  // nrt*Q
-  const double* phiP;  // nphi*Q Poisson DGQ_{k-1} basis at cell qp
-  const double* mref;  // n1*n1  unit-square mass matrix
-  // FP32 copies for the mixed-precision path
-  const float *phi_f, *qw_f, *fphi_f, *fw_f, *psix_f, *psiy_f;
-  // drift tensors of the current equations, sum_q phi_a phi_b psi_c w_q on
-  // the unit square, over the RT basis functions with a non-zero x (y)
-  // component only -- nrt/2 of them on rectangles: [a][b][j], n1*n1*(nrt/2)
-  const double *drift_x, *drift_y;
-  const int *drift_cx, *drift_cy;  // their RT indices, nrt/2 each
-  // Poisson charge matrix sum_q phiP_a phi_b w_q on the unit square, nphi x n1
-  const double* charge;
-  // FP32-pair copies (hi, lo) of the drift tensors and the mass matrix for the
-  // mixed-precision path
-  const float2 *drift_x_ff, *drift_y_ff, *mref_ff;
+  const double* fphi;   // 4*n1*nq face values
+  const double* fw;     // nq
+  const double* charge; // Poisson charge matrix sum_q phiP_a phi_b w_q on the unit square, nphi x n1
+};
+
+// One-dimensional factors of the carrier element's tables, a kernel argument: the
+// products take them as constant-bank operands, without loads.  All cells are
+// axis-aligned rectangles and every basis is a tensor product (fe.hpp), so the
+// element integrals are products of these.
+// K: LDG degree; KP: the Poisson element is RT_{KP-1} x DGQ_{KP-1}.  V: double, or
+// float2 (FP32 pairs); Tq: the arithmetic type of the quadrature terms.
+template <int K, int KP, typename V, typename Tq>
+struct Tab1D {
+  static constexpr int m = K + 1, nq = K + 2;
+  Tq L[nq][m];      // Lagrange basis at the Gauss points
+  Tq w[nq];         // Gauss weights
+  V mass[m][m];     // int l_a l_b
+  V X[m][m][KP + 1];  // int l_a l_b xi_j, xi: the RT normal direction's basis
+  V Y[m][m][KP];      // int l_a l_b eta_j, eta: the tangential direction's
 };
 
 struct RegionDev {
@@ -99,34 +98,78 @@ __device__ __forceinline__ double from_q(Tq x) {
   if constexpr (sizeof(Tq) == 4) return f2d_exact(x); else return x;
 }
 
-template <typename Tq>
-__device__ __forceinline__ const Tq* tab(const double* d, const float* f);
-template <>
-__device__ __forceinline__ const double* tab<double>(const double* d, const float*) { return d; }
-template <>
-__device__ __forceinline__ const float* tab<float>(const double*, const float* f) { return f; }
+// Sums of products in double, or in FP32 pairs: products exact through fmaf, the
+// high parts added by TwoSum, the low parts in plain FP32 (the residuals' scheme;
+// ~46 bits of the sum).
+struct SumF64 {
+  using V = double;
+  double s = 0.0;
+  __device__ __forceinline__ void add(double a, double b) { s += a * b; }
+  __device__ __forceinline__ double get() const { return s; }
+};
+struct SumFF {
+  using V = float2;
+  float h = 0.f, l = 0.f;
+  __device__ __forceinline__ void add(float2 a, float2 b) {
+    const float p = a.x * b.x;
+    const float pe = fmaf(a.x, b.x, -p) + fmaf(a.x, b.y, a.y * b.x);
+    const float t = h + p;
+    const float z = t - h;
+    const float e = (h - (t - z)) + (p - z);
+    h = t;
+    l += e + pe;
+  }
+  __device__ __forceinline__ float2 get() const { return ff_fast_two_sum(h, l); }
+};
+
+__device__ __forceinline__ double v_of(double x, double) { return x; }
+__device__ __forceinline__ float2 v_of(double x, float2) { return d2ff(x); }
+__device__ __forceinline__ double v_mul(double a, double b) { return a * b; }
+__device__ __forceinline__ float2 v_mul(float2 a, float2 b) { return ff_mul(a, b); }
+__device__ __forceinline__ double v_neg(double a) { return -a; }
+__device__ __forceinline__ float2 v_neg(float2 a) { return make_float2(-a.x, -a.y); }
+// constant part + value, as double (pairs: 32-bit integer operations only)
+__device__ __forceinline__ double v_out(double bc, double v) { return bc + v; }
+__device__ __forceinline__ double v_out(double bc, float2 v) { return ff2d_i32(ff_add(d2ff(bc), v)); }
+__device__ __forceinline__ double v_out(double bc, double v, double q) { return bc + v + q; }
+__device__ __forceinline__ double v_out(double bc, float2 v, float q) {
+  return ff2d_i32(ff_add(ff_add(d2ff(bc), v), q));
+}
 
 // grid: x over (cells of both regions) * 2 carriers, y over instances.
-// Tq is the arithmetic type of the quadrature terms (SRH, interface, Schottky,
-// and in the FP64 path the drift).  Tq = double is the FP64 path.  Tq = float
-// is the mixed path: (1/dt) M u^{n-1} and the drift term of the current
-// equations, (q/eps) u D, keep ~47-bit accuracy -- the drift is large (|D|/h
-// relative to the density terms) and its rounding would leave a per-step
-// noise of ~eps32 |D| dt / h in the densities, above a 1e-8 steady-state
-// criterion -- but run in FP32-pair arithmetic on the FP32 pipe (fp_bits.cuh;
-// inputs split on the integer pipe), the drift as the bilinear form
-// sum_bc T_abc u_b D_c with precomputed tensors; the small recombination and
-// interface terms run in plain FP32, and only the final additions to the
-// constant part are FP64 (GB300 issues FP32 operations ~60x faster than FP64,
-// conversions included).
+// Tq is the arithmetic type of the quadrature terms (SRH, interface, Schottky).
+// Tq = double is the FP64 path.  Tq = float is the mixed path: (1/dt) M u^{n-1} and
+// the drift term of the current equations, (q/eps) u D, keep ~46-bit accuracy --
+// the drift is large (|D|/h relative to the density terms) and its rounding
+// would leave a per-step noise of ~eps32 |D| dt / h in the densities, above a 1e-8
+// steady-state criterion -- but run in FP32-pair arithmetic on the FP32 pipe
+// (fp_bits.cuh; inputs split on the integer pipe); the small recombination and
+// interface terms run in plain FP32 (GB300 issues FP32 operations ~60x faster than
+// FP64, conversions included).
+//
+// The kernel is bound by its arithmetic: the FP64 path by the FP64 unit, where a
+// warp instruction takes 64 cycles of its quarter SM however few warps there are; the
+// mixed path by the FP32 and integer pipes.  So the element integrals are taken
+// direction by direction (drift: for each tangential RT index, the normal
+// direction's 1-D matrix sum_j X_abj D_j, applied to u along it, then Y along the other:
+// 44 products per carrier at degree 1 where the full tensors took 80, 288 against 1,080
+// at degree 2), the tables are constant operands, and the recombination, the same for
+// both carriers, is evaluated by the two threads of a cell at half of the
+// quadrature points each.  Measured per launch, us, before -> after: 64 instances of
+// the 64x64+64x64 half cell, degree 1, mixed 232 -> 156; one instance, FP64 32 -> 21;
+// 8 instances, degree 2, mixed 263 -> 119; 12 instances of 29x37+23x37 cells,
+// degree 2, FP64 224 -> 80; 3 instances of 72x72+72x72, degree 2, RT_2 FP64 300 -> 118.
 template <int K, int KP, typename Tq>
 __global__ void __launch_bounds__(128, (K == 1 && sizeof(Tq) == 4) ? 8 : 1)
-    k_carrier_rhs(Tables T, RegionDev semi, RegionDev elec, int n_regions, FieldPtrs F,
+    k_carrier_rhs(const __grid_constant__ Tab1D<K, KP, typename std::conditional<sizeof(Tq) == 4, float2, double>::type, Tq> T,
+                  RegionDev semi, RegionDev elec, int n_regions, FieldPtrs F,
                   const InstDev* __restrict__ inst, const double* __restrict__ iface_ne,
                   const double* __restrict__ iface_pe, int n_iface, const double* __restrict__ sch_ne,
                   const double* __restrict__ sch_pe, const int* __restrict__ active) {
   using D = Dims<K, KP>;
-  constexpr int n1 = D::n1, nq = D::nq, Q = D::Q, nrt = D::nrt;
+  using Sum = typename std::conditional<sizeof(Tq) == 4, SumFF, SumF64>::type;
+  using V = typename Sum::V;
+  constexpr int n1 = D::n1, nq = D::nq, nrt = D::nrt, m = K + 1;
   const int i = blockIdx.y;
   if (active && !active[i]) return;
   int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -141,124 +184,162 @@ __global__ void __launch_bounds__(128, (K == 1 && sizeof(Tq) == 4) ? 8 : 1)
   const int f1 = R.field1, f = f1 + which;
   const int nc = R.nc, nd = R.nd;
   const InstDev P = inst[i];
-  const Tq* phi = tab<Tq>(T.phi, T.phi_f);
-  const Tq* qw = tab<Tq>(T.qw, T.qw_f);
-  const Tq* fphi = tab<Tq>(T.fphi, T.fphi_f);
-  const Tq* fw = tab<Tq>(T.fw, T.fw_f);
-  const Tq* psix = tab<Tq>(T.psix, T.psix_f);
-  const Tq* psiy = tab<Tq>(T.psiy, T.psiy_f);
   const double* u1p = F.u[f1] + (size_t)i * F.nd[f1] + 2 * nc * n1 + c * n1;
   const double* u2p = F.u[f1 + 1] + (size_t)i * F.nd[f1 + 1] + 2 * nc * n1 + c * n1;
-  double uown[n1];
+  const double* Pv = F.u[4] + (size_t)i * F.nd[4];
+  const double* bcp = F.bc[f] + (size_t)i * nd;
+  double* outp = F.out[f] + (size_t)i * nd;
+  const double2 h = R.h[c];
   Tq u1[n1], u2[n1];
+  V u[n1];  // the thread's own carrier
 #pragma unroll
   for (int a = 0; a < n1; ++a) {
     const double x1 = u1p[a], x2 = u2p[a];
-    uown[a] = which ? x2 : x1;
+    u[a] = v_of(which ? x2 : x1, V());
     u1[a] = to_q<Tq>(x1);
     u2[a] = to_q<Tq>(x2);
   }
-  const double* Pv = F.u[4] + (size_t)i * F.nd[4];
-  Tq Dd[nrt];
-#pragma unroll
-  for (int b = 0; b < nrt; ++b) Dd[b] = to_q<Tq>(Pv[R.rt[c * nrt + b]]);
-  const double2 h = R.h[c];
-  const Tq hxhy_q = std::is_same<Tq, double>::value ? (Tq)(h.x * h.y) : to_q<Tq>(h.x) * to_q<Tq>(h.y);
-  const Tq charge = which ? Tq(1) : Tq(-1);
-  const Tq inv_eps = to_q<Tq>(R.inv_eps);
-  // quadrature-term accumulators: [Jx (n1) | Jy (n1) | u (n1)]
-  Tq r[3 * n1];
-  float2 drift_ff[2 * n1];  // mixed path: FP32-pair drift of the current rows
-#pragma unroll
-  for (int a = 0; a < 2 * n1; ++a) drift_ff[a] = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int a = 0; a < 3 * n1; ++a) r[a] = Tq(0);
-  const bool srh = in_semi && P.srh;
-  const Tq ni = to_q<Tq>(P.n_i), taun = to_q<Tq>(P.tau_n), taup = to_q<Tq>(P.tau_p);
+  // current rows: (charge / eps) hx hy sum_bc T_abc u_b D_c.  dir 0: x components
+  // (normal direction x); dir 1 with the roles of x and y exchanged
+  const V area = v_mul(v_of(h.x, V()), v_of(h.y, V()));
+  {
+    V sc = v_mul(v_of(R.inv_eps, V()), area);
+    if (!which) sc = v_neg(sc);
 #pragma unroll 1
-  for (int q = 0; q < Q; ++q) {
-    const Tq JxW = qw[q] * hxhy_q;
-    Tq n = 0, p = 0;
-#pragma unroll
-    for (int a = 0; a < n1; ++a) {
-      const Tq ph = phi[a * Q + q];
-      n += ph * u1[a];
-      p += ph * u2[a];
-    }
-    const Tq uq = which ? p : n;
-    Tq Ex = 0, Ey = 0;
-#pragma unroll
-    for (int b = 0; b < nrt; ++b) {
-      Ex += psix[b * Q + q] * Dd[b];
-      Ey += psiy[b * Q + q] * Dd[b];
-    }
-    const Tq w = charge * inv_eps * uq * JxW;
-    Tq Rq = 0;
-    if (srh) Rq = (ni * ni - n * p) / (taun * (n + ni) + taup * (p + ni)) * JxW;
-#pragma unroll
-    for (int a = 0; a < n1; ++a) {
-      const Tq ph = phi[a * Q + q];
-      if constexpr (std::is_same<Tq, double>::value) {
-        r[a] += ph * Ex * w;
-        r[n1 + a] += ph * Ey * w;
-      }
-      r[2 * n1 + a] += ph * Rq;
-    }
-  }
-  float2 uff[n1];  // mixed path: the own density in FP32 pairs
-  if constexpr (!std::is_same<Tq, double>::value) {
-#pragma unroll
-    for (int a = 0; a < n1; ++a) uff[a] = d2ff(uown[a]);
-    // drift of the current equations: (q/eps) hx hy sum_bj T_abj u_b D_j, each
-    // product u_b D_j formed once and added into every row a
-    constexpr int NC = nrt / 2;
+    for (int dir = 0; dir < 2; ++dir) {
+      Sum W[m][m];  // [normal a1][tangential a2]
 #pragma unroll 1
-    for (int j = 0; j < NC; ++j) {
-      const float2 dx = d2ff(Pv[R.rt[c * nrt + T.drift_cx[j]]]);
-      const float2 dy = d2ff(Pv[R.rt[c * nrt + T.drift_cy[j]]]);
+      for (int j2 = 0; j2 < KP; ++j2) {
+        V Dv[KP + 1];
 #pragma unroll
-      for (int b = 0; b < n1; ++b) {
-        const float2 px = ff_mul(uff[b], dx), py = ff_mul(uff[b], dy);
+        for (int j1 = 0; j1 <= KP; ++j1) {
+          const int b = dir == 0 ? j1 + (KP + 1) * j2 : nrt / 2 + j2 + KP * j1;
+          Dv[j1] = v_of(Pv[R.rt[c * nrt + b]], V());
+        }
+        V C[m][m];  // symmetric
 #pragma unroll
-        for (int a = 0; a < n1; ++a) {
-          drift_ff[a] = ff_fma(T.drift_x_ff[(a * n1 + b) * NC + j], px, drift_ff[a]);
-          drift_ff[n1 + a] = ff_fma(T.drift_y_ff[(a * n1 + b) * NC + j], py, drift_ff[n1 + a]);
+        for (int a = 0; a < m; ++a)
+#pragma unroll
+          for (int b = a; b < m; ++b) {
+            Sum s;
+#pragma unroll
+            for (int j1 = 0; j1 <= KP; ++j1) s.add(T.X[a][b][j1], Dv[j1]);
+            C[a][b] = C[b][a] = s.get();
+          }
+#pragma unroll
+        for (int a1 = 0; a1 < m; ++a1) {
+          V vv[m];
+#pragma unroll
+          for (int b2 = 0; b2 < m; ++b2) {
+            Sum s;
+#pragma unroll
+            for (int b1 = 0; b1 < m; ++b1) s.add(C[a1][b1], dir == 0 ? u[b1 + m * b2] : u[b2 + m * b1]);
+            vv[b2] = s.get();
+          }
+#pragma unroll
+          for (int a2 = 0; a2 < m; ++a2)
+#pragma unroll
+            for (int b2 = 0; b2 < m; ++b2) W[a1][a2].add(T.Y[a2][b2][j2], vv[b2]);
         }
       }
-    }
-    float2 sc = ff_mul(ff_mul(d2ff(R.inv_eps), d2ff(h.x)), d2ff(h.y));
-    if (!which) sc = make_float2(-sc.x, -sc.y);
+      const size_t o = (size_t)dir * nc * n1 + c * n1;
 #pragma unroll
-    for (int a = 0; a < 2 * n1; ++a) drift_ff[a] = ff_mul(sc, drift_ff[a]);
+      for (int a1 = 0; a1 < m; ++a1)
+#pragma unroll
+        for (int a2 = 0; a2 < m; ++a2) {
+          const int a = dir == 0 ? a1 + m * a2 : a2 + m * a1;
+          outp[o + a] = v_out(bcp[o + a], v_mul(sc, W[a1][a2].get()));
+        }
+    }
   }
-  // interface Robin transfer (SolarCell.cpp:1265-1347, 1630-1716)
+  // quadrature terms of the density rows
+  Tq r[n1];
+#pragma unroll
+  for (int a = 0; a < n1; ++a) r[a] = Tq(0);
+  if (in_semi && P.srh) {
+    // Quadrature rows of this thread: nq / 2 whole ones from its end, and where nq
+    // is odd its part of the middle one (thread 0 the larger).  The other thread of
+    // the cell adds the rest.
+    const Tq hxhy_q = std::is_same<Tq, double>::value ? (Tq)(h.x * h.y) : to_q<Tq>(h.x) * to_q<Tq>(h.y);
+    const Tq ni = to_q<Tq>(P.n_i), taun = to_q<Tq>(P.tau_n), taup = to_q<Tq>(P.tau_p);
+#pragma unroll 1
+    for (int row = 0; row < (nq + 1) / 2; ++row) {
+      const bool middle = nq % 2 == 1 && row == nq / 2;
+      const int qy = which ? nq - 1 - row : row;
+      Tq Ly[m];
+#pragma unroll
+      for (int a = 0; a < m; ++a) Ly[a] = T.L[qy][a];
+      Tq g1[m], g2[m], hr[m];
+#pragma unroll
+      for (int ax = 0; ax < m; ++ax) {
+        g1[ax] = g2[ax] = hr[ax] = Tq(0);
+#pragma unroll
+        for (int ay = 0; ay < m; ++ay) {
+          g1[ax] += Ly[ay] * u1[ax + m * ay];
+          g2[ax] += Ly[ay] * u2[ax + m * ay];
+        }
+      }
+      const int x0 = middle && which ? (nq + 1) / 2 : 0;
+      const int x1 = middle && !which ? (nq + 1) / 2 : nq;
+#pragma unroll 1
+      for (int qx = x0; qx < x1; ++qx) {
+        Tq n = 0, p = 0;
+#pragma unroll
+        for (int ax = 0; ax < m; ++ax) {
+          n += T.L[qx][ax] * g1[ax];
+          p += T.L[qx][ax] * g2[ax];
+        }
+        const Tq JxW = T.w[qx] * T.w[qy] * hxhy_q;
+        const Tq Rq = (ni * ni - n * p) / (taun * (n + ni) + taup * (p + ni)) * JxW;
+#pragma unroll
+        for (int ax = 0; ax < m; ++ax) hr[ax] += T.L[qx][ax] * Rq;
+      }
+#pragma unroll
+      for (int ay = 0; ay < m; ++ay)
+#pragma unroll
+        for (int ax = 0; ax < m; ++ax) r[ax + m * ay] += Ly[ay] * hr[ax];
+    }
+    // both threads of a cell are here; each gets the same sum
+    const unsigned pair = 3u << (threadIdx.x & 30);
+#pragma unroll
+    for (int a = 0; a < n1; ++a) r[a] += __shfl_xor_sync(pair, r[a], 1);
+  }
+  // interface Robin transfer (SolarCell.cpp:1265-1347, 1630-1716); a face's traces
+  // are its own nodes' values
   const int4 bid = R.bid[c];
   const int bids[4] = {bid.x, bid.y, bid.z, bid.w};
-  if (n_regions > 1 && R.iface[c] >= 0 && bids[R.iface_face] == 0) {
+  if (n_regions > 1 && R.iface[c] >= 0 && (R.iface_face == 0 ? bids[0] : bids[1]) == 0) {
     const int pc = R.partner[c], ii = R.iface[c];
     const double* o1p = F.u[O.field1] + (size_t)i * F.nd[O.field1] + 2 * O.nc * n1 + pc * n1;
     const double* o2p = F.u[O.field1 + 1] + (size_t)i * F.nd[O.field1 + 1] + 2 * O.nc * n1 + pc * n1;
-    const int ff = R.iface_face, pf = R.partner_face;
-    const Tq flen = to_q<Tq>((ff == 0 || ff == 1) ? h.y : h.x);
+    const bool right = R.iface_face == 1, p_right = R.partner_face == 1;
+    const Tq flen = to_q<Tq>(h.y);
     const Tq ket = to_q<Tq>(P.k_et), kht = to_q<Tq>(P.k_ht);
+    Tq f1v[m], f2v[m], g1v[m], g2v[m], hr[m];
+#pragma unroll
+    for (int y = 0; y < m; ++y) {
+      f1v[y] = right ? u1[K + m * y] : u1[m * y];
+      f2v[y] = right ? u2[K + m * y] : u2[m * y];
+      g1v[y] = to_q<Tq>(o1p[(p_right ? K : 0) + m * y]);
+      g2v[y] = to_q<Tq>(o2p[(p_right ? K : 0) + m * y]);
+      hr[y] = Tq(0);
+    }
 #pragma unroll 1
     for (int q = 0; q < nq; ++q) {
       Tq a1 = 0, a2 = 0, b1 = 0, b2 = 0;
 #pragma unroll
-      for (int a = 0; a < n1; ++a) {
-        const Tq fo = fphi[(ff * n1 + a) * nq + q];
-        const Tq fp = fphi[(pf * n1 + a) * nq + q];
-        a1 += fo * u1[a];
-        a2 += fo * u2[a];
-        b1 += fp * to_q<Tq>(o1p[a]);
-        b2 += fp * to_q<Tq>(o2p[a]);
+      for (int y = 0; y < m; ++y) {
+        a1 += T.L[q][y] * f1v[y];
+        a2 += T.L[q][y] * f2v[y];
+        b1 += T.L[q][y] * g1v[y];
+        b2 += T.L[q][y] * g2v[y];
       }
       // semiconductor-side values n, p and electrolyte-side r, o
       const Tq n = in_semi ? a1 : b1, p = in_semi ? a2 : b2;
       const Tq rr = in_semi ? b1 : a1, oo = in_semi ? b2 : a2;
       const Tq ne = to_q<Tq>(iface_ne[(size_t)i * n_iface * nq + ii * nq + q]);
       const Tq pe = to_q<Tq>(iface_pe[(size_t)i * n_iface * nq + ii * nq + q]);
-      const Tq Jf = fw[q] * flen;
+      const Tq Jf = T.w[q] * flen;
       const Tq tn = -ket * (n - ne) * oo * Jf;
       const Tq tp = kht * (p - pe) * rr * Jf;
       Tq coef;
@@ -267,62 +348,64 @@ __global__ void __launch_bounds__(128, (K == 1 && sizeof(Tq) == 4) ? 8 : 1)
       else
         coef = which ? -(tn + tp) : (tn + tp);
 #pragma unroll
-      for (int a = 0; a < n1; ++a) r[2 * n1 + a] += fphi[(ff * n1 + a) * nq + q] * coef;
+      for (int y = 0; y < m; ++y) hr[y] += T.L[q][y] * coef;
+    }
+#pragma unroll
+    for (int y = 0; y < m; ++y) {
+      if (right)
+        r[K + m * y] += hr[y];
+      else
+        r[m * y] += hr[y];
     }
   }
   // Schottky faces (SolarCell.cpp:1348-1404)
   if (in_semi && sch_ne) {
-#pragma unroll 1
+#pragma unroll
     for (int fc = 0; fc < 4; ++fc) {
       if (bids[fc] != 3) continue;
       const Tq flen = to_q<Tq>((fc == 0 || fc == 1) ? h.y : h.x);
+#pragma unroll 1
       for (int q = 0; q < nq; ++q) {
         Tq val = 0;
 #pragma unroll
-        for (int a = 0; a < n1; ++a) val += fphi[(fc * n1 + a) * nq + q] * (which ? u2[a] : u1[a]);
+        for (int y = 0; y < m; ++y) {
+          const int a = fc == 0 ? m * y : fc == 1 ? K + m * y : fc == 2 ? y : y + m * K;
+          val += T.L[q][y] * (which ? u2[a] : u1[a]);
+        }
         const size_t o = (size_t)i * nc * 4 * nq + (size_t)(c * 4 + fc) * nq + q;
-        const Tq Jf = fw[q] * flen;
+        const Tq Jf = T.w[q] * flen;
         const Tq coef = which ? to_q<Tq>(P.s_p) * (val - to_q<Tq>(sch_pe[o])) * Jf
                               : -to_q<Tq>(P.s_n) * (val - to_q<Tq>(sch_ne[o])) * Jf;
 #pragma unroll
-        for (int a = 0; a < n1; ++a) r[2 * n1 + a] += fphi[(fc * n1 + a) * nq + q] * coef;
+        for (int y = 0; y < m; ++y) {
+          const int a = fc == 0 ? m * y : fc == 1 ? K + m * y : fc == 2 ? y : y + m * K;
+          r[a] += T.L[q][y] * coef;
+        }
       }
     }
   }
-  // constant part + (1/dt) M u^{n-1} (FP64, or FP32 pairs in the mixed path),
-  // then the quadrature terms
-  const double* bcp = F.bc[f] + (size_t)i * nd;
-  double* outp = F.out[f] + (size_t)i * nd;
+  // density rows: constant part + (1/dt) M u^{n-1} + quadrature terms
+  const V md = v_mul(area, v_of(R.inv_dt, V()));
+  V mx[n1];
 #pragma unroll
-  for (int comp = 0; comp < 2; ++comp)
+  for (int ay = 0; ay < m; ++ay)
 #pragma unroll
-    for (int a = 0; a < n1; ++a) {
-      const size_t o = (size_t)comp * nc * n1 + c * n1 + a;
-      if constexpr (std::is_same<Tq, double>::value)
-        outp[o] = bcp[o] + (double)r[comp * n1 + a];
-      else
-        outp[o] = ff2d_i32(ff_add(d2ff(bcp[o]), drift_ff[comp * n1 + a]));
+    for (int ax = 0; ax < m; ++ax) {
+      Sum s;
+#pragma unroll
+      for (int b = 0; b < m; ++b) s.add(T.mass[ax][b], u[b + m * ay]);
+      mx[ax + m * ay] = s.get();
     }
-  if constexpr (std::is_same<Tq, double>::value) {
 #pragma unroll
-    for (int a = 0; a < n1; ++a) {
-      double s = 0.0;
+  for (int ay = 0; ay < m; ++ay)
 #pragma unroll
-      for (int b = 0; b < n1; ++b) s += T.mref[a * n1 + b] * uown[b];
-      const size_t o = (size_t)2 * nc * n1 + c * n1 + a;
-      outp[o] = bcp[o] + s * (h.x * h.y) * R.inv_dt + from_q<Tq>(r[2 * n1 + a]);
+    for (int ax = 0; ax < m; ++ax) {
+      Sum s;
+#pragma unroll
+      for (int b = 0; b < m; ++b) s.add(T.mass[ay][b], mx[ax + m * b]);
+      const size_t o = (size_t)2 * nc * n1 + c * n1 + ax + m * ay;
+      outp[o] = v_out(bcp[o], v_mul(s.get(), md), r[ax + m * ay]);
     }
-  } else {
-    const float2 md = ff_mul(ff_mul(d2ff(h.x), d2ff(h.y)), d2ff(R.inv_dt));
-#pragma unroll
-    for (int a = 0; a < n1; ++a) {
-      float2 s = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int b = 0; b < n1; ++b) s = ff_fma(T.mref_ff[a * n1 + b], uff[b], s);
-      const size_t o = (size_t)2 * nc * n1 + c * n1 + a;
-      outp[o] = ff2d_i32(ff_add(ff_add(d2ff(bcp[o]), ff_mul(s, md)), r[2 * n1 + a]));
-    }
-  }
 }
 
 // grid: x over max(n_rt_total, cells of both regions), y over instances
