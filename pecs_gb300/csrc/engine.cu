@@ -14,6 +14,8 @@
 // -> steady-state reduction (2) + snapshot (1).  pecs_run_to_steady_state
 // replays a CUDA graph of two steps (even/odd ping-pong).
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <thread>
@@ -553,6 +555,45 @@ void set_error_external(const std::string& m) { g_last_error = m; }
 // ---------------------------------------------------------------------------
 // Engine
 // ---------------------------------------------------------------------------
+
+// Faults the pages of result buffers in on host threads while the GPU works, so
+// that the copies into them at the end do not (a fresh 127 MB result: 50 ms of
+// copies at 2 GB/s, 1 ms when its pages are there).  The contents are untouched; where
+// the system lacks the call the copies fault the pages in as before.
+class PageFaulter {
+ public:
+  // pointers with their bytes; nothing is done for small results
+  explicit PageFaulter(const std::vector<std::pair<void*, size_t>>& buffers) {
+#ifdef MADV_POPULATE_WRITE
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    for (const auto& b : buffers) {
+      // whole pages inside the buffer
+      const uintptr_t lo = ((uintptr_t)b.first + page - 1) / page * page;
+      const uintptr_t hi = ((uintptr_t)b.first + b.second) / page * page;
+      if (hi <= lo || b.second < (size_t)1 << 20) continue;
+      try {
+        threads_.emplace_back([this, lo, hi] {
+          const uintptr_t piece = (uintptr_t)4 << 20;
+          for (uintptr_t p = lo; p < hi && !stop_.load(std::memory_order_relaxed); p += piece)
+            if (madvise((void*)p, std::min(piece, hi - p), MADV_POPULATE_WRITE) != 0) return;
+        });
+      } catch (const std::exception&) {
+        return;  // no thread to be had: the copies fault the pages in
+      }
+    }
+#else
+    (void)buffers;
+#endif
+  }
+  ~PageFaulter() {
+    stop_ = true;
+    for (auto& t : threads_) t.join();
+  }
+
+ private:
+  std::vector<std::thread> threads_;
+  std::atomic<bool> stop_{false};
+};
 
 struct Engine {
   pecs_options opt{};
@@ -1112,10 +1153,16 @@ struct Engine {
     if (!err.empty()) throw PecsError(PECS_E_ARG, err);
     S->compute_instances(P);
     auto put = [&](DBuf<double>& d, const std::vector<std::vector<double>>& src) {
-      std::vector<double> v;
-      for (auto& x : src) v.insert(v.end(), x.begin(), x.end());
-      if (v.size() != d.n) throw PecsError(PECS_E_STATE, "instance data size changed");
-      if (!v.empty()) PECS_CUDA(cudaMemcpy(d.p, v.data(), v.size() * 8, cudaMemcpyHostToDevice));
+      // each instance's vector from where it lies: 200 MB of a 64-instance bank
+      // are not gathered in host memory first
+      size_t n = 0;
+      for (auto& x : src) n += x.size();
+      if (n != d.n) throw PecsError(PECS_E_STATE, "instance data size changed");
+      n = 0;
+      for (auto& x : src) {
+        if (!x.empty()) PECS_CUDA(cudaMemcpy(d.p + n, x.data(), x.size() * 8, cudaMemcpyHostToDevice));
+        n += x.size();
+      }
     };
     for (int f = 0; f < 5; ++f)
       if (nd[f]) put(bconst[f], S->bconst[f]);
@@ -1594,6 +1641,10 @@ struct Engine {
     if (max_steps < 1) throw PecsError(PECS_E_ARG, "max_steps < 1");
     if (check_every <= 0) check_every = 50;
     check_every += check_every & 1;
+    std::vector<std::pair<void*, size_t>> results;
+    for (int f = 0; out_fields && f < 5; ++f)
+      if (nd[f] && out_fields[f]) results.emplace_back(out_fields[f], (size_t)n_points * nd[f] * 8);
+    PageFaulter faulter(results);
     std::vector<int> slot_point(n_inst, -1);
     int next = 0;
     // The points after the first fill have their per-instance data (the

@@ -768,25 +768,36 @@ void Setup::compute_instance_data(const pecs_params& Pi, InstanceData& d, int th
       const CarrierSystem& CS = reg == 0 ? semi : elec;
       const Grid& g = CS.grid;
       const int nc = g.nc();
+      // generation rows, the same for both carriers: one evaluation per quadrature
+      // point (an exponential each; per basis function and carrier they took nearly
+      // all of the 5.8 ms of a 64x64+64x64 instance)
+      std::vector<double> gen;
+      if (reg == 0 && Pi.gen_kind != 0) {
+        gen.resize((size_t)nc * n1);
+        par_range(nc, threads, [&](int K0, int K1) {
+          std::vector<double> gq(Q);
+          for (int K = K0; K < K1; ++K) {
+            double x0, y0, hx, hy;
+            g.geom(K, x0, y0, hx, hy);
+            for (int q = 0; q < Q; ++q) gq[q] = generation(Pi, x0 + hx * ct.qx[q], y0 + hy * ct.qy[q]);
+            for (int a = 0; a < n1; ++a) {
+              double sacc = 0.0;
+              for (int q = 0; q < Q; ++q) sacc += ct.phi[a * Q + q] * gq[q] * ct.qw[q] * hx * hy;
+              gen[(size_t)K * n1 + a] = sacc;
+            }
+          }
+        });
+      }
       for (int cc = 0; cc < 2; ++cc) {
         int fld = 2 * reg + cc;
         std::vector<double> b(CS.ndofs, 0.0);
+        if (!gen.empty()) std::copy(gen.begin(), gen.end(), b.begin() + 2 * (size_t)nc * n1);
         // every cell writes only its own rows of b
         par_range(nc, threads, [&](int K0, int K1) {
         for (int K = K0; K < K1; ++K) {
           double x0, y0, hx, hy;
           g.geom(K, x0, y0, hx, hy);
           double diam = std::sqrt(hx * hx + hy * hy);
-          if (reg == 0 && Pi.gen_kind != 0) {
-            for (int a = 0; a < n1; ++a) {
-              double sacc = 0.0;
-              for (int q = 0; q < Q; ++q) {
-                double X = x0 + hx * ct.qx[q], Y = y0 + hy * ct.qy[q];
-                sacc += ct.phi[a * Q + q] * generation(Pi, X, Y) * ct.qw[q] * hx * hy;
-              }
-              b[2 * nc * n1 + K * n1 + a] += sacc;
-            }
-          }
           for (int f = 0; f < 4; ++f) {
             if (g.face_bid(K, f) != kDirichlet) continue;
             double flen = (f == kLeft || f == kRight) ? hy : hx;
@@ -824,33 +835,40 @@ void Setup::compute_instance_data(const pecs_params& Pi, InstanceData& d, int th
                 for (int qx_ = 0; qx_ < nq; ++qx_)
                   Mref[a * n1 + bb] += L[qx_][a % m] * L[qy_][a / m] * L[qx_][bb % m] * L[qy_][bb / m] *
                                        w1[qx_] * w1[qy_];
+          // Gaussian elimination with partial pivoting of Mref, the same for every
+          // cell: pivots and multipliers kept, applied to each cell's right-hand side
+          std::vector<double> M = Mref, mult(n1 * n1, 0.0);
+          std::vector<int> pivot(n1);
+          for (int col = 0; col < n1; ++col) {
+            int piv = col;
+            for (int rr = col + 1; rr < n1; ++rr)
+              if (std::fabs(M[rr * n1 + col]) > std::fabs(M[piv * n1 + col])) piv = rr;
+            pivot[col] = piv;
+            if (piv != col)
+              for (int cc2 = 0; cc2 < n1; ++cc2) std::swap(M[col * n1 + cc2], M[piv * n1 + cc2]);
+            for (int rr = col + 1; rr < n1; ++rr) {
+              const double f = M[rr * n1 + col] / M[col * n1 + col];
+              mult[rr * n1 + col] = f;
+              for (int cc2 = col; cc2 < n1; ++cc2) M[rr * n1 + cc2] -= f * M[col * n1 + cc2];
+            }
+          }
           par_range(nc, threads, [&](int K0, int K1) {
+          std::vector<double> prof(nq * nq), c(n1);
           for (int K = K0; K < K1; ++K) {
             double x0, y0, hx, hy;
             g.geom(K, x0, y0, hx, hy);
-            std::vector<double> rhs(n1, 0.0);
-            for (int a = 0; a < n1; ++a)
+            for (int qy_ = 0; qy_ < nq; ++qy_)
+              for (int qx_ = 0; qx_ < nq; ++qx_)
+                prof[qx_ + nq * qy_] = initial_profile(Pi, fld, x0 + hx * g1[qx_], y0 + hy * g1[qy_]);
+            for (int a = 0; a < n1; ++a) {
+              c[a] = 0.0;
               for (int qy_ = 0; qy_ < nq; ++qy_)
                 for (int qx_ = 0; qx_ < nq; ++qx_)
-                  rhs[a] += L[qx_][a % m] * L[qy_][a / m] *
-                            initial_profile(Pi, fld, x0 + hx * g1[qx_], y0 + hy * g1[qy_]) * w1[qx_] *
-                            w1[qy_];
-            // solve Mref c = rhs (Gaussian elimination with partial pivoting)
-            std::vector<double> M = Mref;
-            std::vector<double> c = rhs;
+                  c[a] += L[qx_][a % m] * L[qy_][a / m] * prof[qx_ + nq * qy_] * w1[qx_] * w1[qy_];
+            }
             for (int col = 0; col < n1; ++col) {
-              int piv = col;
-              for (int rr = col + 1; rr < n1; ++rr)
-                if (std::fabs(M[rr * n1 + col]) > std::fabs(M[piv * n1 + col])) piv = rr;
-              if (piv != col) {
-                for (int cc2 = 0; cc2 < n1; ++cc2) std::swap(M[col * n1 + cc2], M[piv * n1 + cc2]);
-                std::swap(c[col], c[piv]);
-              }
-              for (int rr = col + 1; rr < n1; ++rr) {
-                double f = M[rr * n1 + col] / M[col * n1 + col];
-                for (int cc2 = col; cc2 < n1; ++cc2) M[rr * n1 + cc2] -= f * M[col * n1 + cc2];
-                c[rr] -= f * c[col];
-              }
+              if (pivot[col] != col) std::swap(c[col], c[pivot[col]]);
+              for (int rr = col + 1; rr < n1; ++rr) c[rr] -= mult[rr * n1 + col] * c[col];
             }
             for (int rr = n1 - 1; rr >= 0; --rr) {
               double sacc = c[rr];
