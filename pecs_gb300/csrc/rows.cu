@@ -5,6 +5,7 @@
 #include <memory>
 #include <type_traits>
 
+#include "bulk_copy.cuh"
 #include "rows.cuh"
 #include "sweep_sync.cuh"
 
@@ -123,34 +124,6 @@ template <typename T>
 __host__ __device__ inline int red_stride(int n) {
   constexpr int line = 128 / (int)sizeof(T), vec = 16 / (int)sizeof(T);
   return (n + line - 1) / line * line + vec;
-}
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void bar_init(unsigned bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar) : "memory");
-}
-
-// Bulk copy of `bytes` (a multiple of 16, both sides 16-byte aligned) that completes on `bar`.
-__device__ __forceinline__ void bulk_load(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
-               "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
-
-// Bounded wait for a barrier phase; false when the copies did not arrive.
-__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity) {
-  for (int i = 0; i < (1 << 20); ++i) {
-    unsigned done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
 }
 
 // A column's value -- b minus the children's updates -- or (COL = false) a

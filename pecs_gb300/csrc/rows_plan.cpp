@@ -12,6 +12,47 @@
 
 namespace pecs {
 
+NodeSpans node_spans(const MfFactor& F, int j) {
+  NodeSpans S;
+  const int s = F.nodes[j].s, f = s + F.nodes[j].m;
+  const std::vector<double>&G = F.Gf[j], &H = F.Hb[j];
+  std::vector<int> first(s, s);
+  S.order.resize(s), S.start.resize(s), S.reach.assign(s + 1, s);
+  for (int r = 0; r < s; ++r)
+    for (int c = 0; c < s; ++c)
+      if (first[c] == s && G[(size_t)r * s + c] != 0.0) first[c] = r;
+  std::iota(S.order.begin(), S.order.end(), 0);
+  std::stable_sort(S.order.begin(), S.order.end(), [&](int a, int b) { return first[a] < first[b]; });
+  for (int k = 0; k < s; ++k) S.start[k] = first[S.order[k]];
+  for (int r = s - 1; r >= 0; --r) {
+    int c = 0;
+    while (c < s && H[(size_t)r * f + c] == 0.0) ++c;
+    S.reach[r] = std::min(S.reach[r + 1], c);
+  }
+  return S;
+}
+
+void NodeSpans::columns(bool fwd, int s, int m, int r0, int r1, int& k0, int& K) const {
+  k0 = 0;
+  K = fwd ? s : s + m;
+  if (fwd && r1 <= s) K = (int)(std::lower_bound(start.begin(), start.end(), r1) - start.begin());
+  if (!fwd) k0 = std::min(reach[r0], K - 1), K -= k0;
+  K = std::max(K, 1);
+}
+
+RowRec make_rec(int src, const std::vector<int>& l, std::vector<int>& more) {
+  RowRec r;
+  r.src = src;
+  const int n = (int)l.size(), k = n <= kRowsSlots ? n : kRowsSlots - 1;
+  for (int i = 0; i < kRowsSlots; ++i) r.slot[i] = i < k ? l[i] : -1;
+  if (n > k) {
+    r.slot[kRowsSlots - 1] = -2 - (int)more.size();
+    more.push_back(n - k);
+    more.insert(more.end(), l.begin() + k, l.end());
+  }
+  return r;
+}
+
 namespace {
 
 template <typename F>
@@ -26,7 +67,6 @@ void parallel(int n, F f) {
 // A batch applies small leaves thread by output; its columns are read once per
 // output, so only FP64 values (no conversions) and short rows.
 constexpr int kBatchArea = 1280, kBatchCols = 64, kBatchRows = 256;
-constexpr int kRowsSms = 152;
 
 template <typename T>
 void pack(const RowsPlan& P, const std::vector<const MfFactor*>& factors, int d, T* out) {
@@ -47,7 +87,7 @@ void pack(const RowsPlan& P, const std::vector<const MfFactor*>& factors, int d,
       const double* A = (d == 0 ? factors[x.set]->Gf[x.j] : factors[x.set]->Hb[x.j]).data() + (size_t)it.row0 * ld;
       const int k0 = batch[i] ? 0 : it.src - D.src0[g];
       for (int k = 0; k < it.cols; ++k, p += pad) {
-        const int c = d == 0 ? P.order[g][k0 + k] : k0 + k;
+        const int c = d == 0 ? P.spans[g].order[k0 + k] : k0 + k;
         for (int r = 0; r < it.rows; ++r) p[r] = (T)A[(size_t)r * ld + c];
         for (int r = it.rows; r < pad; ++r) p[r] = T(0);
       }
@@ -105,34 +145,8 @@ RowsPlan plan_rows(const std::vector<const MfFactor*>& factors, int vr, int max_
   for (int g = 0; g < (int)nodes.size(); ++g)
     if (is_batch(g, 1)) nodes[g].level[1] = nl[1] - 1;
   const int N = (int)nodes.size();
-  // The blocks hold triangular inverses (L11^-1 P, U11^-1): a tile leaves out
-  // the columns that are zero in all of its rows.  Forward, a node's columns are
-  // taken in the order of their first nonzero row, and a tile of the first s
-  // rows covers those that start above its end; backward, a tile covers the
-  // columns from the first one that reaches its rows or later ones.
-  std::vector<std::vector<int>> start(N), reach(N);
-  R.order.resize(N);
-  parallel(N, [&](int g) {
-    const RowsPlan::Node& x = nodes[g];
-    const int s = x.s, f = s + x.m;
-    const std::vector<double>& G = factors[x.set]->Gf[x.j];
-    const std::vector<double>& H = factors[x.set]->Hb[x.j];
-    std::vector<int> first(s, s), o(s), lo(s + 1, s);
-    for (int r = 0; r < s; ++r)
-      for (int c = 0; c < s; ++c)
-        if (first[c] == s && G[(size_t)r * s + c] != 0.0) first[c] = r;
-    std::iota(o.begin(), o.end(), 0);
-    std::stable_sort(o.begin(), o.end(), [&](int a, int b) { return first[a] < first[b]; });
-    start[g].resize(s);
-    for (int k = 0; k < s; ++k) start[g][k] = first[o[k]];
-    R.order[g] = std::move(o);
-    for (int r = s - 1; r >= 0; --r) {
-      int c = 0;
-      while (c < s && H[(size_t)r * f + c] == 0.0) ++c;
-      lo[r] = std::min(lo[r + 1], c);
-    }
-    reach[g] = std::move(lo);
-  });
+  R.spans.resize(N);
+  parallel(N, [&](int g) { R.spans[g] = node_spans(*factors[nodes[g].set], nodes[g].j); });
   // nodes in level order (tiles, then batches by shape), and the lists
   std::vector<std::vector<int>> lv[2];
   for (int d = 0; d < 2; ++d) {
@@ -154,7 +168,7 @@ RowsPlan plan_rows(const std::vector<const MfFactor*>& factors, int vr, int max_
         D.pos[g] = (int)D.at.size();
         D.at.push_back(g);
         D.src0[g] = (int)D.src.size();
-        for (int t = 0; t < x.s; ++t) D.src.push_back(nd.own[d == 0 ? R.order[g][t] : t]);
+        for (int t = 0; t < x.s; ++t) D.src.push_back(nd.own[d == 0 ? R.spans[g].order[t] : t]);
         if (d == 1)
           for (int t = 0; t < x.m; ++t) D.src.push_back(~nd.upd[t]);
         D.dst0[g] = (int)D.dst.size();
@@ -180,7 +194,7 @@ RowsPlan plan_rows(const std::vector<const MfFactor*>& factors, int vr, int max_
       for (int j = 0; j < (int)F.nodes.size(); ++j) {
         const int g = base + j;
         const MfNode& x = F.nodes[j];
-        for (int t = 0; t < x.s; ++t) fpos[x.own[R.order[g][t]]] = t;
+        for (int t = 0; t < x.s; ++t) fpos[x.own[R.spans[g].order[t]]] = t;
         for (int t = 0; t < x.m; ++t) fpos[x.upd[t]] = x.s + t;
         lists.assign(x.s + x.m, {});
         for (int c : x.children)
@@ -193,15 +207,7 @@ RowsPlan plan_rows(const std::vector<const MfFactor*>& factors, int vr, int max_
         for (int t = 0; t < x.m; ++t) fpos[x.upd[t]] = -1;
         for (int p = 0; p < x.s + x.m; ++p) {
           RowRec& r = p < x.s ? R.rec[R.dir[0].src0[g] + p] : R.upd[upd0[g] + p - x.s];
-          r.src = p < x.s ? x.own[R.order[g][p]] : nodes[g].w_off + p - x.s;
-          const std::vector<int>& l = lists[p];
-          const int n = (int)l.size(), k = n <= kRowsSlots ? n : kRowsSlots - 1;
-          for (int i = 0; i < kRowsSlots; ++i) r.slot[i] = i < k ? l[i] : -1;
-          if (n > k) {
-            r.slot[kRowsSlots - 1] = -2 - (int)R.more.size();
-            R.more.push_back(n - k);
-            R.more.insert(R.more.end(), l.begin() + k, l.end());
-          }
+          r = make_rec(p < x.s ? x.own[R.spans[g].order[p]] : nodes[g].w_off + p - x.s, lists[p], R.more);
         }
       }
       base += (int)F.nodes.size();
@@ -251,11 +257,9 @@ RowsPlan plan_rows(const std::vector<const MfFactor*>& factors, int vr, int max_
         L.leaf = L.leaf && x.leaf;
         // columns [k0, k0 + K) of rows [r0, r1)
         auto span = [&](int r0, int r1, int& k0) {
-          k0 = 0;
-          int K = cols_of(g);
-          if (fwd && r1 <= x.s) K = (int)(std::lower_bound(start[g].begin(), start[g].end(), r1) - start[g].begin());
-          if (!fwd) k0 = std::min(reach[g][r0], K - 1), K -= k0;
-          return std::max(K, 1);
+          int K = 0;
+          R.spans[g].columns(fwd, x.s, x.m, r0, r1, k0, K);
+          return K;
         };
         // tiles of about `want` values, the rows of a triangular part in unequal
         // ones; forward, none across the end of the own rows unless the whole node

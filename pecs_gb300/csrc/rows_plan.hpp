@@ -11,6 +11,21 @@ constexpr int kRowsThreads = 256;  // threads of a CTA
 constexpr int kRowsMaxSets = 4;
 constexpr int kRowsSlots = 7;      // child update slots in a record
 
+constexpr int kRowsSms = 152;      // multiprocessors of a GB300
+
+// The blocks hold triangular inverses (L11^-1 P, U11^-1): a tile leaves out the
+// columns that are zero in all of its rows.  Forward, a node's columns are taken
+// in the order of their first nonzero row, and a tile of the first s rows covers
+// those that start above its end; backward, a tile covers the columns from the
+// first one that reaches its rows or later ones.
+struct NodeSpans {
+  std::vector<int> order, start, reach;
+  // columns [k0, k0 + K) of rows [r0, r1) of a node of s own and m update rows (forward:
+  // places in `order`)
+  void columns(bool fwd, int s, int m, int r0, int r1, int& k0, int& K) const;
+};
+NodeSpans node_spans(const MfFactor& F, int j);
+
 // Where a front position's value comes from (forward): the right-hand side of
 // dof src (update rows: their own slot) and up to kRowsSlots child update slots (-1: no more); with
 // more of them the last entry is -2 - i, and more[i] holds their number, then them.
@@ -64,6 +79,9 @@ struct alignas(16) RowSync {
   int wait, target, signal, unused;
 };
 
+// A record with these child update slots (more than it holds: in `more`).
+RowRec make_rec(int src, const std::vector<int>& slots, std::vector<int>& more);
+
 struct RowsPlan {
   struct Node {
     int set, j, s, m, level[2], parent, w_off;
@@ -87,7 +105,7 @@ struct RowsPlan {
   std::vector<int> wtotal;           // update slots per set
   std::vector<RowRec> rec, upd;      // forward: columns (as dir[0].src), update rows
   std::vector<int> more;
-  std::vector<std::vector<int>> order;  // per node: its columns in forward order
+  std::vector<NodeSpans> spans;      // per node
   long long entries = 0;             // stored values of the factors, zeros included
 };
 

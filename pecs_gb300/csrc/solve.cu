@@ -8,6 +8,8 @@
 #include <cstring>
 #include <type_traits>
 
+#include "bulk_copy.cuh"
+#include "panel_plan.hpp"
 #include "solve.cuh"
 #include "sweep_sync.cuh"
 
@@ -16,17 +18,10 @@ namespace pecs {
 namespace {
 
 // ---- panel path --------------------------------------------------------------
-constexpr int kPanelKcF32 = 128;  // staged columns per chunk, FP32 blocks
-constexpr int kPanelKcF64 = 64;   // staged columns per chunk, FP64 blocks
-// chunk sizes the launch may fall back to (per-level child-row counts are
-// precomputed for each)
-constexpr int kPanelKcSteps = 8;
-constexpr int kPanelKc[kPanelKcSteps] = {128, 64, 32, 16, 8, 4, 2, 1};
 constexpr size_t kPanelSmem = 160 * 1024;
-constexpr int kPanelCmMax = 4096;  // staged child-update rows per node (more: read from global)
-constexpr int kSplitMaxParts = 8;  // split-K: at most this many column parts per tile
-constexpr int kSplitPart = 128;    // split-K: columns per part (a multiple of every chunk size)
-constexpr int kSplitMinK = 192;    // split-K: only nodes with at least this many columns
+constexpr size_t kTileSmem = 200 * 1024;   // most of a level launch
+constexpr size_t kTileOnce = 100 * 1024;   // columns staged in one go up to here, else in two buffers
+constexpr size_t kTileBuffer = 48 * 1024;  // ... of this size
 constexpr size_t kWarpSmem = 48 * 1024;  // leaf levels: shared memory per CTA
 
 // RPL consecutive values of one interleaved row (offset a multiple of RPL),
@@ -124,7 +119,7 @@ __device__ __forceinline__ void sts(T* p, const VR (&v)[N]) {
   }
 }
 
-// One item = rows [r0, r1) of one node's block (Gf for the forward sweep, Hb
+// Flow sweeps: one item = rows [r0, r1) of one node's block (Gf for the forward sweep, Hb
 // for the backward sweep; both column-major with leading dimension = row
 // count), applied to the right-hand-side chunk blockIdx.y (32 * RPL RHS).
 // Rows are tiled ri at a time (ri in {4, 8, 16, 32}): warp (g, part) owns rows
@@ -212,11 +207,9 @@ struct PanelShape {
 // vector is read; it returns false when the inputs could not be waited for,
 // and the item then writes NaN (the solve's results are flagged non-finite).
 // main_done() is called once the item no longer reads its inputs.
-template <typename T, int RPL, bool FWD, typename SVT, typename Wait, typename Done>
+template <typename T, int RPL, bool FWD, typename SVT, typename Wait>
 __device__ __forceinline__ void panel_tile(const BankView& B, const SVT& S, const PanelItem& I, int rc0,
-                                           int chunk, const PanelShape& P, T* __restrict__ partials,
-                                           int* __restrict__ counters, int parts_ld, int ychunks,
-                                           unsigned char* smem_raw, Wait wait_inputs, Done main_done) {
+                                           const PanelShape& P, unsigned char* smem_raw, Wait wait_inputs) {
   constexpr int RC = 32 * RPL;
   constexpr int NW = kSolveThreads / 32;
   const int r0 = I.a.y, r1 = I.a.z, ri = I.a.w;
@@ -238,11 +231,7 @@ __device__ __forceinline__ void panel_tile(const BankView& B, const SVT& S, cons
   const int nrows = r1 - r0;
   const int wpr = 32 / ri;  // warps sharing a row group (column parts)
   const int g = warp / wpr, part = warp % wpr;
-  // split-K: this CTA covers columns [k_lo, k_hi) of a tile split in n_parts;
-  // an unsplit item may carry its own (smaller) chunk width in e.x
-  const bool split = I.e.z >= 0;
-  const int k_lo = split ? I.e.x : 0, k_hi = split ? I.e.y : K;
-  const int kc_cap = (!split && I.e.x > 0) ? min(I.e.x, P.kc_cap) : P.kc_cap;
+  const int kc_cap = min(I.kc, P.kc_cap);
   bool bad = false;
   const int nbuf = P.nbuf;
   // staging buffers, nbuf of each: Ds [ds_rows][RC] (nbuf * ds_rows >= 32 when
@@ -283,7 +272,7 @@ __device__ __forceinline__ void panel_tile(const BankView& B, const SVT& S, cons
   // child-update rows
   const int ri_log = 31 - __clz(ri);  // ri is a power of two
   auto stage_block = [&](int k0, int b) {
-    const int kc = min(kc_cap, k_hi - k0);
+    const int kc = min(kc_cap, K - k0);
     T* Gs = Gs0 + (size_t)b * P.kc_cap * ri_max;
     const T* Mk = M + (size_t)k0 * ld + r0;
     for (int idx = tid; idx < kc * ri; idx += kSolveThreads) {
@@ -295,7 +284,7 @@ __device__ __forceinline__ void panel_tile(const BankView& B, const SVT& S, cons
     }
   };
   auto stage_rows = [&](int k0, int b) {
-    const int kc = min(kc_cap, k_hi - k0);
+    const int kc = min(kc_cap, K - k0);
     T* Ds = Ds0 + (size_t)b * ds_rows * RC;
     for (int k = warp; k < kc; k += NW) {
       const int sr = src_s[k0 + k];
@@ -315,14 +304,14 @@ __device__ __forceinline__ void panel_tile(const BankView& B, const SVT& S, cons
     }
     cp_async_commit();
   };
-  if (k_lo < k_hi) stage_block(k_lo, 0);
+  if (K > 0) stage_block(0, 0);
   bad = !wait_inputs();  // vectors below are written by earlier work
-  if (k_lo < k_hi) stage_rows(k_lo, 0);
+  if (K > 0) stage_rows(0, 0);
   int chunk_i = 0;
-  for (int k0 = k_lo; k0 < k_hi; k0 += kc_cap, ++chunk_i) {
-    const int kc = min(kc_cap, k_hi - k0);
+  for (int k0 = 0; k0 < K; k0 += kc_cap, ++chunk_i) {
+    const int kc = min(kc_cap, K - k0);
     const int b = nbuf == 2 ? (chunk_i & 1) : 0;
-    const bool more = k0 + kc_cap < k_hi;
+    const bool more = k0 + kc_cap < K;
     if (more && nbuf == 2) {
       stage_block(k0 + kc_cap, b ^ 1);
       stage_rows(k0 + kc_cap, b ^ 1);
@@ -372,7 +361,6 @@ __device__ __forceinline__ void panel_tile(const BankView& B, const SVT& S, cons
       stage_rows(k0 + kc_cap, 0);
     }
   }
-  main_done();
   // row i of the item -> its destination
   auto emit = [&](int i, T (&v)[RPL]) {
     const int row = r0 + i;
@@ -397,21 +385,11 @@ __device__ __forceinline__ void panel_tile(const BankView& B, const SVT& S, cons
       st_rhs<RPL>(st.x + (size_t)src_s[row] * R + rl, v);
     }
   };
-  // row totals -> destination, or (split-K) this part's slab of partials
-  auto finish = [&](int i, T (&v)[RPL]) {
-    if (!split) {
-      emit(i, v);
-    } else {
-      T* dst = partials + ((size_t)(I.e.z * kSplitMaxParts + I.d.w) * 32 + i) * parts_ld + rl;
-#pragma unroll
-      for (int q = 0; q < RPL; ++q) dst[q] = v[q];
-    }
-  };
   if (wpr == 1) {
     if (lane_ok) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        if (4 * g + i < nrows) finish(4 * g + i, acc[i]);
+        if (4 * g + i < nrows) emit(4 * g + i, acc[i]);
     }
   } else {
     T* red = Ds0;  // [wpr][ri][RC] = 32 * RC values
@@ -430,50 +408,328 @@ __device__ __forceinline__ void panel_tile(const BankView& B, const SVT& S, cons
           for (int p = 0; p < wpr; ++p) t += red[((size_t)p * ri + i) * RC + lane * RPL + q];
           v[q] = t;
         }
-        finish(i, v);
+        emit(i, v);
       }
     }
   }
-  if (!split) return;
-  // split-K: the last CTA of the tile to arrive adds the parts in part order
-  // (the result does not depend on which CTA is last) and writes the rows
-  __shared__ int ticket;
-  __threadfence();
-  __syncthreads();
-  int* ctr = counters + (size_t)I.e.z * ychunks + chunk;
-  if (tid == 0) ticket = atomicAdd(ctr, 1);
-  __syncthreads();
-  if (ticket != I.e.w - 1) return;
-  __threadfence();
-  if (lane_ok) {
-    for (int i = warp; i < nrows; i += NW) {
-      T v[RPL];
-#pragma unroll
-      for (int q = 0; q < RPL; ++q) v[q] = T(0);
-      for (int p = 0; p < I.e.w; ++p) {
-        const T* src = partials + ((size_t)(I.e.z * kSplitMaxParts + p) * 32 + i) * parts_ld + rl;
-#pragma unroll
-        for (int q = 0; q < RPL; ++q) v[q] += __ldcg(src + q);
-      }
-      emit(i, v);
-    }
-  }
-  if (tid == 0) *ctr = 0;
 }
 
-template <typename T, int RPL, bool FWD, typename SVT>
+// ---- level sweeps --------------------------------------------------------------
+// A tile applies up to 32 rows of a node's block to a chunk of 32 * NW right-hand
+// sides.  A warp holds the sums of all of the tile's rows for 32 of them (lanes 4 x 8:
+// pad / 4 rows by 4 right-hand sides each); the warps left over split the columns
+// and add their sums through shared memory.  What bounds a level is latency -- it
+// has 1 to 10 MB of values and a few of arithmetic per multiprocessor -- so a
+// tile needs one round trip for what is constant (record, then values and index list
+// by bulk copies, under the previous level's tail) and one for the vectors' rows.
+// Forward, the nodes' columns and pass-through sums are formed once by k_panel_assemble
+// in a launch before (into x, which the backward sweep overwrites): in each tile of
+// a node that was 4 to 11 times the reading, and half of the shared memory.
+// 64x64+64x64 cells, 64 instances, FP32, us per carrier sweep of 128 / Poisson sweep of
+// 64 right-hand sides: 510 / 188 with the columns assembled in every tile and the blocks
+// read column-major (4-byte copies), 346 / 115 with both done once, 337 / 110 with packed
+// multiply-adds and fewer instructions in the assembly.  Tried without gain: 8 x 8
+// sums per thread (343 / 110), four smaller buffers (339 to 367), pass-through rows
+// loaded into the sums (366 / 129).  The multiply-adds alone are 65 / 13.
+struct TileShape {
+  int kc, lg_nw;          // staged columns; log2 of 32-right-hand-side groups per CTA
+  unsigned a, b, p;       // shared-memory offsets: values, vector rows, pass-through rows
+  unsigned a_buf, b_buf;  // one buffer of values, of rows
+};
+
+// MR x 4 sums of one thread.  FP32: two rows per register pair, so that one packed
+// instruction (fma.rn.f32x2, each half rounded as fmaf) does two of them.
+template <typename T, int MR>
+struct TileAcc {
+  T v_[MR][4];
+  __device__ __forceinline__ void set(int i, const T (&v)[4]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v_[i][q] = v[q];
+  }
+  __device__ __forceinline__ void get(int i, T (&v)[4]) const {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = v_[i][q];
+  }
+  __device__ __forceinline__ void fma(const T (&a)[MR], const T (&d)[4]) {
+#pragma unroll
+    for (int i = 0; i < MR; ++i)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v_[i][q] += a[i] * d[q];
+  }
+};
+template <int MR>
+struct TileAcc<float, MR> {
+  unsigned long long v_[MR / 2][4];
+  static __device__ __forceinline__ unsigned long long pack(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+  }
+  static __device__ __forceinline__ float2 unpack(unsigned long long p) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p));
+    return r;
+  }
+  __device__ __forceinline__ void set(int i, const float (&v)[4]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float2 t = i % 2 ? unpack(v_[i / 2][q]) : make_float2(0.f, 0.f);
+      (i % 2 ? t.y : t.x) = v[q];
+      v_[i / 2][q] = pack(t.x, t.y);
+    }
+  }
+  __device__ __forceinline__ void get(int i, float (&v)[4]) const {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float2 t = unpack(v_[i / 2][q]);
+      v[q] = i % 2 ? t.y : t.x;
+    }
+  }
+  __device__ __forceinline__ void fma(const float (&a)[MR], const float (&d)[4]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const unsigned long long dd = pack(d[q], d[q]);
+#pragma unroll
+      for (int i = 0; i < MR / 2; ++i)
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(v_[i][q]) : "l"(pack(a[2 * i], a[2 * i + 1])), "l"(dd));
+    }
+  }
+};
+
+// 4 right-hand sides from column c of a row (c a multiple of 4; R: their number)
+template <typename T>
+__device__ __forceinline__ void st4(T* row, int c, int R, const T (&v)[4]) {
+  if (R % 4 == 0) {
+    if (c < R) sts<T, 4>(row + c, v);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (c + q < R) row[c + q] = v[q];
+  }
+}
+
+template <typename T, int MR, bool FWD, typename SV>
+__device__ __forceinline__ void tile_apply(const TilesView& B, const SV& st, const PanelTile& I, const TileShape& P,
+                                           int c0, unsigned char* smem) {
+  constexpr int BM = 4 * MR;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x;
+  const int lg = P.lg_nw, nw = warp & ((1 << lg) - 1), kg = warp >> lg, KG = nthr >> (5 + lg);
+  const int BN = 32 << lg, R = st.nrhs, K = I.cols, kc_max = P.kc, K4 = (K + 3) & ~3;
+  const unsigned bar = smem_u32(smem);
+  const T* val = static_cast<const T*>(B.val) + I.off;
+  const int* idx = reinterpret_cast<const int*>(smem + 16);
+  if (tid == 0) {
+    bar_init(bar);
+    bar_init(bar + 8);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    const unsigned nv = min(K, kc_max) * BM * (unsigned)sizeof(T), ni = (K4 + BM) * 4u;
+    bar_expect(bar, nv + ni);
+    bulk_copy(bar + 16, B.idx + I.idx, ni, bar);
+    bulk_copy(bar + P.a, val, nv, bar);
+    if (K > kc_max)
+      bulk_load(bar + P.a + P.a_buf, val + (size_t)kc_max * BM, min(K - kc_max, kc_max) * BM * (unsigned)sizeof(T), bar + 8);
+  }
+  __syncthreads();
+  bool ok = bar_wait(bar, 0);
+  pdl_wait();  // vectors below are written by earlier work
+  // n rows given by their indices -> dst [n][BN], zeros past the last right-hand side
+  auto stage = [&](T* dst, const int* rows, int n, auto row_of) {
+    constexpr int V = 16 / (int)sizeof(T);
+    if (R % V == 0) {
+      const int lp = lg + (sizeof(T) == 4 ? 3 : 4);  // log2 of 16-byte pieces per row
+      for (int e = tid; e < n << lp; e += nthr) {
+        const int c = c0 + (e & ((1 << lp) - 1)) * V;
+        if (c < R)
+          cp_async<16>(dst + (size_t)e * V, row_of(rows[e >> lp]) + c);
+        else
+          *reinterpret_cast<float4*>(dst + (size_t)e * V) = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    } else {
+      for (int e = tid; e < n << (lg + 5); e += nthr) {
+        const int c = c0 + (e & (BN - 1));
+        if (c < R)
+          cp_async<sizeof(T)>(dst + e, row_of(rows[e >> (lg + 5)]) + c);
+        else
+          dst[e] = T(0);
+      }
+    }
+  };
+  auto stage_columns = [&](int k0, int b) {
+    T* dst = reinterpret_cast<T*>(smem + P.b + b * P.b_buf);
+    const int n = min(kc_max, K - k0);
+    if constexpr (FWD) {
+      const T* src = I.leaf ? st.b : st.x;
+      stage(dst, idx + k0, n, [&](int z) { return src + (size_t)z * R; });
+    } else {
+      stage(dst, idx + k0, n,
+            [&](int z) { return z >= 0 ? static_cast<const T*>(st.y) + (size_t)z * R : static_cast<const T*>(st.x) + (size_t)(~z) * R; });
+    }
+  };
+  stage_columns(0, 0);
+  T* Ps = reinterpret_cast<T*>(smem + P.p);
+  if (FWD && I.npt > 0)
+    stage(Ps, idx + K4 + I.rows - I.npt, I.npt, [&](int z) { return static_cast<const T*>(st.w) + (size_t)(~z) * R; });
+  cp_async_commit();
+  if (K > kc_max) stage_columns(kc_max, 1);
+  cp_async_commit();
+  const int rg = lane >> 3, cg = lane & 7;
+  TileAcc<T, MR> acc;
+#pragma unroll
+  for (int i = 0; i < MR; ++i) {
+    const T zero[4] = {T(0), T(0), T(0), T(0)};
+    acc.set(i, zero);
+  }
+  for (int k0 = 0, c = 0;; ++c) {
+    const int b = c & 1, kc = min(kc_max, K - k0);
+    cp_async_wait_group<1>();  // chunk c; the next one's copies may be in flight
+    if (c > 0) ok = bar_wait(bar + 8 * b, (c >> 1) & 1) && ok;
+    __syncthreads();
+    const T* a = reinterpret_cast<const T*>(smem + P.a + b * P.a_buf) + kg * BM + rg * MR;
+    const T* d = reinterpret_cast<const T*>(smem + P.b + b * P.b_buf) + kg * BN + nw * 32 + cg * 4;
+#pragma unroll 4
+    for (int k = kg; k < kc; k += KG) {
+      T av[MR], dv[4];
+      lds<T, MR>(a, av);
+      lds<T, 4>(d, dv);
+      acc.fma(av, dv);
+      a += KG * BM;
+      d += KG * BN;
+    }
+    k0 += kc;
+    if (k0 >= K) break;
+    __syncthreads();  // buffer b is free
+    const int next = k0 + min(kc_max, K - k0);
+    if (next < K) {
+      if (tid == 0)
+        bulk_load(bar + P.a + b * P.a_buf, val + (size_t)next * BM, min(K - next, kc_max) * BM * (unsigned)sizeof(T), bar + 8 * b);
+      stage_columns(next, b);
+    }
+    cp_async_commit();
+  }
+  pdl_trigger();
+  // row totals -> destination
+  auto emit = [&](int row, int c, T (&v)[4]) {
+    const int z = idx[K4 + row];
+    if (FWD && row >= I.rows - I.npt) {
+      T u[4];
+      lds<T, 4>(Ps + (size_t)(row - (I.rows - I.npt)) * BN + c, u);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] += u[q];
+    }
+    if (!ok) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = quiet_nan<T>();
+    }
+    T* dst = FWD ? (z >= 0 ? st.y + (size_t)z * R : st.w + (size_t)(~z) * R) : st.x + (size_t)z * R;
+    st4(dst, c0 + c, R, v);
+  };
+  if (KG == 1) {
+#pragma unroll
+    for (int i = 0; i < MR; ++i) {
+      T v[4];
+      acc.get(i, v);
+      if (rg * MR + i < I.rows) emit(rg * MR + i, nw * 32 + cg * 4, v);
+    }
+    return;
+  }
+  __syncthreads();  // the partial sums overlay the values and rows
+  T* red = reinterpret_cast<T*>(smem + P.a);  // [KG][BM][BN]
+#pragma unroll
+  for (int i = 0; i < MR; ++i) {
+    T v[4];
+    acc.get(i, v);
+    sts<T, 4>(red + (size_t)(kg * BM + rg * MR + i) * BN + nw * 32 + cg * 4, v);
+  }
+  __syncthreads();
+  for (int e = tid; e < I.rows << (lg + 3); e += nthr) {
+    const int row = e >> (lg + 3), c = (e & ((8 << lg) - 1)) * 4;
+    T v[4] = {T(0), T(0), T(0), T(0)};
+    for (int g = 0; g < KG; ++g) {
+      T u[4];
+      lds<T, 4>(red + (size_t)(g * BM + row) * BN + c, u);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] += u[q];
+    }
+    emit(row, c, v);
+  }
+}
+
+template <typename T, bool FWD, typename SVT>
 __global__ void __launch_bounds__(kSolveThreads)
-    k_panel(BankView B, SVT S, const PanelItem* __restrict__ items, PanelShape P, T* __restrict__ partials,
-            int* __restrict__ counters, int parts_ld, int ychunks) {
+    k_panel_tiles(TilesView B, SVT S, int first, TileShape P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const PanelItem I = items[blockIdx.x];
-  panel_tile<T, RPL, FWD, SVT>(
-      B, S, I, (int)blockIdx.y * 32 * RPL, (int)blockIdx.y, P, partials, counters, parts_ld, ychunks, smem_raw,
-      [] {
-        pdl_wait();
-        return true;
-      },
-      [] { pdl_trigger(); });
+  const PanelTile I = B.tiles[first + blockIdx.x];
+  const auto& st = S.set[I.set];
+  const int c0 = (int)blockIdx.y * (32 << P.lg_nw);
+  if (c0 >= st.nrhs) return;
+  if (I.pad == 32)
+    tile_apply<T, 8, FWD>(B, st, I, P, c0, smem_raw);
+  else if (I.pad == 16)
+    tile_apply<T, 4, FWD>(B, st, I, P, c0, smem_raw);
+  else
+    tile_apply<T, 2, FWD>(B, st, I, P, c0, smem_raw);
+}
+
+// Forward, before a level's tiles: its nodes' columns, b minus the children's updates,
+// into x, and the pass-through sums into their update slots.  V right-hand sides of a
+// front position per thread.
+struct AsmSets {
+  int rec[kMaxSets], n[kMaxSets];
+};
+
+template <typename T, int V, typename SVT>
+__global__ void __launch_bounds__(kSolveThreads) k_panel_assemble(TilesView B, SVT S, AsmSets A, int lg) {
+  // 2^lg threads share a position
+  const auto& st = S.set[blockIdx.y];
+  const int R = st.nrhs;
+  const unsigned e = blockIdx.x * (unsigned)kSolveThreads + threadIdx.x;
+  const int p = (int)(e >> lg);
+  const bool in = p < A.n[blockIdx.y];
+  int4 q0 = make_int4(0, -1, -1, -1), q1 = make_int4(-1, -1, -1, -1);
+  if (in) {
+    const int4* rec = reinterpret_cast<const int4*>(B.rec + A.rec[blockIdx.y] + p);
+    q0 = rec[0];
+    q1 = rec[1];
+  }
+  pdl_trigger();
+  pdl_wait();
+  if (!in) return;
+  for (int r = (int)(e & ((1u << lg) - 1)) * V; r < R; r += V << lg) {
+    const T* w = st.w + r;
+    T v[V], u[4][V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      v[i] = T(0);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) u[j][i] = T(0);
+    }
+    if (q0.x >= 0) ld_rhs<V>(st.b + (size_t)q0.x * R + r, v);
+    if (q0.y >= 0) ld_rhs<V>(w + (size_t)q0.y * R, u[0]);
+    if (q0.z >= 0) ld_rhs<V>(w + (size_t)q0.z * R, u[1]);
+    if (q0.w >= 0) ld_rhs<V>(w + (size_t)q0.w * R, u[2]);
+    if (q1.x >= 0) ld_rhs<V>(w + (size_t)q1.x * R, u[3]);
+    const T sign = q0.x >= 0 ? T(-1) : T(1);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int i = 0; i < V; ++i) v[i] += sign * u[j][i];
+    auto add = [&](int slot) {
+      T t[V];
+      ld_rhs<V>(w + (size_t)slot * R, t);
+#pragma unroll
+      for (int i = 0; i < V; ++i) v[i] += sign * t[i];
+    };
+    if (q1.y >= 0) {  // few positions have so many children
+      add(q1.y);
+      if (q1.z >= 0) add(q1.z);
+      if (q1.w >= 0) add(q1.w);
+      if (q1.w < -1) {
+        const int* m = B.more + (-2 - q1.w);
+        for (int j = 1; j <= m[0]; ++j) add(m[j]);
+      }
+    }
+    st_rhs<V>(q0.x >= 0 ? st.x + (size_t)q0.x * R + r : st.w + (size_t)(~q0.x) * R + r, v);
+  }
 }
 
 // Leaf levels: a warp per node (all of its rows) and right-hand-side chunk,
@@ -651,13 +907,11 @@ __global__ void __launch_bounds__(kSolveThreads, 3)
     if (e.x == 0) {
       const int4 sy = F.sync[e.y];
       panel_tile<T, RPL, FWD, SVT>(
-          B, S, F.items[e.y], rc0, e.w, P, nullptr, nullptr, 0, 0, smem_raw,
-          [&] {
+          B, S, F.items[e.y], rc0, P, smem_raw, [&] {
             if (tid == 0) s_ok = sy.x < 0 || flow_wait(F.ctr + sy.x, sy.y, F.err);
             __syncthreads();
             return s_ok != 0;
-          },
-          [] {});
+          });
       if (tid == 0) pending = sy.z;
     } else if (warp < e.z) {
       const int ii = e.y + warp;
@@ -703,185 +957,140 @@ void launch_flow(bool forward, const BankView& B, const SVT& S, const FlowPlan& 
   PECS_CUDA(cudaGetLastError());
 }
 
-// Tile shape of one level for nrhs right-hand sides: the longest row tiles and
-// the most right-hand sides per lane that still give the GPU two CTAs per SM.
-// Fewer right-hand sides per CTA is tried first (it keeps the staged columns
-// per output value higher than shorter row tiles do).
-struct PanelChoice {
-  int cap_idx, rpl;
-};
-
-PanelChoice choose_panel(const PanelPlan& L, int max_nrhs, int rpl_max, int min_ctas) {
-  static const int order[6][2] = {{0, 4}, {0, 2}, {0, 1}, {1, 1}, {2, 1}, {3, 1}};
-  PanelChoice best{0, 1};
-  long long best_ctas = -1;
-  for (auto& o : order) {
-    if (o[1] > rpl_max) continue;
-    const long long ctas = (long long)L.tiles[o[0]].n_items * ((max_nrhs + 32 * o[1] - 1) / (32 * o[1]));
-    if (ctas >= min_ctas) return PanelChoice{o[0], o[1]};
-    if (ctas > best_ctas) {
-      best_ctas = ctas;
-      best = PanelChoice{o[0], o[1]};
-    }
-  }
-  return best;
+template <typename T, typename SVT>
+void set_panel_smem_limit() {
+  auto set = [&](const void* fn, size_t lim) {
+    PECS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim));
+  };
+  set((const void*)k_panel_tiles<T, true, SVT>, kTileSmem);
+  set((const void*)k_panel_tiles<T, false, SVT>, kTileSmem);
 }
 
-template <typename T, int RPL, typename SVT>
-void launch_panel(bool forward, const BankView& B, const SVT& S, const PanelPlan& L,
-                  const PanelTiles& P, int max_nrhs, int kcap, int parts_ld, cudaStream_t st) {
-  const int ychunks = (parts_ld + 31) / 32;
-  if (P.n_items == 0) return;
-  constexpr int RC = 32 * RPL;
-  const int meta = forward ? L.max_s + L.max_f + 1 + L.cm_cap : L.max_f;
-  // columns per chunk: the tuned cap, halved until the chunk's staging fits
-  int ci = 0;
-  while (ci + 1 < kPanelKcSteps && (kPanelKc[ci] > kcap || kPanelKc[ci + 1] >= std::max(1, L.max_k))) ++ci;
-  size_t smem = 0;
-  int kc = 1, ds_rows = 32, sc_rows = 0, nbuf = 1;
-  for (;; ++ci) {
-    kc = std::min(kPanelKc[ci], std::max(1, L.max_k));
-    nbuf = 1;  // level launches: single-buffered (measured faster: more CTAs per SM)
-    ds_rows = P.min_ri < 32 ? std::max(kc, 32 / nbuf) : kc;
-    sc_rows = forward ? L.sc_rows[ci] : 0;
-    smem = panel_smem_bytes<T>(ds_rows, RC, kc, P.max_ri, sc_rows, meta, nbuf);
-    if (smem <= kPanelSmem || ci + 1 == kPanelKcSteps) break;
-  }
-  if (smem > kPanelSmem) throw PecsError(PECS_E_ARG, "panel staging exceeds shared memory");
-  const dim3 grid(P.n_items, (max_nrhs + RC - 1) / RC);
+// launches with programmatic stream serialisation
+template <typename... P, typename... A>
+void launch_pdl(void (*fn)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
-  cfg.blockDim = dim3(kSolveThreads);
+  cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  T* parts = reinterpret_cast<T*>(L.partials.p);
-  const PanelShape shape{kc, ds_rows, P.max_ri, sc_rows, L.max_s, L.max_f, L.cm_cap, nbuf};
-  if (forward)
-    PECS_CUDA(cudaLaunchKernelEx(&cfg, k_panel<T, RPL, true, SVT>, B, S, (const PanelItem*)P.items.p, shape,
-                                 parts, L.counters.p, parts_ld, ychunks));
-  else
-    PECS_CUDA(cudaLaunchKernelEx(&cfg, k_panel<T, RPL, false, SVT>, B, S, (const PanelItem*)P.items.p, shape,
-                                 parts, L.counters.p, parts_ld, ychunks));
+  PECS_CUDA(cudaLaunchKernelEx(&cfg, fn, args...));
 }
 
-template <typename T, typename SVT>
-void set_panel_smem_limit() {
-  const int lim = (int)kPanelSmem;
-  auto set = [&](const void* fn) {
-    PECS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
-  };
-  set((const void*)k_panel<T, 1, true, SVT>);
-  set((const void*)k_panel<T, 2, true, SVT>);
-  set((const void*)k_panel<T, 4, true, SVT>);
-  set((const void*)k_panel<T, 1, false, SVT>);
-  set((const void*)k_panel<T, 2, false, SVT>);
-  set((const void*)k_panel<T, 4, false, SVT>);
-  set((const void*)k_panel_warp<T, 1, true, SVT>);
-  set((const void*)k_panel_warp<T, 2, true, SVT>);
-  set((const void*)k_panel_warp<T, 4, true, SVT>);
-  set((const void*)k_panel_warp<T, 1, false, SVT>);
-  set((const void*)k_panel_warp<T, 2, false, SVT>);
-  set((const void*)k_panel_warp<T, 4, false, SVT>);
+// Shared memory of a level's tiles: the columns of its longest tile at once where
+// they fit kTileOnce (two CTAs on a multiprocessor), else in two buffers.
+template <typename T>
+TileShape tile_shape(const PanelLevel& L, const PanelOption& o, int chunk, size_t& smem) {
+  const int bn = 32 * o.n, kgroups = o.warps / o.n;
+  const size_t col = (size_t)(L.pad + bn) * sizeof(T);
+  TileShape P{};
+  P.lg_nw = o.n == 4 ? 2 : (o.n == 2 ? 1 : 0);
+  P.kc = L.cols;
+  if (chunk > 0) P.kc = std::min(P.kc, chunk);
+  if ((size_t)P.kc * col > kTileOnce) P.kc = std::max(1, (int)(kTileBuffer / col));
+  const int nbuf = P.kc < L.cols ? 2 : 1;
+  P.a = 16 + (unsigned)(((L.cols + 3) & ~3) + 32) * 4;
+  P.a_buf = (unsigned)((size_t)P.kc * L.pad * sizeof(T));
+  P.b = P.a + nbuf * P.a_buf;
+  P.b_buf = (unsigned)((size_t)P.kc * bn * sizeof(T));
+  size_t end = P.b + (size_t)nbuf * P.b_buf;
+  if (kgroups > 1) end = std::max(end, P.a + (size_t)kgroups * L.pad * bn * sizeof(T));
+  P.p = (unsigned)end;
+  if (L.passes) end += (size_t)L.pad * bn * sizeof(T);
+  smem = end;
+  return P;
+}
+
+template <typename T, bool FWD, typename SVT>
+void launch_tiles(const TilesView& B, const SVT& S, int n_sets, const PanelPlan& L, const PanelOption& o,
+                  int max_nrhs, int chunk, cudaStream_t st) {
+  if (FWD && L.assembled) {
+    AsmSets A{};
+    int most = 0;
+    bool vec = true;
+    constexpr int V = 16 / (int)sizeof(T);
+    for (int q = 0; q < n_sets; ++q) {
+      A.rec[q] = L.tiles.rec[q], A.n[q] = L.tiles.n_rec[q];
+      most = std::max(most, A.n[q]);
+      vec = vec && S.set[q].nrhs % V == 0;
+    }
+    int lg = 3;  // threads per position
+    while (lg < 8 && ((vec ? V : 1) << lg) < max_nrhs) ++lg;
+    const dim3 grid((unsigned)((((long long)most << lg) + kSolveThreads - 1) / kSolveThreads), n_sets);
+    launch_pdl(vec ? k_panel_assemble<T, V, SVT> : k_panel_assemble<T, 1, SVT>, grid, kSolveThreads, 0, st, B, S, A, lg);
+  }
+  size_t smem = 0;
+  const TileShape P = tile_shape<T>(L.tiles, o, chunk, smem);
+  if (smem > kTileSmem) throw PecsError(PECS_E_ARG, "panel staging exceeds shared memory");
+  const int rc = 32 * o.n;
+  launch_pdl(k_panel_tiles<T, FWD, SVT>, dim3(L.tiles.n, (max_nrhs + rc - 1) / rc), 32 * o.warps, smem, st, B, S,
+             L.tiles.first, P);
 }
 
 template <typename T, int RPL, typename SVT>
 void launch_panel_warp(bool forward, const BankView& B, const SVT& S, const PanelPlan& L,
                        int max_nrhs, cudaStream_t st) {
   constexpr int RC = 32 * RPL;
-  const int rows_pad = (L.warp_rows + 3) & ~3;
+  const int rows_pad = (L.warp_rows + 3) & ~3, n = (int)L.warp.n;
   const size_t smem = kWarpNodesPerCta * panel_warp_bytes<T>(L.max_k, rows_pad, RC);
-  const dim3 grid((L.warp.n_items + kWarpNodesPerCta - 1) / kWarpNodesPerCta, (max_nrhs + RC - 1) / RC);
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(kSolveThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (forward)
-    PECS_CUDA(cudaLaunchKernelEx(&cfg, k_panel_warp<T, RPL, true, SVT>, B, S, (const PanelItem*)L.warp.items.p,
-                                 L.warp.n_items, L.max_k, rows_pad));
-  else
-    PECS_CUDA(cudaLaunchKernelEx(&cfg, k_panel_warp<T, RPL, false, SVT>, B, S, (const PanelItem*)L.warp.items.p,
-                                 L.warp.n_items, L.max_k, rows_pad));
+  const dim3 grid((n + kWarpNodesPerCta - 1) / kWarpNodesPerCta, (max_nrhs + RC - 1) / RC);
+  launch_pdl(forward ? k_panel_warp<T, RPL, true, SVT> : k_panel_warp<T, RPL, false, SVT>, grid, kSolveThreads, smem, st,
+             B, S, (const PanelItem*)L.warp.p, n, L.max_k, rows_pad);
 }
 
-// One tiling option of a level: kind 0 = whole-row items (row-tile cap
-// 32 >> cap_idx), 1 = split-K items, 2 = leaf warps; rpl = RHS per lane.
+// The valid options of a level for rpl_max right-hand sides per lane.
+template <typename T>
+std::vector<PanelOption> panel_options(const PanelPlan& L, int max_nrhs, int rpl_max) {
+  std::vector<PanelOption> v;
+  if (L.warp.n > 0)
+    for (int rpl = rpl_max; rpl >= 1; rpl /= 2) {
+      const int rows_pad = (L.warp_rows + 3) & ~3;
+      if (kWarpNodesPerCta * panel_warp_bytes<T>(L.max_k, rows_pad, 32 * rpl) <= kWarpSmem)
+        v.push_back(PanelOption{2, 8, rpl});
+    }
+  for (int n = 4; n >= 1; n /= 2)
+    for (int warps : {8, 4})
+      if (n == 1 || 16 * n < max_nrhs) v.push_back(PanelOption{0, warps, n});
+  return v;
+}
+
+// Untuned banks: leaf warps where the level has them; else the most right-hand sides per
+// CTA that give every multiprocessor two.
+template <typename T>
+PanelOption panel_default_option(const PanelPlan& L, int max_nrhs, int rpl_max, const PanelTuning& tu) {
+  if (L.warp.n > 0) {
+    int rpl = rpl_max;
+    const int rows_pad = (L.warp_rows + 3) & ~3;
+    while (rpl > 1 && kWarpNodesPerCta * panel_warp_bytes<T>(L.max_k, rows_pad, 32 * rpl) > kWarpSmem) rpl /= 2;
+    return PanelOption{2, 8, rpl};
+  }
+  int n = max_nrhs > 64 ? 4 : (max_nrhs > 32 ? 2 : 1);
+  while (n > 1 && (long long)L.tiles.n * ((max_nrhs + 32 * n - 1) / (32 * n)) < 2 * tu.min_ctas) n /= 2;
+  return PanelOption{0, 8, n};
+}
+
 template <typename T, typename SVT>
-void launch_panel_option(const PanelOption& o, bool forward, const BankView& B, const SVT& S,
-                         const PanelPlan& L, int max_nrhs, const PanelTuning& tu, int parts_ld,
-                         cudaStream_t st) {
+void launch_panel_level(bool forward, const BankView& B, const TilesView& V, const SVT& S, int n_sets,
+                        const PanelPlan& L, int max_nrhs, int rpl_max, const PanelTuning& tu, cudaStream_t st) {
+  if (L.tiles.n == 0) return;
+  PanelOption o = L.tuned;
+  if (o.kind < 0 || (o.kind == 2 && o.n > rpl_max)) o = panel_default_option<T>(L, max_nrhs, rpl_max, tu);
   if (o.kind == 2) {
-    switch (o.rpl) {
+    switch (o.n) {
       case 1: launch_panel_warp<T, 1, SVT>(forward, B, S, L, max_nrhs, st); break;
       case 2: launch_panel_warp<T, 2, SVT>(forward, B, S, L, max_nrhs, st); break;
       default: launch_panel_warp<T, 4, SVT>(forward, B, S, L, max_nrhs, st); break;
     }
-    return;
+  } else if (forward) {
+    launch_tiles<T, true, SVT>(V, S, n_sets, L, o, max_nrhs, tu.chunk, st);
+  } else {
+    launch_tiles<T, false, SVT>(V, S, n_sets, L, o, max_nrhs, tu.chunk, st);
   }
-  const PanelTiles& P = o.kind == 1 ? L.split : L.tiles[o.cap_idx];
-  switch (o.rpl) {
-    case 1: launch_panel<T, 1, SVT>(forward, B, S, L, P, max_nrhs, tu.chunk, parts_ld, st); break;
-    case 2: launch_panel<T, 2, SVT>(forward, B, S, L, P, max_nrhs, tu.chunk, parts_ld, st); break;
-    default: launch_panel<T, 4, SVT>(forward, B, S, L, P, max_nrhs, tu.chunk, parts_ld, st); break;
-  }
-}
-
-// The valid options of a level for rpl_max RHS per lane.
-template <typename T>
-std::vector<PanelOption> panel_options(const PanelPlan& L, int max_nrhs, int rpl_max, int parts_ld) {
-  std::vector<PanelOption> v;
-  for (int rpl = rpl_max; rpl >= 1; rpl /= 2) {
-    if (L.warp.n_items > 0) {
-      const int rows_pad = (L.warp_rows + 3) & ~3;
-      if (kWarpNodesPerCta * panel_warp_bytes<T>(L.max_k, rows_pad, 32 * rpl) <= kWarpSmem)
-        v.push_back(PanelOption{2, 0, rpl});
-    }
-    for (int ci = 0; ci < 4; ++ci) v.push_back(PanelOption{0, ci, rpl});
-    if (L.split.n_items > 0 && max_nrhs <= parts_ld) v.push_back(PanelOption{1, 0, rpl});
-  }
-  return v;
-}
-
-// Heuristic option (untuned banks): leaf warps where the level has them; else
-// split-K when full-height tiles give too few CTAs; else the row-tile height
-// and RHS per lane of choose_panel.
-template <typename T>
-PanelOption panel_default_option(const PanelPlan& L, int max_nrhs, int rpl_max, const PanelTuning& tu,
-                                 int parts_ld) {
-  if (L.warp.n_items > 0) {
-    int rpl = rpl_max;
-    const int rows_pad = (L.warp_rows + 3) & ~3;
-    while (rpl > 1 && kWarpNodesPerCta * panel_warp_bytes<T>(L.max_k, rows_pad, 32 * rpl) > kWarpSmem) rpl /= 2;
-    return PanelOption{2, 0, rpl};
-  }
-  const long long full_tiles = (long long)L.tiles[0].n_items * ((max_nrhs + 31) / 32);
-  if (L.split.n_items > 0 && full_tiles < tu.min_ctas && max_nrhs <= parts_ld) {
-    int rpl = rpl_max;
-    while (rpl > 1 && (long long)L.split.n_items * ((max_nrhs + 32 * rpl - 1) / (32 * rpl)) < tu.min_ctas)
-      rpl /= 2;
-    return PanelOption{1, 0, rpl};
-  }
-  const PanelChoice c = choose_panel(L, max_nrhs, rpl_max, tu.min_ctas);
-  return PanelOption{0, c.cap_idx, c.rpl};
-}
-
-template <typename T, typename SVT>
-void launch_panel_level(bool forward, const BankView& B, const SVT& S, const PanelPlan& L,
-                        int max_nrhs, int rpl_max, const PanelTuning& tu, int parts_ld,
-                        cudaStream_t st) {
-  PanelOption o = L.tuned;
-  if (o.kind < 0 || o.rpl > rpl_max) o = panel_default_option<T>(L, max_nrhs, rpl_max, tu, parts_ld);
-  launch_panel_option<T, SVT>(o, forward, B, S, L, max_nrhs, tu, parts_ld, st);
 }
 }  // namespace
 
@@ -974,7 +1183,6 @@ FlowPlanHost plan_flow(const FlowNodes& nd, bool forward, int top, int rpl, int 
       if (warp_level[l]) {
         it.a = make_int4(g, 0, rows, 32);
         it.d = make_int4(nd.cm_off[g], cb, 0, 0);
-        it.e = make_int4(0, 0, -1, 1);
         H.items.push_back(it);
         H.sync.push_back(sy);
         continue;
@@ -1001,7 +1209,7 @@ FlowPlanHost plan_flow(const FlowNodes& nd, bool forward, int top, int rpl, int 
       H.ri_max = std::max(H.ri_max, ri);
       min_ri = std::min(min_ri, ri);
       it.d = make_int4(nd.cm_off[g], cb, ncm, 0);
-      it.e = make_int4(kc, 0, -1, 1);  // no split; this node's chunk width
+      it.kc = kc;
       for (int r0 = 0; r0 < rows; r0 += per) {
         it.a = make_int4(g, r0, std::min(rows, r0 + per), ri);
         H.items.push_back(it);
@@ -1048,18 +1256,23 @@ BankView FactorBank::view() const {
   return v;
 }
 
+TilesView FactorBank::tiles_view(int d) const {
+  return TilesView{tiles_[d].p, prec_ == PECS_PREC_FP64 ? (const void*)tval64_[d].p : (const void*)tval32_[d].p,
+                   tidx_[d].p, rec_.p, more_.p};
+}
+
 int FactorBank::kernel_launches_per_solve() const {
   if (!panel_) return rows_.launches_per_solve(max_nrhs_);
   if (flow_sel_ >= 0) {
     const int top = flow_cfg_[flow_sel_].top;
     int n = 2;
-    for (size_t l = 0; l + top < pfwd_.size(); ++l) n += pfwd_[l].tiles[0].n_items > 0;
-    for (size_t l = top; l < pbwd_.size(); ++l) n += pbwd_[l].tiles[0].n_items > 0;
+    for (size_t l = 0; l + top < pfwd_.size(); ++l) n += pfwd_[l].launches();
+    for (size_t l = top; l < pbwd_.size(); ++l) n += pbwd_[l].launches();
     return n;
   }
   int n = 0;
-  for (auto& l : pfwd_) n += l.tiles[0].n_items > 0;
-  for (auto& l : pbwd_) n += l.tiles[0].n_items > 0;
+  for (auto& l : pfwd_) n += l.launches();
+  for (auto& l : pbwd_) n += l.launches();
   return n;
 }
 
@@ -1070,11 +1283,8 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
   prec_ = precision;
   panel_ = panel;
   tune_ = tuning;
-  parts_ld_ = std::max(32, max_nrhs);
   if (tune_.chunk < 0 || tune_.chunk > 128 || tune_.min_ctas < 0)
     throw PecsError(PECS_E_ARG, "panel tuning out of range");
-  if (tune_.chunk == 0) tune_.chunk = precision == PECS_PREC_FP64 ? kPanelKcF64 : kPanelKcF32;
-  if (prec_ == PECS_PREC_FP64) tune_.chunk = std::min(tune_.chunk, kPanelKcF64);
   if (tune_.min_ctas == 0) tune_.min_ctas = kTargetCtas;
   n_sets_ = (int)factors.size();
   max_nrhs_ = max_nrhs;
@@ -1156,12 +1366,13 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
       }
       cmap_ptr.push_back((int)cmap_idx.size());
       if ((int)fl.size() <= nd.height) fl.resize(nd.height + 1);
-      if ((int)bl.size() <= nd.depth) bl.resize(nd.depth + 1);
       fl[nd.height].nodes.push_back(base + j);
-      bl[nd.depth].nodes.push_back(base + j);
     }
     base += N;
   }
+  // backward: from the greatest height down (a parent is higher than its children).
+  // Levels by depth mix cell blocks of 8 rows with separators of hundreds.
+  bl.assign(fl.rbegin(), fl.rend());
   entries_ = go + ho;
   s_.upload(hs);
   m_.upload(hm);
@@ -1187,159 +1398,60 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
     bytes_ = (long long)(G.size() + H.size()) * 4;
   }
   {
-    // panel items: a node's rows in tiles of ri <= cap rows, for caps 32, 16,
-    // 8 and 4 (levels that would not fill the GPU use shorter tiles: more
-    // CTAs, column parts per warp)
-    auto make_panel = [&](const std::vector<LevelNodes>& lv, bool forward, std::vector<PanelPlan>& out) {
+    // level plans: tiles of packed values (panel_plan.hpp), and leaf warps
+    const PanelTilesPlan H = plan_panel(factors, (std::max(1, max_nrhs) + 31) / 32, tune_.min_ctas);
+    const int esz = prec_ == PECS_PREC_FP64 ? 8 : 4;
+    rec_.upload(H.rec);
+    more_.upload(H.more);
+    for (int d = 0; d < 2; ++d) {
+      const bool forward = d == 0;
+      const PanelTilesPlan::Dir& D = H.dir[d];
+      tiles_[d].upload(D.tiles);
+      tidx_[d].upload(D.idx);
+      if (prec_ == PECS_PREC_FP64) {
+        std::vector<double> v(D.n_values);
+        pack_panel(H, factors, d, v.data());
+        tval64_[d].upload(v);
+      } else {
+        std::vector<float> v(D.n_values);
+        pack_panel(H, factors, d, v.data());
+        tval32_[d].upload(v);
+      }
+      std::vector<PanelPlan>& out = forward ? pfwd_ : pbwd_;
+      const std::vector<LevelNodes>& lv = forward ? fl : bl;
       out.clear();
       out.resize(lv.size());
       for (size_t l = 0; l < lv.size(); ++l) {
-        int max_k = 0, max_s = 1, max_f = 1, max_cm = 0;
-        for (int g : lv[l].nodes) {
-          const int f = hs[g] + hm[g];
-          max_k = std::max(max_k, forward ? hs[g] : f);
-          max_s = std::max(max_s, hs[g]);
-          max_f = std::max(max_f, f);
-          max_cm = std::max(max_cm, cmap_ptr[cm_off[g] + f] - cmap_ptr[cm_off[g]]);
-        }
-        out[l].max_k = max_k;
-        out[l].max_s = max_s;
-        out[l].max_f = max_f;
-        out[l].cm_cap = std::min(max_cm, kPanelCmMax);
-        // forward: most child-update rows landing on one chunk of columns
-        for (int ci = 0; ci < kPanelKcSteps; ++ci) {
-          int mx = 0;
-          if (forward) {
-            const int kc = kPanelKc[ci];
-            for (int g : lv[l].nodes) {
-              const int* cp = cmap_ptr.data() + cm_off[g];
-              for (int k0 = 0; k0 < hs[g]; k0 += kc) mx = std::max(mx, cp[std::min(k0 + kc, hs[g])] - cp[k0]);
-            }
-          }
-          out[l].sc_rows[ci] = mx;
-        }
-        // split-K items: nodes with long rows in 32-row tiles x column parts
-        // of kSplitPart (at most kSplitMaxParts); shorter nodes of the level
-        // as whole-row items
-        if (max_k >= kSplitMinK) {
-          std::vector<PanelItem> items;
-          int max_ri = 4, min_ri = 32, tiles = 0;
-          for (int g : lv[l].nodes) {
-            const int rows = forward ? hs[g] + hm[g] : hs[g];
-            const int K = forward ? hs[g] : hs[g] + hm[g];
-            const int nit = (rows + 31) / 32;
-            const int per = (rows + nit - 1) / nit;
-            int ri = 4;
-            while (ri < per) ri *= 2;
-            max_ri = std::max(max_ri, ri);
-            min_ri = std::min(min_ri, ri);
-            const long long off = forward ? goff[g] : hoff[g];
-            const int cb = cmap_ptr[cm_off[g]];
-            const int ncm = cmap_ptr[cm_off[g] + hs[g] + hm[g]] - cb;
-            int parts = 1, part_len = K;
-            if (K >= kSplitMinK) {
-              parts = std::min(kSplitMaxParts, (K + kSplitPart - 1) / kSplitPart);
-              part_len = ((K + parts - 1) / parts + kSplitPart - 1) / kSplitPart * kSplitPart;
-              parts = (K + part_len - 1) / part_len;
-            }
-            for (int r0 = 0; r0 < rows; r0 += per) {
-              const int tile = parts > 1 ? tiles++ : -1;
-              for (int p = 0; p < parts; ++p) {
-                PanelItem it;
-                it.a = make_int4(g, r0, std::min(rows, r0 + per), ri);
-                it.b = make_int4(hs[g], hm[g], node_set[g], w_off[g]);
-                it.c = make_int4((int)(off & 0xffffffffll), (int)(off >> 32), own_off[g], upd_off[g]);
-                it.d = make_int4(cm_off[g], cb, ncm, p);
-                it.e = make_int4(p * part_len, std::min(K, (p + 1) * part_len), tile, parts);
-                items.push_back(it);
-              }
-            }
-          }
-          if (tiles > 0) {
-            PanelTiles& P = out[l].split;
-            P.n_items = (int)items.size();
-            P.max_ri = max_ri;
-            P.min_ri = min_ri;
-            for (const PanelItem& it : items) P.max_span = std::max(P.max_span, it.e.y - it.e.x);
-            P.items.upload(items);
-            out[l].split_tiles = tiles;
-            const int ych = (parts_ld_ + 31) / 32;
-            out[l].counters.alloc((size_t)tiles * ych);
-            out[l].counters.zero();
-            const size_t esz = prec_ == PECS_PREC_FP64 ? 8 : 4;
-            out[l].partials.alloc((size_t)tiles * kSplitMaxParts * 32 * parts_ld_ * esz);
-          }
-        }
+        PanelPlan& L = out[l];
+        L.tiles = D.levels[l];
+        for (int q = 0; q < n_sets_; ++q) L.assembled = L.assembled || (forward && L.tiles.n_rec[q] > 0);
         // leaf level: every node small and, forward, without children
         bool leaf = true;
-        int max_rows = 0;
         for (int g : lv[l].nodes) {
           const int f = hs[g] + hm[g];
           const int rows = forward ? f : hs[g];
           const int k = forward ? hs[g] : f;
           const bool kids = cmap_ptr[cm_off[g] + f] > cmap_ptr[cm_off[g]];
           if (k > kWarpMaxK || rows > kWarpMaxRows || (forward && kids)) leaf = false;
-          max_rows = std::max(max_rows, rows);
+          L.max_k = std::max(L.max_k, k);
+          L.warp_rows = std::max(L.warp_rows, rows);
         }
-        {
-          const size_t esz = prec_ == PECS_PREC_FP64 ? 8 : 4;
-          const size_t rows_pad = (size_t)((max_rows + 3) & ~3);
-          const size_t wb = (((size_t)max_k * 32 + (size_t)max_k * rows_pad) * esz + (size_t)max_k * 4 + 15) & ~(size_t)15;
-          if (kWarpNodesPerCta * wb > kWarpSmem) leaf = false;
+        const size_t rows_pad = (size_t)((L.warp_rows + 3) & ~3);
+        const size_t wb = (((size_t)L.max_k * 32 + (size_t)L.max_k * rows_pad) * esz + (size_t)L.max_k * 4 + 15) & ~(size_t)15;
+        if (!leaf || kWarpNodesPerCta * wb > kWarpSmem) continue;
+        std::vector<PanelItem> items;
+        for (int g : lv[l].nodes) {
+          const long long off = forward ? goff[g] : hoff[g];
+          PanelItem it;
+          it.a = make_int4(g, 0, forward ? hs[g] + hm[g] : hs[g], 32);
+          it.b = make_int4(hs[g], hm[g], node_set[g], w_off[g]);
+          it.c = make_int4((int)(off & 0xffffffffll), (int)(off >> 32), own_off[g], upd_off[g]);
+          it.d = make_int4(cm_off[g], cmap_ptr[cm_off[g]], 0, 0);
+          items.push_back(it);
         }
-        if (leaf) {
-          std::vector<PanelItem> items;
-          for (int g : lv[l].nodes) {
-            const int rows = forward ? hs[g] + hm[g] : hs[g];
-            const long long off = forward ? goff[g] : hoff[g];
-            PanelItem it;
-            it.a = make_int4(g, 0, rows, 32);
-            it.b = make_int4(hs[g], hm[g], node_set[g], w_off[g]);
-            it.c = make_int4((int)(off & 0xffffffffll), (int)(off >> 32), own_off[g], upd_off[g]);
-            it.d = make_int4(cm_off[g], cmap_ptr[cm_off[g]], 0, 0);
-            it.e = make_int4(0, 0, -1, 1);
-            items.push_back(it);
-          }
-          out[l].warp.n_items = (int)items.size();
-          out[l].warp.items.upload(items);
-          out[l].warp_rows = max_rows;
-        }
-        for (int ci = 0; ci < 4; ++ci) {
-          const int cap = 32 >> ci;
-          std::vector<PanelItem> items;
-          int max_ri = 4, min_ri = 32;
-          for (int g : lv[l].nodes) {
-            const int rows = forward ? hs[g] + hm[g] : hs[g];
-            const int nit = (rows + cap - 1) / cap;
-            const int per = (rows + nit - 1) / nit;
-            int ri = 4;
-            while (ri < per) ri *= 2;
-            max_ri = std::max(max_ri, ri);
-            min_ri = std::min(min_ri, ri);
-            const long long off = forward ? goff[g] : hoff[g];
-            const int cb = cmap_ptr[cm_off[g]];
-            const int ncm = cmap_ptr[cm_off[g] + hs[g] + hm[g]] - cb;
-            for (int r0 = 0; r0 < rows; r0 += per) {
-              PanelItem it;
-              it.a = make_int4(g, r0, std::min(rows, r0 + per), ri);
-              it.b = make_int4(hs[g], hm[g], node_set[g], w_off[g]);
-              it.c = make_int4((int)(off & 0xffffffffll), (int)(off >> 32), own_off[g], upd_off[g]);
-              it.d = make_int4(cm_off[g], cb, ncm, 0);
-              it.e = make_int4(0, 0, -1, 1);  // no split
-              items.push_back(it);
-            }
-          }
-          PanelTiles& P = out[l].tiles[ci];
-          P.n_items = (int)items.size();
-          P.max_ri = max_ri;
-          P.min_ri = min_ri;
-          P.max_span = max_k;
-          P.items.upload(items);
-        }
+        L.warp.upload(items);
       }
-    };
-    make_panel(fl, true, pfwd_);
-    make_panel(bl, false, pbwd_);
+    }
     if (prec_ == PECS_PREC_FP64)
       set_panel_smem_limit<double, IlSetsView>();
     else
@@ -1367,7 +1479,6 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
     FlowNodes nodes{hs, hm, node_set, w_off, own_off, upd_off, cm_off, cmap_ptr, goff, hoff, parent, {}, {}};
     for (auto& l : fl) nodes.by_height.push_back(l.nodes);
     for (auto& l : bl) nodes.by_depth.push_back(l.nodes);
-    const int esz = prec_ == PECS_PREC_FP64 ? 8 : 4;
     flow_cfg_.clear();
     flow_sel_ = -1;
     const int n_levels = (int)std::max(fl.size(), bl.size());
@@ -1379,7 +1490,7 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
         for (int rpl : {1, 2, 4}) {
           FlowConfig cfg;
           cfg.top = top;
-          cfg.kc = std::min(kc, tune_.chunk);
+          cfg.kc = tune_.chunk > 0 ? std::min(kc, tune_.chunk) : kc;
           cfg.rpl = rpl;
           bool ok = true;
           for (int d = 0; d < 2 && ok; ++d) {
@@ -1517,7 +1628,7 @@ void FactorBank::solve_flow(const SVT& sets, int max_nrhs, int cfg, cudaStream_t
   int* queue[2] = {base + 2 * (size_t)n_nodes_, base + 2 * (size_t)n_nodes_ + 1};
   int* err = base + 2 * (size_t)n_nodes_ + 2;
   for (size_t l = 0; l + C.top < pfwd_.size(); ++l)
-    launch_panel_level<T, SVT>(true, B, sets, pfwd_[l], max_nrhs, lrpl, tune_, parts_ld_, st);
+    launch_panel_level<T, SVT>(true, B, tiles_view(0), sets, n_sets_, pfwd_[l], max_nrhs, lrpl, tune_, st);
   for (int d = 0; d < 2; ++d) {
     const FlowPlan& FP = C.plan[d];
     const FlowView F{FP.entries.p, FP.items.p, FP.sync.p, ctr[d], ctr[1 - d], n_nodes_,
@@ -1529,7 +1640,7 @@ void FactorBank::solve_flow(const SVT& sets, int max_nrhs, int cfg, cudaStream_t
     }
   }
   for (size_t l = C.top; l < pbwd_.size(); ++l)
-    launch_panel_level<T, SVT>(false, B, sets, pbwd_[l], max_nrhs, lrpl, tune_, parts_ld_, st);
+    launch_panel_level<T, SVT>(false, B, tiles_view(1), sets, n_sets_, pbwd_[l], max_nrhs, lrpl, tune_, st);
 }
 
 template <typename SVT>
@@ -1544,9 +1655,9 @@ void FactorBank::solve_panel(const SVT& sets, int max_nrhs, cudaStream_t st) con
     const bool fwd = pass == 0;
     for (const PanelPlan& L : fwd ? pfwd_ : pbwd_) {
       if constexpr (std::is_same<SVT, IlSetsViewF>::value)
-        launch_panel_level<float, SVT>(fwd, B, sets, L, max_nrhs, rpl, tune_, parts_ld_, st);
+        launch_panel_level<float, SVT>(fwd, B, tiles_view(pass), sets, n_sets_, L, max_nrhs, rpl, tune_, st);
       else
-        launch_panel_level<double, SVT>(fwd, B, sets, L, max_nrhs, rpl, tune_, parts_ld_, st);
+        launch_panel_level<double, SVT>(fwd, B, tiles_view(pass), sets, n_sets_, L, max_nrhs, rpl, tune_, st);
     }
   }
 }
@@ -1601,7 +1712,7 @@ void FactorBank::autotune_panel(const SVT& sets, int max_nrhs, cudaStream_t st, 
   PECS_CUDA(cudaEventCreate(&e1));
   for (int pass = 0; pass < 2; ++pass)
     for (PanelPlan& L : pass == 0 ? pfwd_ : pbwd_)
-      L.tuned = panel_default_option<T>(L, max_nrhs, rpl, tune_, parts_ld_);
+      L.tuned = panel_default_option<T>(L, max_nrhs, rpl, tune_);
   auto time_sweep = [&]() {
     const int per_sweep = kernel_launches_per_solve();
     float best = 1e30f;
@@ -1624,8 +1735,8 @@ void FactorBank::autotune_panel(const SVT& sets, int max_nrhs, cudaStream_t st, 
     for (PanelPlan& L : pass == 0 ? pfwd_ : pbwd_) {
       const PanelOption keep = L.tuned;
       PanelOption best = keep;
-      for (const PanelOption& o : panel_options<T>(L, max_nrhs, rpl, parts_ld_)) {
-        if (o.kind == keep.kind && o.cap_idx == keep.cap_idx && o.rpl == keep.rpl) continue;
+      for (const PanelOption& o : panel_options<T>(L, max_nrhs, rpl)) {
+        if (o.kind == keep.kind && o.warps == keep.warps && o.n == keep.n) continue;
         L.tuned = o;
         float ms;
         try {
@@ -1685,7 +1796,7 @@ std::vector<double> FactorBank::time_levels(const IlSetsViewF& sets, int max_nrh
     PECS_CUDA(cudaEventRecord(ev[0], st));
     for (int pass = 0; pass < 2; ++pass)
       for (const PanelPlan& L : pass == 0 ? pfwd_ : pbwd_) {
-        launch_panel_level<float, IlSetsViewF>(pass == 0, B, sets, L, max_nrhs, rpl, tune_, parts_ld_, st);
+        launch_panel_level<float, IlSetsViewF>(pass == 0, B, tiles_view(pass), sets, n_sets_, L, max_nrhs, rpl, tune_, st);
         PECS_CUDA(cudaEventRecord(ev[++l], st));
       }
     PECS_CUDA(cudaEventSynchronize(ev[nl]));

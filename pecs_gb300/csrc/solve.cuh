@@ -6,13 +6,10 @@
 // factor (e.g. electrons and holes of every instance when their mobilities
 // are equal), so that every stored factor entry read from HBM is applied to
 // all of them.  One kernel launch processes one tree level of every factor in
-// the bank.  Banks with few right-hand sides per set apply row tiles of the blocks
-// (rows.cuh); a bank built for many right-hand sides per set ("panel" banks)
-// stores every block column-major and applies each node as a
-// small dense GEMM: a CTA stages a chunk of columns of the right-hand sides
-// (interleaved layout: a dof's values are contiguous) and of the block in
-// shared memory, each warp accumulates a 4-row x (32 * RPL)-RHS register tile
-// with lanes over right-hand sides, so every global access is coalesced.
+// small dense GEMM: forward, a level's columns -- right-hand side minus the children's
+// updates -- are assembled once per node, then every tile of rows takes its packed
+// values by one bulk copy and the vectors' rows (interleaved layout: a dof's values
+// are contiguous) and multiplies them in register tiles.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -20,6 +17,7 @@
 
 #include "common.hpp"
 #include "mf.hpp"
+#include "panel_plan.hpp"
 #include "rows.cuh"
 
 namespace pecs {
@@ -77,48 +75,41 @@ struct IlSetsViewF {
   IlSetViewF set[kMaxSets];
 };
 
-// One level of the panel path: items (node, row0, row1, rows per tile), one
-// CTA each; every item applies its rows of the node's block to a chunk of
-// right-hand sides held in shared memory, lanes over right-hand sides.  Items
-// are kept for row-tile caps 32, 16, 8 and 4; the launch picks one.
-// One panel item: a row range of one node and everything about the node the
-// kernel needs, so that a single round of loads starts it.
+// Device pointers of one direction's level plan.
+struct TilesView {
+  const PanelTile* tiles;
+  const void* val;
+  const int* idx;
+  const RowRec* rec;
+  const int* more;
+};
+
+// A row range of one node and everything about the node that the flow and leaf kernels
+// need, so that a single round of loads starts it.
 struct __align__(16) PanelItem {
   int4 a;  // node, row0, row1, rows per tile
   int4 b;  // s, m, RHS set, update-vector offset
   int4 c;  // block offset (low, high 32 bits), own-index offset, update-index offset
-  int4 d;  // child-map pointer offset, first child-map entry, child-map entries, K part
-  int4 e;  // split-K: first column, end column, tile (-1: no split), K parts of the tile
+  int4 d;  // child-map pointer offset, first child-map entry, child-map entries, unused
+  int kc = 0;  // staged columns per chunk
+  int unused[3];
 };
 
-struct PanelTiles {
-  int n_items = 0;
-  int max_ri = 4;   // largest rows-per-tile of the items
-  int min_ri = 32;  // smallest (< 32: column parts reduce in shared memory)
-  int max_span = 0; // most columns one item covers (> the chunk width: double-buffered staging)
-  DBuf<PanelItem> items;
-};
-
-// A tiling option of one panel level (see launch_panel_option).
+// How a panel level is launched.
 struct PanelOption {
-  int kind = -1;  // -1 untuned, 0 whole-row tiles, 1 split-K tiles, 2 leaf warps
-  int cap_idx = 0;
-  int rpl = 1;
+  int kind = -1;  // -1 untuned, 0 tiles, 2 leaf warps
+  int warps = 8;  // tiles: warps per CTA (4 or 8)
+  int n = 1;      // tiles: 32-right-hand-side groups per CTA; leaf warps: right-hand sides per lane
 };
 
 struct PanelPlan {
-  int max_k = 0;   // largest column count of the level's nodes
-  int max_s = 1, max_f = 1;
-  int cm_cap = 0;  // child-map entries staged per node (the level's largest, capped)
-  int sc_rows[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // forward: child rows per chunk, per chunk size
-  PanelTiles tiles[4];
-  PanelTiles split;   // levels with long rows: 32-row tiles split along K (else empty)
-  int split_tiles = 0;
-  DBuf<int> counters;      // split-K: arrival counter per (tile, RHS chunk); reset by the last CTA
-  DBuf<unsigned char> partials;  // split-K: [tile][part][32 rows][max RHS] partial products
-  PanelTiles warp;    // leaf levels: one item per node, a warp each (else empty)
-  int warp_rows = 0;  // leaf levels: most rows of a node
-  PanelOption tuned;  // the autotuner's choice (kind -1: heuristic)
+  PanelLevel tiles;      // panel_plan.hpp
+  bool assembled = false;  // forward: nodes with children, whose positions are assembled first
+  DBuf<PanelItem> warp;  // leaf levels: one item per node, a warp each (else empty)
+  int max_k = 0;         // leaf levels: largest column count
+  int warp_rows = 0;     // leaf levels: most rows of a node
+  PanelOption tuned;     // the autotuner's choice (kind -1: heuristic)
+  int launches() const { return tiles.n == 0 ? 0 : (assembled ? 2 : 1); }
 };
 
 // A flow sweep of one direction (one persistent launch; solve.cu): work
@@ -177,7 +168,7 @@ FlowPlanHost plan_flow(const FlowNodes& nd, bool forward, int top, int rpl, int 
                        int n_sm);
 
 struct PanelTuning {
-  int chunk = 0;     // staged block columns per chunk (0: 128 FP32, 64 FP64)
+  int chunk = 0;     // most staged block columns per chunk (0: what shared memory holds)
   int min_ctas = 0;  // CTAs a level must reach before shorter tiles are used (0: one per SM)
 };
 
@@ -249,7 +240,12 @@ class FactorBank {
   std::vector<PanelPlan> pfwd_, pbwd_;
   bool panel_ = false;
   PanelTuning tune_;
-  int parts_ld_ = 32;  // split-K scratch: right-hand sides per partial row
+  DBuf<PanelTile> tiles_[2];  // level sweeps: tiles, their values and index lists per direction
+  DBuf<double> tval64_[2];
+  DBuf<float> tval32_[2];
+  DBuf<int> tidx_[2], more_;
+  DBuf<RowRec> rec_;
+  TilesView tiles_view(int d) const;
   template <typename SVT>
   void solve_panel(const SVT& sets, int max_nrhs, cudaStream_t st) const;
   template <typename SVT>
