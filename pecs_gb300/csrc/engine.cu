@@ -1856,6 +1856,7 @@ struct LuHandle {
 namespace {
 // Loads this file's device module on device `dev` (current) and records the
 // device address of the no-alloc solve's static array; defined with it.
+constexpr int kNoAllocMaxRhs = 8;
 void noalloc_reserve(int dev);
 }  // namespace
 
@@ -2406,6 +2407,8 @@ static void lu_upload(LuHandle& h, int nrhs) {
     int dev = -1;
     PECS_CUDA(cudaGetDevice(&dev));
     noalloc_reserve(dev);
+    // nor that of a kernel, whatever its number of right-hand sides
+    h.bank.load_row_kernels(kNoAllocMaxRhs);
     h.uploaded = true;
   }
   if (nrhs > h.nrhs_cap) {
@@ -2484,7 +2487,6 @@ void pecs_lu_destroy(pecs_lu* lu) { delete lu; }
 namespace pecs {
 namespace {
 constexpr size_t kNoAllocScratchDoubles = size_t(1) << 20;  // 8 MiB
-constexpr int kNoAllocMaxRhs = 8;
 constexpr int kNoAllocMaxDevices = 64;
 static __device__ __align__(256) double g_noalloc_scratch[kNoAllocScratchDoubles];
 

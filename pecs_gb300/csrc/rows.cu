@@ -746,6 +746,21 @@ void RowsSweep::ready() const {
   ready_rb_ = RB;
 }
 
+void RowsSweep::load_kernels(int most_rhs) const {
+  auto go = [&](auto tag) {
+    using T = decltype(tag);
+    for (int n = 1, last = 0; n <= most_rhs; ++n) {
+      const int rb = choose_rb<T>(n);
+      if (rb != last) with_rb<T>(rb, [&](auto c) { ready<T, decltype(c)::value>(); });
+      last = rb;
+    }
+  };
+  if (prec_ == PECS_PREC_FP64)
+    go(double{});
+  else
+    go(float{});
+}
+
 bool RowsSweep::assembles(const RowSets& sets, int max_nrhs) const {
   for (int q = 0; q < n_sets_; ++q)
     if (!sets.set[q].d) return false;

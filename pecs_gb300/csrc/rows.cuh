@@ -60,6 +60,9 @@ class RowsSweep {
   void build(const std::vector<const MfFactor*>& factors, int precision, int max_nrhs);
   // y = forward(b), x = backward(y) for every set
   void solve(const RowSets& sets, int max_nrhs, cudaStream_t st) const;
+  // Loads the kernels of every solve of 1 to most_rhs right-hand sides without
+  // assembled columns, so that those solves load nothing themselves.
+  void load_kernels(int most_rhs) const;
   int set_wtotal(int set) const { return wtotal_[set]; }
   int dofs(int set) const { return dofs_[set]; }
   long long entries() const { return entries_; }

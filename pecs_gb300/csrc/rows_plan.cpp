@@ -59,7 +59,8 @@ template <typename F>
 void parallel(int n, F f) {
   const int threads = (int)std::max(1u, std::min(std::thread::hardware_concurrency(), 16u));
   std::atomic<int> next(0);
-  dense::run_threads(std::max(1, std::min(threads, n / 8)), [&](int) {
+  // a thread takes about as long to start as 64 nodes of a small mesh to plan
+  dense::run_threads(std::max(1, std::min(threads, n / 64)), [&](int) {
     for (int i; (i = next.fetch_add(1)) < n;) f(i);
   });
 }

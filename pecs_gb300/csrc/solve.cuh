@@ -183,6 +183,7 @@ class FactorBank {
              PanelTuning tuning = PanelTuning(), int max_nrhs = 0);
   // y = forward(b), x = backward(y); w is workspace.  All sets must be bound.
   void solve(const RowSets& sets, int max_nrhs, cudaStream_t st) const;  // few right-hand sides
+  void load_row_kernels(int most_rhs) const { rows_.load_kernels(most_rhs); }
   void solve(const IlSetsView& sets, int max_nrhs, cudaStream_t st) const;
   void solve(const IlSetsViewF& sets, int max_nrhs, cudaStream_t st) const;
   int set_wtotal(int set) const { return set_wtotal_[set]; }
