@@ -142,14 +142,29 @@ __global__ void k_scatter_il(ElemSets E, const int* __restrict__ mask, int n_ins
   }
 }
 
+// Pairs of interleaved vectors: (hi, lo) one after another, or, for the residual
+// kernel that takes right-hand sides two at a time (QUAD; R even), hi, hi, lo, lo
+// of two neighbours, so that its packed operands come straight from a load.
+template <bool QUAD>
+__device__ __forceinline__ void st_pair(float2* Xs, size_t i, float2 v) {
+  if constexpr (QUAD) {
+    float* q = reinterpret_cast<float*>(Xs) + 2 * (i & ~(size_t)1) + (i & 1);
+    q[0] = v.x;
+    q[2] = v.y;
+  } else {
+    Xs[i] = v;
+  }
+}
+
 // Xs = X as FP32 pairs
+template <bool QUAD>
 __global__ void k_split_il(ElemSets E) {
   const ElemSet& S = E.s[blockIdx.y];
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= (size_t)S.n * S.R) return;
   const double a = S.X[i];
   const float hi = __double2float_rn(a);
-  S.Xs[i] = make_float2(hi, __double2float_rn(a - (double)hi));
+  st_pair<QUAD>(S.Xs, i, make_float2(hi, __double2float_rn(a - (double)hi)));
 }
 
 // between refinements: X += D (the correction's type), X = X32 + D32, X = X32
@@ -167,42 +182,116 @@ __global__ void k_update_il(ElemSets E) {
 }
 
 // Xs[d * R + k] = old_k[d] as an FP32 pair (the previous step's solution,
-// interleaved for the residual of an increment solve)
-__global__ void k_gather_pairs_il(ElemSets E) {
+// interleaved for the residual of an increment solve).  Bound by memory: the four
+// loads of a thread are issued together (one after another, 12.6 M values took 51 us).
+template <bool QUAD>
+__global__ void __launch_bounds__(256) k_gather_pairs_il(ElemSets E) {
   const ElemSet& S = E.s[blockIdx.z];
   __shared__ double t[32][33];
   const int n = S.n, R = S.R, d0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
   if (d0 >= n || k0 >= R) return;
-  for (int kk = threadIdx.y; kk < 32; kk += blockDim.y) {
-    const int k = k0 + kk, d = d0 + threadIdx.x;
-    t[kk][threadIdx.x] = (k < R && d < n) ? S.old[k][d] : 0.0;
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  double v[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int k = k0 + ty + 8 * j;
+    v[j] = k < R && d0 + tx < n ? S.old[k][d0 + tx] : 0.0;
   }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) t[ty + 8 * j][tx] = v[j];
   __syncthreads();
-  for (int dd = threadIdx.y; dd < 32; dd += blockDim.y) {
-    const int d = d0 + dd, k = k0 + threadIdx.x;
-    if (d < n && k < R) S.Xs[(size_t)d * R + k] = d2ff(t[threadIdx.x][dd]);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int d = d0 + ty + 8 * j, k = k0 + tx;
+    if (d < n && k < R) st_pair<QUAD>(S.Xs, (size_t)d * R + k, d2ff(t[tx][ty + 8 * j]));
   }
 }
 
+// Partial sums of |new - old|^2 and |new|^2 for the steady-state test: those of
+// instance i, field slot f and chunk c at (i * 5 + f) * stride + c.
+struct ChangeSums {
+  double2* out = nullptr;
+  int stride = 0;
+  int first[kMaxSets] = {}, fields[kMaxSets] = {};  // field slots of each set's columns
+};
+
 // dst_k[d] = old_k[d] + D32[d * R + k]: the previous step's solution plus the
-// increment an increment solve found
-__global__ void k_scatter_delta_il(ElemSets E, const int* __restrict__ mask, int n_inst) {
+// increment an increment solve found.  A CTA takes 32 columns x kDeltaTiles * 32 dofs
+// and, SUMS, also adds up their changes, which it has in registers: the
+// steady-state test then reads neither state again.  Bound by memory (20 bytes per
+// value): a tile's eight loads per thread are issued before the one tile in front of
+// it is finished; each was waited for by itself before.
+constexpr int kDeltaTiles = 4;
+template <bool SUMS>
+__global__ void __launch_bounds__(256, 4) k_scatter_delta_il(ElemSets E, const int* __restrict__ mask, int n_inst,
+                                                          ChangeSums C) {
   const ElemSet& S = E.s[blockIdx.z];
-  __shared__ float t[32][33];
-  const int n = S.n, R = S.R, d0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
-  if (d0 >= n || k0 >= R) return;
-  const int nf = R / n_inst;
-  for (int dd = threadIdx.y; dd < 32; dd += blockDim.y) {
-    const int d = d0 + dd, k = k0 + threadIdx.x;
-    t[dd][threadIdx.x] = (d < n && k < R) ? S.D32[(size_t)d * R + k] : 0.f;
+  __shared__ float t[2][32][33];
+  const int n = S.n, R = S.R, k0 = blockIdx.y * 32, d00 = blockIdx.x * 32 * kDeltaTiles;
+  if (d00 >= n || k0 >= R) return;
+  const int nf = R / n_inst, tx = threadIdx.x, ty = threadIdx.y;
+  const double* old[4];
+  double* dst[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int k = min(k0 + ty + 8 * j, R - 1);
+    old[j] = S.old[k];
+    dst[j] = k0 + ty + 8 * j < R && (!mask || mask[k / nf]) ? S.dst[k] : nullptr;
   }
-  __syncthreads();
-  for (int kk = threadIdx.y; kk < 32; kk += blockDim.y) {
-    const int k = k0 + kk, d = d0 + threadIdx.x;
-    // FP32-pair sum converted with integer operations (FP64 additions are
-    // the scarce resource on GB300): the state keeps ~47 bits of the update
-    if (k < R && d < n && (!mask || mask[k / nf]))
-      S.dst[k][d] = ff2d_i32(ff_add(d2ff(S.old[k][d]), t[threadIdx.x][kk]));
+  float inc[4], d2[4] = {0.f, 0.f, 0.f, 0.f}, n2[4] = {0.f, 0.f, 0.f, 0.f};
+  double was[4];
+  auto load = [&](int d0) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int d = d0 + ty + 8 * j, k = k0 + tx;
+      inc[j] = d < n && k < R ? S.D32[(size_t)d * R + k] : 0.f;
+      was[j] = d0 + tx < n ? old[j][d0 + tx] : 0.0;
+    }
+  };
+  load(d00);
+#pragma unroll 1
+  for (int q = 0; q < kDeltaTiles; ++q) {
+    const int d0 = d00 + 32 * q;
+    if (d0 >= n) break;
+    float(*tq)[33] = t[q & 1];  // the other half may still be read
+#pragma unroll
+    for (int j = 0; j < 4; ++j) tq[ty + 8 * j][tx] = inc[j];
+    double u[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) u[j] = was[j];
+    if (q + 1 < kDeltaTiles) load(d0 + 32);
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      // FP32-pair sum converted with integer operations (FP64 additions are
+      // the scarce resource on GB300): the state keeps ~47 bits of the update
+      const double x = ff2d_i32(ff_add(d2ff(u[j]), tq[tx][ty + 8 * j]));
+      if (d0 + tx >= n || !dst[j]) continue;
+      dst[j][d0 + tx] = x;
+      if (SUMS) {
+        const float d = d2f_trunc(x - u[j]), a = d2f_trunc(x);  // the one FP64 operation per value
+        d2[j] += d * d;
+        n2[j] += a * a;
+      }
+    }
+  }
+  if constexpr (SUMS) {
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) t[0][ty + 8 * j][tx] = d2[j], t[1][ty + 8 * j][tx] = n2[j];
+    __syncthreads();
+    __shared__ double sum[2][32];
+    if (ty < 2) {  // a column's 32 sums, by one thread in FP64
+      double a = 0.0;
+#pragma unroll 8
+      for (int i = 0; i < 32; ++i) a += f2d_exact(t[ty][tx][i]);
+      sum[ty][tx] = a;
+    }
+    __syncthreads();
+    const int k = k0 + tx;
+    if (ty == 0 && k < R)
+      C.out[((size_t)(k / nf) * 5 + C.first[blockIdx.z] + k % nf) * C.stride + blockIdx.x] =
+          make_double2(sum[0][tx], sum[1][tx]);
   }
 }
 
@@ -274,23 +363,40 @@ __global__ void k_residual_df_il(ElemSets E, int in_place) {
   residual_of<RT>(S)[o] = df_residual<RT>(in_place ? S.src[k][row] : S.B[o], sh, sl);
 }
 
-// Four right-hand sides per lane (128 per warp, R a multiple of 4): the row's
-// column indices and values are read once for all of them and every x row is
-// one 512 B (float) / 1 KB (pair) coalesced access.  Same arithmetic as above.
-__device__ __forceinline__ void ld_pairs4(const float* p, float2 (&v)[4]) {
-  const float4 t = *reinterpret_cast<const float4*>(p);
-  v[0] = make_float2(t.x, 0.f);
-  v[1] = make_float2(t.y, 0.f);
-  v[2] = make_float2(t.z, 0.f);
-  v[3] = make_float2(t.w, 0.f);
+// Two FP32 values in one 64-bit register: one instruction works on both, each
+// rounded as by itself (f32x2, Blackwell).
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 f2_of(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
 }
-__device__ __forceinline__ void ld_pairs4(const float2* p, float2 (&v)[4]) {
-  const float4 t0 = reinterpret_cast<const float4*>(p)[0], t1 = reinterpret_cast<const float4*>(p)[1];
-  v[0] = make_float2(t0.x, t0.y);
-  v[1] = make_float2(t0.z, t0.w);
-  v[2] = make_float2(t1.x, t1.y);
-  v[3] = make_float2(t1.z, t1.w);
+__device__ __forceinline__ float2 f2_get(F2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
 }
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) {
+  F2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
 __device__ __forceinline__ void st4(float* p, const float (&v)[4]) {
   *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
 }
@@ -299,42 +405,100 @@ __device__ __forceinline__ void st4(double* p, const double (&v)[4]) {
   reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
 }
 
+// Four right-hand sides per lane (128 per warp, R a multiple of 4): the row's
+// column indices and values are read once for all of them and every x row is one
+// 512 B (float) / 1 KB (pairs, laid out by st_pair<true>) coalesced access.  The same
+// operations in the same order as above, two right-hand sides per instruction
+// (instruction issue was the largest part: 52 per entry), a row's entries fetched
+// by its lanes at once and the x rows of U entries in flight (they were waited
+// for entry by entry).
 template <typename X, typename RT>
-__global__ void k_residual_df_il4(ElemSets E, int in_place) {
+__global__ void __launch_bounds__(256, 4) k_residual_df_il4(ElemSets E, int in_place) {
+  constexpr bool kPair = sizeof(X) == 8;
+  constexpr int U = kPair ? 2 : 4;  // entries in flight
+  __shared__ double bt[8][132];  // in place: the CTA's 8 rows of 128 right-hand sides
   const ElemSet& S = E.s[blockIdx.z];
-  const int row = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, R = S.R;
-  const int k = blockIdx.y * 128 + (threadIdx.x & 31) * 4;
-  if (row >= S.n || k >= R) return;
-  const X* xs = pair_x<X>(S);
-  float sh[4] = {0.f, 0.f, 0.f, 0.f}, sl[4] = {0.f, 0.f, 0.f, 0.f};
-  const int p1 = S.Adf.rp[row + 1];
-  for (int p = S.Adf.rp[row]; p < p1; ++p) {
-    const float2 a = S.Adf.v[p];
-    float2 xv[4];
-    ld_pairs4(xs + (size_t)S.Adf.ci[p] * R + k, xv);
+  const int row0 = blockIdx.x * 8, warp = threadIdx.x >> 5, row = row0 + warp, R = S.R, lane = threadIdx.x & 31;
+  const int k0 = blockIdx.y * 128, k = k0 + lane * 4;
+  if (row0 >= S.n || k0 >= R) return;
+  if (in_place) {
+    // eight threads take a column's eight values: 16 lines per row of the tile, where
+    // a row's own lanes touched 128
+    double v[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float ph = a.x * xv[q].x;
-      const float pe = fmaf(a.x, xv[q].x, -ph) + fmaf(a.x, xv[q].y, a.y * xv[q].x);
-      const float t = sh[q] + ph;
-      const float z = t - sh[q];
-      const float e = (sh[q] - (t - z)) + (ph - z);
-      sh[q] = t;
-      sl[q] += e + pe;
+    for (int j = 0; j < 4; ++j) {
+      const int c = (threadIdx.x >> 3) + 32 * j, r = row0 + (threadIdx.x & 7);
+      v[j] = k0 + c < R && r < S.n ? S.src[k0 + c][r] : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) bt[threadIdx.x & 7][(threadIdx.x >> 3) + 32 * j] = v[j];
+    __syncthreads();
+  }
+  if (row >= S.n) return;  // whole warps
+  const bool in = k < R;
+  const float* xs = reinterpret_cast<const float*>(pair_x<X>(S)) + (size_t)(in ? k : 0) * (kPair ? 2 : 1);
+  const size_t xstride = (size_t)R * (kPair ? 2 : 1);
+  F2 sh[2] = {0, 0}, sl[2] = {0, 0};
+  const int p1 = S.Adf.rp[row + 1];
+  for (int pb = S.Adf.rp[row]; pb < p1; pb += 32) {
+    const int m = min(32, p1 - pb);
+    int ci = 0;
+    float2 av = make_float2(0.f, 0.f);
+    if (lane < m) ci = S.Adf.ci[pb + lane], av = S.Adf.v[pb + lane];
+    for (int j = 0; j < m; j += U) {
+      float4 x[U][kPair ? 2 : 1];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int c = __shfl_sync(0xffffffffu, ci, (j + u) & 31);
+        if (j + u < m) {
+          const float4* xp = reinterpret_cast<const float4*>(xs + (size_t)c * xstride);
+          x[u][0] = xp[0];
+          if constexpr (kPair) x[u][1] = xp[1];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const float ah = __shfl_sync(0xffffffffu, av.x, (j + u) & 31);
+        const float al = __shfl_sync(0xffffffffu, av.y, (j + u) & 31);
+        if (j + u >= m) break;
+        const F2 A = f2_of(ah, ah), NA = f2_of(-ah, -ah), L = f2_of(al, al);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          F2 xh, xl;
+          if constexpr (kPair) {
+            xh = f2_of(x[u][q].x, x[u][q].y), xl = f2_of(x[u][q].z, x[u][q].w);
+          } else {
+            xh = q ? f2_of(x[u][0].z, x[u][0].w) : f2_of(x[u][0].x, x[u][0].y), xl = 0;
+          }
+          const F2 ph = f2_mul(A, xh);
+          const F2 en = f2_fma(NA, xh, ph);  // minus the product's rounding error (exact)
+          const F2 pe = f2_sub(f2_fma(A, xl, f2_mul(L, xh)), en);
+          const F2 t = f2_add(sh[q], ph);
+          const F2 z = f2_sub(t, sh[q]);
+          const F2 e = f2_add(f2_sub(sh[q], f2_sub(t, z)), f2_sub(ph, z));
+          sh[q] = t;
+          sl[q] = f2_add(sl[q], f2_add(e, pe));
+        }
+      }
     }
   }
+  if (!in) return;
   const size_t o = (size_t)row * R + k;
   double bb[4];
   if (in_place) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) bb[q] = S.src[k + q][row];
+    for (int q = 0; q < 4; ++q) bb[q] = bt[warp][lane * 4 + q];
   } else {
     const double2 b0 = reinterpret_cast<const double2*>(S.B + o)[0], b1 = reinterpret_cast<const double2*>(S.B + o)[1];
     bb[0] = b0.x, bb[1] = b0.y, bb[2] = b1.x, bb[3] = b1.y;
   }
   RT v[4];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) v[q] = df_residual<RT>(bb[q], sh[q], sl[q]);
+  for (int q = 0; q < 2; ++q) {
+    const float2 h = f2_get(sh[q]), l = f2_get(sl[q]);
+    v[2 * q] = df_residual<RT>(bb[2 * q], h.x, l.x);
+    v[2 * q + 1] = df_residual<RT>(bb[2 * q + 1], h.y, l.y);
+  }
   st4(residual_of<RT>(S) + o, v);
 }
 
@@ -386,7 +550,7 @@ constexpr int kRedChunks = 16;
 // FP32 resolution); Acc is the type the squares are summed in.
 template <typename Acc>
 __global__ void k_relchange_partial(FieldPtrs NEW, FieldPtrs OLD, int n_fields,
-                                    double2* __restrict__ partial) {
+                                    double2* __restrict__ partial, int stride) {
   const int chunk = blockIdx.x, fld = blockIdx.y, i = blockIdx.z;
   __shared__ double sd[kRedThreads], sn[kRedThreads];
   Acc d2 = 0, n2 = 0;
@@ -432,7 +596,7 @@ __global__ void k_relchange_partial(FieldPtrs NEW, FieldPtrs OLD, int n_fields,
     __syncthreads();
   }
   if (threadIdx.x == 0)
-    partial[((size_t)i * 5 + fld) * kRedChunks + chunk] = make_double2(sd[0], sn[0]);
+    partial[((size_t)i * 5 + fld) * stride + chunk] = make_double2(sd[0], sn[0]);
 }
 
 // Per-instance convergence test after a step (rel = max over fields of
@@ -440,36 +604,50 @@ __global__ void k_relchange_partial(FieldPtrs NEW, FieldPtrs OLD, int n_fields,
 // its relative change is <= tol (conv_step = the step), when its state is not
 // finite (conv_step = -step), or when it has marched max_steps since its start
 // step (conv_step = the step, capped = 1; streamed sweeps refill such slots).
-__global__ void k_converge(const double2* __restrict__ partial, int n_inst, int n_fields, double tol,
-                           int* __restrict__ conv_step, double* __restrict__ rel,
-                           int* __restrict__ step_ctr, int* __restrict__ active,
-                           int* __restrict__ n_active, const int* __restrict__ start, int max_steps,
-                           int* __restrict__ capped) {
-  // a warp per instance; 16 lanes add one field's chunks (a serial walk over
-  // them took 17 us of every step, whatever the instances' number)
-  static_assert(kRedChunks == 16, "half a warp adds the chunks of a field");
+// A CTA per instance, a warp per field: FP64 additions are slow, and one CTA for all
+// instances took 13 us of every step of 64.  The last CTA to arrive closes the
+// step (ticket[0] CTAs, ticket[1] active instances; it resets both).
+struct ChunkCounts {
+  int n[5];
+};
+constexpr int kConvergeThreads = 160;
+__global__ void __launch_bounds__(kConvergeThreads)
+    k_converge(const double2* __restrict__ partial, int stride, ChunkCounts counts, int n_inst, int n_fields, double tol,
+               int* __restrict__ conv_step, double* __restrict__ rel, int* __restrict__ step_ctr,
+               int* __restrict__ active, int* __restrict__ n_active, const int* __restrict__ start, int max_steps,
+               int* __restrict__ capped, int* __restrict__ ticket) {
+  __shared__ double sr[5];
+  __shared__ int sf[5];
+  const int i = blockIdx.x, fld = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int step = *step_ctr + 1;
-  __shared__ int cnt;
-  if (threadIdx.x == 0) cnt = 0;
+  double2 v = make_double2(0.0, 0.0);
+  if (fld < n_fields) {
+    const double2* p = partial + ((size_t)i * 5 + fld) * stride;
+#pragma unroll 4
+    for (int c = lane; c < counts.n[fld]; c += 32) {
+      const double2 w = p[c];
+      v.x += w.x;
+      v.y += w.y;
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+  }
+  if (lane == 0) {
+    sr[fld] = v.y > 0.0 ? sqrt(v.x / v.y) : sqrt(v.x);
+    sf[fld] = isfinite(v.x) && isfinite(v.y);
+  }
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int i = warp; i < n_inst; i += blockDim.x >> 5) {
+  if (threadIdx.x != 0) return;
+  int stays = 0;
+  if (active[i]) {
     double r = 0.0;
     bool finite = true;
-    for (int f0 = 0; f0 < n_fields; f0 += 2) {
-      const int fld = f0 + (lane >> 4);
-      double2 v = make_double2(0.0, 0.0);
-      if (fld < n_fields) v = partial[((size_t)i * 5 + fld) * kRedChunks + (lane & 15)];
-      for (int o = 8; o > 0; o >>= 1) {
-        v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-        v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-      }
-      finite = finite && isfinite(v.x) && isfinite(v.y);
-      if (fld < n_fields) r = fmax(r, v.y > 0.0 ? sqrt(v.x / v.y) : sqrt(v.x));
+    for (int f = 0; f < n_fields; ++f) {
+      r = fmax(r, sr[f]);
+      finite = finite && sf[f];
     }
-    r = fmax(r, __shfl_xor_sync(0xffffffffu, r, 16));
-    finite = __all_sync(0xffffffffu, finite);
-    if (lane != 0 || !active[i]) continue;
     rel[i] = finite ? r : __longlong_as_double(0x7ff8000000000000LL);
     if (!finite) {
       active[i] = 0;
@@ -482,13 +660,16 @@ __global__ void k_converge(const double2* __restrict__ partial, int n_inst, int 
       conv_step[i] = step;
       capped[i] = 1;
     } else {
-      atomicAdd(&cnt, 1);
+      stays = 1;
     }
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  if (stays) atomicAdd(ticket + 1, 1);
+  __threadfence();
+  if (atomicAdd(ticket, 1) == n_inst - 1) {
+    __threadfence();
+    *n_active = atomicExch(ticket + 1, 0);
     *step_ctr = step;
-    *n_active = cnt;
+    atomicExch(ticket, 0);
   }
 }
 
@@ -646,7 +827,11 @@ struct Engine {
   IlBank il[2];
   DBuf<double*> snap_ptrs;
   // steady state
-  DBuf<double2> partial;
+  DBuf<double2> partial;  // [instance][5][partial_stride], change_chunks of them in use
+  int partial_stride = kRedChunks;
+  ChunkCounts change_chunks{};
+  bool delta_sums = false;  // the step being launched takes its changes from the increment solves
+  DBuf<int> converge_ticket;
   DBuf<int> conv_step, step_ctr, active, n_active, start_step, capped, refill_mask;
   int step_cap = 1 << 30;  // per-instance step cap seen by k_converge (streamed sweeps)
   const int* scatter_mask = nullptr;  // solves write only these instances (slot refills)
@@ -695,7 +880,7 @@ struct Engine {
     // scatter, one sweep
     const bool dc = delta_solves() && il_f32(0), dp = delta_solves() && il_f32(1);
     return 1 + (dc ? lc + 3 : lc * (1 + ir_iters(0)) + elem_launches_per_solve(0)) + 1 +
-           (dp ? lp + 3 : lp * (1 + ir_iters(1)) + elem_launches_per_solve(1)) + 3;
+           (dp ? lp + 3 : lp * (1 + ir_iters(1)) + elem_launches_per_solve(1)) + (dc && dp ? 2 : 3);
   }
   // algorithmic bytes of one application of a bank to all of its right-hand
   // sides: every stored factor entry once, plus the vectors (b read, y write +
@@ -864,31 +1049,60 @@ struct Engine {
     for (int si = 0; si < I.n_sets; ++si) m = std::max(m, (size_t)I.set[si].n * I.set[si].R);
     return dim3((unsigned)((m + 255) / 256), I.n_sets);
   }
+  // residuals with four right-hand sides per lane: most lanes of a warp work
+  bool residual_by_four(int which) const {
+    const IlBank& I = il[which];
+    for (int si = 0; si < I.n_sets; ++si)
+      if (I.set[si].R % 4 != 0 || I.set[si].R < 96) return false;
+    return true;
+  }
   template <typename X, typename RT>
   void launch_residual_df(int which, const ElemSets& E, bool in_place, cudaStream_t s) const {
     const IlBank& I = il[which];
-    bool four = true;
     int n = 0;
-    for (int si = 0; si < I.n_sets; ++si) {
-      four = four && I.set[si].R % 4 == 0 && I.set[si].R >= 96;
-      n = std::max(n, I.set[si].n);
-    }
-    if (four)
+    for (int si = 0; si < I.n_sets; ++si) n = std::max(n, I.set[si].n);
+    if (residual_by_four(which))
       k_residual_df_il4<X, RT><<<dim3((n + 7) / 8, (I.max_R + 127) / 128, I.n_sets), 256, 0, s>>>(E, in_place);
     else
       k_residual_df_il<X, RT><<<elem_grid(which), 256, 0, s>>>(E, in_place);
     PECS_CUDA(cudaGetLastError());
   }
 
+  void launch_split(int which, const ElemSets& E, cudaStream_t s) const {
+    if (residual_by_four(which))
+      k_split_il<true><<<elem_grid(which), 256, 0, s>>>(E);
+    else
+      k_split_il<false><<<elem_grid(which), 256, 0, s>>>(E);
+    PECS_CUDA(cudaGetLastError());
+  }
+
   void solve_bank_delta(const FactorBank& bank, int which, int target, cudaStream_t s) {
     const ElemSets E = elem_sets(which, target);
     const dim3 tb(32, 8), tg = tile_grid(which);
-    k_gather_pairs_il<<<tg, tb, 0, s>>>(E);
+    if (residual_by_four(which))
+      k_gather_pairs_il<true><<<tg, tb, 0, s>>>(E);
+    else
+      k_gather_pairs_il<false><<<tg, tb, 0, s>>>(E);
     PECS_CUDA(cudaGetLastError());
     // the right-hand sides are read in place from the per-instance vectors
     launch_residual_df<float2, float>(which, E, true, s);
     bank_sweep(bank, which, true, s);
-    k_scatter_delta_il<<<tg, tb, 0, s>>>(E, scatter_mask, n_inst);
+    const dim3 dg((tg.x + kDeltaTiles - 1) / kDeltaTiles, tg.y, tg.z);
+    if (delta_sums) {
+      ChangeSums C;
+      C.out = partial.p;
+      C.stride = partial_stride;
+      const IlBank& I = il[which];
+      for (int si = 0; si < I.n_sets; ++si) {
+        C.fields[si] = I.set[si].R / n_inst;
+        C.first[si] = which == 1 ? n_fields - 1 : I.set[si].mat;
+        for (int f = 0; f < C.fields[si]; ++f)
+          change_chunks.n[C.first[si] + f] = (I.set[si].n + 32 * kDeltaTiles - 1) / (32 * kDeltaTiles);
+      }
+      k_scatter_delta_il<true><<<dg, tb, 0, s>>>(E, scatter_mask, n_inst, C);
+    } else {
+      k_scatter_delta_il<false><<<dg, tb, 0, s>>>(E, scatter_mask, n_inst, ChangeSums());
+    }
     PECS_CUDA(cudaGetLastError());
   }
 
@@ -911,8 +1125,7 @@ struct Engine {
         if (mixed && it == 0) {
           launch_residual_df<float, float>(which, E, false, s);
         } else if (mixed) {
-          k_split_il<<<eg, 256, 0, s>>>(E);
-          PECS_CUDA(cudaGetLastError());
+          launch_split(which, E, s);
           launch_residual_df<float2, float>(which, E, false, s);
         } else {
           if (it == 0) {
@@ -922,8 +1135,7 @@ struct Engine {
           k_residual_il<float><<<eg, 256, 0, s>>>(E);
         }
       } else if (mixed) {
-        k_split_il<<<eg, 256, 0, s>>>(E);
-        PECS_CUDA(cudaGetLastError());
+        launch_split(which, E, s);
         launch_residual_df<float2, double>(which, E, false, s);
       } else {
         k_residual_il<double><<<eg, 256, 0, s>>>(E);
@@ -1121,8 +1333,15 @@ struct Engine {
       PECS_CUDA(cudaStreamSynchronize(st));
     }
     // steady-state buffers
-    partial.alloc((size_t)n_inst * 5 * kRedChunks);
+    partial_stride = kRedChunks;
+    if (delta_solves() && il_f32(0) && il_f32(1))
+      for (const IlBank& I : il)
+        for (int si = 0; si < I.n_sets; ++si)
+          partial_stride = std::max(partial_stride, (I.set[si].n + 32 * kDeltaTiles - 1) / (32 * kDeltaTiles));
+    partial.alloc((size_t)n_inst * 5 * partial_stride);
     partial.zero();
+    converge_ticket.alloc(2);
+    converge_ticket.zero();
     conv_step.alloc(n_inst);
     start_step.alloc(n_inst);
     start_step.zero();
@@ -1412,17 +1631,28 @@ struct Engine {
   // step + steady-state bookkeeping (state[cur] -> state[nxt], compares both)
   void step_with_check(cudaStream_t s, double tol) {
     const int old = cur;
-    full_step(s, active.p);
+    // increment solves of every field add the changes up where they have them
+    delta_sums = delta_solves() && il_f32(0) && il_f32(1) && !scatter_mask;
+    try {
+      full_step(s, active.p);
+    } catch (...) {
+      delta_sums = false;
+      throw;
+    }
     FieldPtrs NEW = fields(state[cur], nullptr), OLD = fields(state[old], nullptr);
-    if (opt.precision == PECS_PREC_FP32_MIXED)
-      k_relchange_partial<float><<<dim3(kRedChunks, 5, n_inst), kRedThreads, 0, s>>>(NEW, OLD, n_fields,
-                                                                                    partial.p);
-    else
-      k_relchange_partial<double><<<dim3(kRedChunks, 5, n_inst), kRedThreads, 0, s>>>(NEW, OLD, n_fields,
-                                                                                     partial.p);
-    PECS_CUDA(cudaGetLastError());
-    k_converge<<<1, 1024, 0, s>>>(partial.p, n_inst, n_fields, tol, conv_step.p, rel.p, step_ctr.p,
-                                 active.p, n_active.p, start_step.p, step_cap, capped.p);
+    if (!delta_sums) {
+      for (int& c : change_chunks.n) c = kRedChunks;
+      const dim3 g(kRedChunks, 5, n_inst);
+      if (opt.precision == PECS_PREC_FP32_MIXED)
+        k_relchange_partial<float><<<g, kRedThreads, 0, s>>>(NEW, OLD, n_fields, partial.p, partial_stride);
+      else
+        k_relchange_partial<double><<<g, kRedThreads, 0, s>>>(NEW, OLD, n_fields, partial.p, partial_stride);
+      PECS_CUDA(cudaGetLastError());
+    }
+    delta_sums = false;
+    k_converge<<<n_inst, kConvergeThreads, 0, s>>>(partial.p, partial_stride, change_chunks, n_inst, n_fields, tol,
+                                                   conv_step.p, rel.p, step_ctr.p, active.p, n_active.p, start_step.p,
+                                                   step_cap, capped.p, converge_ticket.p);
     PECS_CUDA(cudaGetLastError());
     k_snapshot<<<dim3(8, 5, n_inst), 256, 0, s>>>(NEW, snap_ptrs.p, conv_step.p, step_ctr.p, 5);
     PECS_CUDA(cudaGetLastError());
