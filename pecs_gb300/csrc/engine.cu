@@ -142,29 +142,14 @@ __global__ void k_scatter_il(ElemSets E, const int* __restrict__ mask, int n_ins
   }
 }
 
-// Pairs of interleaved vectors: (hi, lo) one after another, or, for the residual
-// kernel that takes right-hand sides two at a time (QUAD; R even), hi, hi, lo, lo
-// of two neighbours, so that its packed operands come straight from a load.
-template <bool QUAD>
-__device__ __forceinline__ void st_pair(float2* Xs, size_t i, float2 v) {
-  if constexpr (QUAD) {
-    float* q = reinterpret_cast<float*>(Xs) + 2 * (i & ~(size_t)1) + (i & 1);
-    q[0] = v.x;
-    q[2] = v.y;
-  } else {
-    Xs[i] = v;
-  }
-}
-
 // Xs = X as FP32 pairs
-template <bool QUAD>
 __global__ void k_split_il(ElemSets E) {
   const ElemSet& S = E.s[blockIdx.y];
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= (size_t)S.n * S.R) return;
   const double a = S.X[i];
   const float hi = __double2float_rn(a);
-  st_pair<QUAD>(S.Xs, i, make_float2(hi, __double2float_rn(a - (double)hi)));
+  S.Xs[i] = make_float2(hi, __double2float_rn(a - (double)hi));
 }
 
 // between refinements: X += D (the correction's type), X = X32 + D32, X = X32
@@ -184,7 +169,6 @@ __global__ void k_update_il(ElemSets E) {
 // Xs[d * R + k] = old_k[d] as an FP32 pair (the previous step's solution,
 // interleaved for the residual of an increment solve).  Bound by memory: the four
 // loads of a thread are issued together (one after another, 12.6 M values took 51 us).
-template <bool QUAD>
 __global__ void __launch_bounds__(256) k_gather_pairs_il(ElemSets E) {
   const ElemSet& S = E.s[blockIdx.z];
   __shared__ double t[32][33];
@@ -203,7 +187,7 @@ __global__ void __launch_bounds__(256) k_gather_pairs_il(ElemSets E) {
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int d = d0 + ty + 8 * j, k = k0 + tx;
-    if (d < n && k < R) st_pair<QUAD>(S.Xs, (size_t)d * R + k, d2ff(t[tx][ty + 8 * j]));
+    if (d < n && k < R) S.Xs[(size_t)d * R + k] = d2ff(t[tx][ty + 8 * j]);
   }
 }
 
@@ -363,40 +347,29 @@ __global__ void k_residual_df_il(ElemSets E, int in_place) {
   residual_of<RT>(S)[o] = df_residual<RT>(in_place ? S.src[k][row] : S.B[o], sh, sl);
 }
 
-// Two FP32 values in one 64-bit register: one instruction works on both, each
-// rounded as by itself (f32x2, Blackwell).
-using F2 = unsigned long long;
-__device__ __forceinline__ F2 f2_of(float a, float b) {
-  F2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
+// Four right-hand sides per lane (128 per warp, R a multiple of 4): the row's
+// column indices and values are read once for all of them and every x row is
+// one 512 B (float) / 1 KB (pair) coalesced access.  Same arithmetic as above.  The
+// pairs' arithmetic keeps the FMA pipe and the x rows the L1 busy about half of the time
+// each: 49,152 rows x 128 right-hand sides x 2 sets take 155 us with the right-hand
+// sides of the CTA's eight rows read together, 169 with each row's by its own lanes.
+// Tried without gain: two right-hand sides per instruction (f32x2) and two or
+// four entries in flight (12 and 30 us more: fewer warps), the x rows of the eight rows
+// staged in shared memory (8 us more).
+__device__ __forceinline__ void ld_pairs4(const float* p, float2 (&v)[4]) {
+  const float4 t = *reinterpret_cast<const float4*>(p);
+  v[0] = make_float2(t.x, 0.f);
+  v[1] = make_float2(t.y, 0.f);
+  v[2] = make_float2(t.z, 0.f);
+  v[3] = make_float2(t.w, 0.f);
 }
-__device__ __forceinline__ float2 f2_get(F2 v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
+__device__ __forceinline__ void ld_pairs4(const float2* p, float2 (&v)[4]) {
+  const float4 t0 = reinterpret_cast<const float4*>(p)[0], t1 = reinterpret_cast<const float4*>(p)[1];
+  v[0] = make_float2(t0.x, t0.y);
+  v[1] = make_float2(t0.z, t0.w);
+  v[2] = make_float2(t1.x, t1.y);
+  v[3] = make_float2(t1.z, t1.w);
 }
-__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
-  F2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) {
-  F2 r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
-  F2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
-  F2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-
 __device__ __forceinline__ void st4(float* p, const float (&v)[4]) {
   *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
 }
@@ -405,21 +378,12 @@ __device__ __forceinline__ void st4(double* p, const double (&v)[4]) {
   reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
 }
 
-// Four right-hand sides per lane (128 per warp, R a multiple of 4): the row's
-// column indices and values are read once for all of them and every x row is one
-// 512 B (float) / 1 KB (pairs, laid out by st_pair<true>) coalesced access.  The same
-// operations in the same order as above, two right-hand sides per instruction
-// (instruction issue was the largest part: 52 per entry), a row's entries fetched
-// by its lanes at once and the x rows of U entries in flight (they were waited
-// for entry by entry).
 template <typename X, typename RT>
-__global__ void __launch_bounds__(256, 4) k_residual_df_il4(ElemSets E, int in_place) {
-  constexpr bool kPair = sizeof(X) == 8;
-  constexpr int U = kPair ? 2 : 4;  // entries in flight
+__global__ void __launch_bounds__(256) k_residual_df_il4(ElemSets E, int in_place) {
   __shared__ double bt[8][132];  // in place: the CTA's 8 rows of 128 right-hand sides
   const ElemSet& S = E.s[blockIdx.z];
-  const int row0 = blockIdx.x * 8, warp = threadIdx.x >> 5, row = row0 + warp, R = S.R, lane = threadIdx.x & 31;
-  const int k0 = blockIdx.y * 128, k = k0 + lane * 4;
+  const int row0 = blockIdx.x * 8, warp = threadIdx.x >> 5, row = row0 + warp, R = S.R;
+  const int k0 = blockIdx.y * 128, k = k0 + (threadIdx.x & 31) * 4;
   if (row0 >= S.n || k0 >= R) return;
   if (in_place) {
     // eight threads take a column's eight values: 16 lines per row of the tile, where
@@ -434,71 +398,37 @@ __global__ void __launch_bounds__(256, 4) k_residual_df_il4(ElemSets E, int in_p
     for (int j = 0; j < 4; ++j) bt[threadIdx.x & 7][(threadIdx.x >> 3) + 32 * j] = v[j];
     __syncthreads();
   }
-  if (row >= S.n) return;  // whole warps
-  const bool in = k < R;
-  const float* xs = reinterpret_cast<const float*>(pair_x<X>(S)) + (size_t)(in ? k : 0) * (kPair ? 2 : 1);
-  const size_t xstride = (size_t)R * (kPair ? 2 : 1);
-  F2 sh[2] = {0, 0}, sl[2] = {0, 0};
+  if (row >= S.n || k >= R) return;
+  const X* xs = pair_x<X>(S);
+  float sh[4] = {0.f, 0.f, 0.f, 0.f}, sl[4] = {0.f, 0.f, 0.f, 0.f};
   const int p1 = S.Adf.rp[row + 1];
-  for (int pb = S.Adf.rp[row]; pb < p1; pb += 32) {
-    const int m = min(32, p1 - pb);
-    int ci = 0;
-    float2 av = make_float2(0.f, 0.f);
-    if (lane < m) ci = S.Adf.ci[pb + lane], av = S.Adf.v[pb + lane];
-    for (int j = 0; j < m; j += U) {
-      float4 x[U][kPair ? 2 : 1];
+  for (int p = S.Adf.rp[row]; p < p1; ++p) {
+    const float2 a = S.Adf.v[p];
+    float2 xv[4];
+    ld_pairs4(xs + (size_t)S.Adf.ci[p] * R + k, xv);
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int c = __shfl_sync(0xffffffffu, ci, (j + u) & 31);
-        if (j + u < m) {
-          const float4* xp = reinterpret_cast<const float4*>(xs + (size_t)c * xstride);
-          x[u][0] = xp[0];
-          if constexpr (kPair) x[u][1] = xp[1];
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const float ah = __shfl_sync(0xffffffffu, av.x, (j + u) & 31);
-        const float al = __shfl_sync(0xffffffffu, av.y, (j + u) & 31);
-        if (j + u >= m) break;
-        const F2 A = f2_of(ah, ah), NA = f2_of(-ah, -ah), L = f2_of(al, al);
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          F2 xh, xl;
-          if constexpr (kPair) {
-            xh = f2_of(x[u][q].x, x[u][q].y), xl = f2_of(x[u][q].z, x[u][q].w);
-          } else {
-            xh = q ? f2_of(x[u][0].z, x[u][0].w) : f2_of(x[u][0].x, x[u][0].y), xl = 0;
-          }
-          const F2 ph = f2_mul(A, xh);
-          const F2 en = f2_fma(NA, xh, ph);  // minus the product's rounding error (exact)
-          const F2 pe = f2_sub(f2_fma(A, xl, f2_mul(L, xh)), en);
-          const F2 t = f2_add(sh[q], ph);
-          const F2 z = f2_sub(t, sh[q]);
-          const F2 e = f2_add(f2_sub(sh[q], f2_sub(t, z)), f2_sub(ph, z));
-          sh[q] = t;
-          sl[q] = f2_add(sl[q], f2_add(e, pe));
-        }
-      }
+    for (int q = 0; q < 4; ++q) {
+      const float ph = a.x * xv[q].x;
+      const float pe = fmaf(a.x, xv[q].x, -ph) + fmaf(a.x, xv[q].y, a.y * xv[q].x);
+      const float t = sh[q] + ph;
+      const float z = t - sh[q];
+      const float e = (sh[q] - (t - z)) + (ph - z);
+      sh[q] = t;
+      sl[q] += e + pe;
     }
   }
-  if (!in) return;
   const size_t o = (size_t)row * R + k;
   double bb[4];
   if (in_place) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) bb[q] = bt[warp][lane * 4 + q];
+    for (int q = 0; q < 4; ++q) bb[q] = bt[warp][k - k0 + q];
   } else {
     const double2 b0 = reinterpret_cast<const double2*>(S.B + o)[0], b1 = reinterpret_cast<const double2*>(S.B + o)[1];
     bb[0] = b0.x, bb[1] = b0.y, bb[2] = b1.x, bb[3] = b1.y;
   }
   RT v[4];
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    const float2 h = f2_get(sh[q]), l = f2_get(sl[q]);
-    v[2 * q] = df_residual<RT>(bb[2 * q], h.x, l.x);
-    v[2 * q + 1] = df_residual<RT>(bb[2 * q + 1], h.y, l.y);
-  }
+  for (int q = 0; q < 4; ++q) v[q] = df_residual<RT>(bb[q], sh[q], sl[q]);
   st4(residual_of<RT>(S) + o, v);
 }
 
@@ -1049,40 +979,26 @@ struct Engine {
     for (int si = 0; si < I.n_sets; ++si) m = std::max(m, (size_t)I.set[si].n * I.set[si].R);
     return dim3((unsigned)((m + 255) / 256), I.n_sets);
   }
-  // residuals with four right-hand sides per lane: most lanes of a warp work
-  bool residual_by_four(int which) const {
-    const IlBank& I = il[which];
-    for (int si = 0; si < I.n_sets; ++si)
-      if (I.set[si].R % 4 != 0 || I.set[si].R < 96) return false;
-    return true;
-  }
   template <typename X, typename RT>
   void launch_residual_df(int which, const ElemSets& E, bool in_place, cudaStream_t s) const {
     const IlBank& I = il[which];
+    bool four = true;
     int n = 0;
-    for (int si = 0; si < I.n_sets; ++si) n = std::max(n, I.set[si].n);
-    if (residual_by_four(which))
+    for (int si = 0; si < I.n_sets; ++si) {
+      four = four && I.set[si].R % 4 == 0 && I.set[si].R >= 96;
+      n = std::max(n, I.set[si].n);
+    }
+    if (four)
       k_residual_df_il4<X, RT><<<dim3((n + 7) / 8, (I.max_R + 127) / 128, I.n_sets), 256, 0, s>>>(E, in_place);
     else
       k_residual_df_il<X, RT><<<elem_grid(which), 256, 0, s>>>(E, in_place);
     PECS_CUDA(cudaGetLastError());
   }
 
-  void launch_split(int which, const ElemSets& E, cudaStream_t s) const {
-    if (residual_by_four(which))
-      k_split_il<true><<<elem_grid(which), 256, 0, s>>>(E);
-    else
-      k_split_il<false><<<elem_grid(which), 256, 0, s>>>(E);
-    PECS_CUDA(cudaGetLastError());
-  }
-
   void solve_bank_delta(const FactorBank& bank, int which, int target, cudaStream_t s) {
     const ElemSets E = elem_sets(which, target);
     const dim3 tb(32, 8), tg = tile_grid(which);
-    if (residual_by_four(which))
-      k_gather_pairs_il<true><<<tg, tb, 0, s>>>(E);
-    else
-      k_gather_pairs_il<false><<<tg, tb, 0, s>>>(E);
+    k_gather_pairs_il<<<tg, tb, 0, s>>>(E);
     PECS_CUDA(cudaGetLastError());
     // the right-hand sides are read in place from the per-instance vectors
     launch_residual_df<float2, float>(which, E, true, s);
@@ -1125,7 +1041,8 @@ struct Engine {
         if (mixed && it == 0) {
           launch_residual_df<float, float>(which, E, false, s);
         } else if (mixed) {
-          launch_split(which, E, s);
+          k_split_il<<<eg, 256, 0, s>>>(E);
+          PECS_CUDA(cudaGetLastError());
           launch_residual_df<float2, float>(which, E, false, s);
         } else {
           if (it == 0) {
@@ -1135,7 +1052,8 @@ struct Engine {
           k_residual_il<float><<<eg, 256, 0, s>>>(E);
         }
       } else if (mixed) {
-        launch_split(which, E, s);
+        k_split_il<<<eg, 256, 0, s>>>(E);
+        PECS_CUDA(cudaGetLastError());
         launch_residual_df<float2, double>(which, E, false, s);
       } else {
         k_residual_il<double><<<eg, 256, 0, s>>>(E);
