@@ -18,6 +18,7 @@ constexpr size_t kRowsSmem = 220 * 1024;
 constexpr size_t kMostColBytes = 200 * 1024;  // one right-hand side of the widest front a bank takes
 constexpr int kAsmMinRhs = 5;              // right-hand sides from which columns are assembled once per node
 constexpr int kAsmMinRb = 3;               // smallest chunk those counts are cut into
+constexpr int kAsmTiles = 8;               // tiles per node from which kAsmMinRb right-hand sides are enough
 
 template <typename T>
 struct VecOf;
@@ -761,10 +762,15 @@ void RowsSweep::load_kernels(int most_rhs) const {
     go(float{});
 }
 
-bool RowsSweep::assembles(const RowSets& sets, int max_nrhs) const {
-  for (int q = 0; q < n_sets_; ++q)
-    if (!sets.set[q].d) return false;
-  return max_nrhs >= kAsmMinRhs;
+// Assembling a level's columns costs a launch, and saves every tile of a node the
+// reading of the children's updates.  From five right-hand sides on that always
+// paid; for three and four it does at levels of many tiles per node.  us per Poisson
+// sweep of 3, never / from 2 / 4 / 8 tiles per node on: 72x72+72x72 cells, k = 2, FP32
+// 603 / 486 / 494 / 501; 40x40+40x40, k = 2, FP64 271 / 261 / 261 / 260; 16x16+16x16,
+// k = 1, FP64 67.6 / 74.9 / 69.1 / 67.8.
+static bool assembles(const RowLevel& L, int max_nrhs) {
+  if (L.leaf || L.n_tile == 0) return false;
+  return max_nrhs >= kAsmMinRhs || (max_nrhs >= kAsmMinRb && L.n_tile >= kAsmTiles * L.n_node);
 }
 
 int RowsSweep::launches_per_solve(int max_nrhs) const {
@@ -773,7 +779,7 @@ int RowsSweep::launches_per_solve(int max_nrhs) const {
   for (int d = 0; d < 2; ++d)
     for (const RowLevel& L : dir_[d].levels) {
       n += L.n_tile + L.n_batch > 0;
-      if (d == 0 && L.n_tile > 0 && !L.leaf && max_nrhs >= kAsmMinRhs) ++n;
+      if (d == 0 && assembles(L, max_nrhs)) ++n;
     }
   return n;
 }
@@ -789,10 +795,11 @@ void RowsSweep::solve(const RowSets& sets, int max_nrhs, cudaStream_t st) const 
         return;
       }
       ready<T, RB>();
-      const bool assemble = assembles(sets, max_nrhs);
+      bool room = true;
+      for (int q = 0; q < n_sets_; ++q) room = room && sets.set[q].d;
       for (const RowLevel& L : dir_[0].levels) {
         if constexpr (RB >= kAsmMinRb) {
-          if (assemble && !L.leaf) {
+          if (room && assembles(L, max_nrhs)) {
             launch_level<T, RB, true, true>(view(0), sets, n_sets_, L, max_nrhs, st);
             continue;
           }

@@ -84,7 +84,6 @@ class RowsSweep {
   void solve_flow(const RowSets& sets, cudaStream_t st) const;
   template <typename T, int RB>
   void ready() const;
-  bool assembles(const RowSets& sets, int max_nrhs) const;
   int prec_ = PECS_PREC_FP64;
   int n_sets_ = 0;
   int wtotal_[kRowsMaxSets] = {0, 0, 0, 0}, dofs_[kRowsMaxSets] = {0, 0, 0, 0};

@@ -112,12 +112,20 @@ RowsPlan plan_rows(const std::vector<const MfFactor*>& factors, int vr, int max_
   // FP32, k = 2, 16 / 8: 451 / 223 for 5 vectors at most, 502 / 226 for 9; FP64, 24 /
   // 12 on 29x37+23x37 cells: 829 / 405 with 0.3 rows, 1005 / 459 with one.
   const bool many = max_nrhs > 4;
-  const double most_vecs = many ? 5 : 16, least_vecs = 2, ctas_per_sm = 3, rows_per_rhs = vr == 2 ? 0.3 : 1.0;
+  const double most_vecs = many ? 5 : 32, least_vecs = 2, ctas_per_sm = 3, rows_per_rhs = vr == 2 ? 0.3 : 1.0;
   // a chunk of more than four right-hand sides is shared by threads of the same rows
   // (rows.cu: four each; FP64 chunks hold up to 8, FP32 up to 16), and needs fewer
   // values staged at a time
   const int rhs_threads = max_nrhs > 0 && !many ? 1 : (vr == 2 ? 2 : 4);
-  const int stage_vecs = many ? 8 : 10;
+  // Values staged at a time.  A large level's tiles (more than kLargeVecs vectors per
+  // thread) go through two small buffers, so that three CTAs share a multiprocessor
+  // and each reads its node's columns for more values; smaller tiles are staged
+  // whole.  72x72+72x72 cells, k = 2, RT_2 Poisson elements, FP32, 3 right-hand sides,
+  // us per Poisson sweep: 876 for 16 vectors at most and 10 staged, 649 for 32 / 10,
+  // 598 for 32 / 5, 609 for 64 / 4; 56x56+56x56, FP64, 1: 810, 736, 688; but 64x64+64x64,
+  // k = 1, FP64, 2, with tiles below that: 223 for 10 staged, 228 for 5.
+  const double kLargeVecs = 16;
+  const int stage_vecs_small = many ? 8 : 10, stage_vecs_large = many ? 8 : 5;
   std::vector<RowsPlan::Node>& nodes = R.nodes;
   int nl[2] = {0, 0};
   for (int fi = 0; fi < (int)factors.size(); ++fi) {
@@ -231,6 +239,7 @@ RowsPlan plan_rows(const std::vector<const MfFactor*>& factors, int vr, int max_
       for (int g : lv[d][l]) {
         if (!is_batch(g, d)) area += (double)rows_of(g) * cols_of(g), ++n;
       }
+      L.n_node = n;
       if (fwd)
         for (int g : lv[d][l]) {  // tile nodes come set by set
           const int q = nodes[g].set;
@@ -245,6 +254,7 @@ RowsPlan plan_rows(const std::vector<const MfFactor*>& factors, int vr, int max_
       const double per_thread =
           std::min(most_vecs, std::max(least_vecs, area / vr / ((double)kRowsSms * kRowsThreads * ctas_per_sm)));
       const double rhs_weight = std::max(1.0, 0.1 * max_nrhs);
+      const int stage_vecs = per_thread > kLargeVecs ? stage_vecs_large : stage_vecs_small;
       // team: the level's average node in one tile where the level has nodes enough
       int ts = 32;
       while (ts < kRowsThreads && area / std::max(1, n) * rhs_weight > per_thread * vr * ts * 1.5) ts *= 2;

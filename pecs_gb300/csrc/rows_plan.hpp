@@ -60,6 +60,7 @@ struct RowShape {
 // One tree level: its tiles (teams of ts threads), then its batches.
 struct RowLevel {
   int first = 0, n_tile = 0, n_batch = 0, ts = kRowsThreads;
+  int n_node = 0;  // nodes of the tiles
   bool leaf = true;  // no tile node has children
   RowShape shape;
   // forward, per set: the tile nodes' column and update records, and their
