@@ -442,7 +442,7 @@ def run_ragged(args):
 def run_profile_sweep(args):
     """Two sweeps of one factor bank over the workload's right-hand sides (the
     launches an ncu capture of one sweep selects with -k regex:k_panel or
-    regex:"k_forward|k_backward" and -c <launches per sweep>)."""
+    regex:"k_rows|k_assemble" and -c <launches per sweep>)."""
     import pecs_gb300 as pg
     pg.build()
     prec = {"fp64": pg.PREC_FP64, "fp32ir": pg.PREC_FP32_IR, "mixed": pg.PREC_FP32_MIXED}[args.precision]
@@ -594,7 +594,7 @@ def run_plain(args):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": peak_kind,
                      "traffic": load_traffic(f"carrier_solve_ref{args.refine}_{args.precision}"),
-                     "kernel": "k_forward/k_backward (carrier multifrontal solve sweep)",
+                     "kernel": "k_rows (carrier multifrontal solve sweep)",
                      "solve_ms": solve_ms, "poisson_solve_ms": pois_ms,
                      "bytes_per_sweep": info.solve_bytes[0], "launches_per_sweep": nlaunch},
         "gpu_launches": launches,
@@ -827,8 +827,8 @@ def run_full(args):
                      "traffic": load_traffic(f"carrier_solve_ref{args.refine}_mixed_b{B}"),
                      "kernel": ("k_panel_flow (carrier multifrontal solve sweep, one persistent "
                                 "launch per direction, FP32, " if info.flow_rpl[0] else
-                                "k_panel / k_panel_warp (carrier multifrontal solve sweep, one launch "
-                                "per tree level, FP32, ") + f"{2 * B} right-hand sides per factor)",
+                                "k_panel_assemble / k_panel_tiles / k_panel_warp (carrier multifrontal "
+                                "solve sweep, launches per tree level, FP32, ") + f"{2 * B} right-hand sides per factor)",
                      "flow_rpl": info.flow_rpl[0], "flow_top": info.flow_top[0],
                      "solve_ms": solve_ms, "launches_per_sweep": nlaunch,
                      "bytes_per_sweep": info.solve_bytes[0],
