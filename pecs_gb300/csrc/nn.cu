@@ -539,10 +539,20 @@ struct Mlp {
 
   static int tiles(int n, int t) { return (n + t - 1) / t; }
 
-  // activations of every layer; the output into y (null: act.back())
+  // Activations of every layer; the output into y (null: act.back()).  x and y may
+  // overlap: the first layer has read x when the last one writes y, and a network of one
+  // layer, whose tiles read and write the same rows at the same time, then goes through
+  // act.back().
   void forward(int B, const float* x, float* y, cudaStream_t s) {
     ensure_batch(B);
     const int L = (int)w.size() - 1;
+    const size_t ny = (size_t)B * w[L] * sizeof(float);
+    const uintptr_t px = reinterpret_cast<uintptr_t>(x), py = reinterpret_cast<uintptr_t>(y);
+    if (L == 1 && y && px < py + ny && py < px + (size_t)B * w[0] * sizeof(float)) {
+      forward(B, x, nullptr, s);
+      PECS_CUDA(cudaMemcpyAsync(y, act.back().p, ny, cudaMemcpyDeviceToDevice, s));
+      return;
+    }
     for (int l = 0; l < L; ++l)
       // act[l+1] = act(act[l] W_l^T + b_l); W_l stored out x in (row-major)
       launch_after(k_mlp_layer, dim3(tiles(w[l + 1], kTcN), tiles(B, kTcM)), s, B, w[l + 1], w[l],
