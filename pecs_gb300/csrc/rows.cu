@@ -13,8 +13,6 @@ namespace pecs {
 
 namespace {
 
-constexpr size_t kRowsColBytes = 32 * 1024;  // staged source values per CTA item; longer rows in chunks
-constexpr size_t kRowsSmem = 220 * 1024;
 constexpr size_t kMostColBytes = 200 * 1024;  // one right-hand side of the widest front a bank takes
 constexpr int kAsmMinRhs = 5;              // right-hand sides from which columns are assembled once per node
 constexpr int kAsmMinRb = 3;               // smallest chunk those counts are cut into
@@ -107,16 +105,6 @@ __device__ __forceinline__ void team_sync(int ts, int team) {
   else
     asm volatile("bar.sync %0, %1;\n" ::"r"(team + 1), "r"(ts) : "memory");
 }
-
-// Shared memory of one team, in bytes from its slice: two barriers, then one or two
-// buffers of tile values, the source values (overlaid by the partial sums) and the
-// pass-through sums (forward).
-struct RowsSmem {
-  int kc = 1;                // staged columns per chunk
-  unsigned buf = 0;          // bytes of one value buffer
-  unsigned ds = 0, cu = 0;   // offsets
-  unsigned team_bytes = 0;
-};
 
 // Partial sums: stride between right-hand sides, in values: one 16-byte step off a
 // multiple of 128 bytes, so that outputs read with the right-hand side fastest
@@ -628,18 +616,7 @@ void with_rb(int rb, F f) {
 
 template <typename T>
 RowsSmem smem_of(const RowShape& P, int rb, int ts) {
-  RowsSmem m;
-  const int most = (int)(kRowsColBytes / ((size_t)rb * sizeof(T)));
-  m.kc = std::max(1, std::min(P.cols, most));
-  m.buf = (unsigned)P.vals * sizeof(T);
-  const bool two = P.chunks > 1 || P.cols > m.kc;
-  m.ds = 16 + (two ? 2 : 1) * m.buf;
-  // a team's partial sums: at most ts x vector x right-hand sides per thread, and the strides' slack
-  const int rt = rb <= 4 ? rb : (rb == 6 ? 3 : 4);
-  const unsigned d = (unsigned)m.kc * rb * sizeof(T), r = (unsigned)ts * 16 * rt + 144u * rb;
-  m.cu = (m.ds + std::max(d, r) + 15) & ~15u;
-  m.team_bytes = (m.cu + (unsigned)P.npt * rb * 8 + 15) & ~15u;
-  return m;
+  return rows_smem(P, VecOf<T>::n, rb, ts);
 }
 
 void check_smem(size_t bytes) {

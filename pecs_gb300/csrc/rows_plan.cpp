@@ -53,6 +53,35 @@ RowRec make_rec(int src, const std::vector<int>& l, std::vector<int>& more) {
   return r;
 }
 
+RowsSmem rows_smem(const RowShape& P, int vr, int rb, int ts) {
+  const size_t kColBytes = 32 * 1024;  // staged source values; longer rows in chunks
+  const unsigned col = 16u / vr * rb;  // bytes of a column's source values
+  // a team's partial sums: at most ts x vector x right-hand sides per thread, and the strides' slack
+  const int rt = rb <= 4 ? rb : (rb == 6 ? 3 : 4);
+  const unsigned sums = (unsigned)ts * 16 * rt + 144u * rb;
+  auto layout = [&](int kc) {
+    RowsSmem m;
+    m.kc = kc;
+    m.buf = (unsigned)P.vals * (16u / vr);
+    const bool two = P.chunks > 1 || P.cols > kc;
+    m.ds = 16 + (two ? 2 : 1) * m.buf;
+    m.cu = (m.ds + std::max(kc * col, sums) + 15) & ~15u;
+    m.team_bytes = (m.cu + (unsigned)P.npt * rb * 8 + 15) & ~15u;
+    return m;
+  };
+  RowsSmem m = layout(std::max(1, std::min(P.cols, (int)(kColBytes / col))));
+  // A team's size follows its level's average node, the layout its widest tile: eight
+  // teams with 32 KB of columns each are more than a multiprocessor has.  They stage
+  // fewer columns at a time.  The values (at most 10 vectors per thread and buffer), sums
+  // and pass-through rows leave room for 13 KB of columns in a team of 32.
+  const size_t most = (kRowsSmem / (kRowsThreads / ts)) & ~(size_t)15;
+  if (m.team_bytes > most) {
+    const size_t rest = 16 + 2 * (size_t)m.buf + (size_t)P.npt * rb * 8 + 32;
+    m = layout((int)std::max<size_t>(1, rest < most ? (most - rest) / col : 1));
+  }
+  return m;
+}
+
 namespace {
 
 template <typename F>

@@ -57,6 +57,22 @@ struct RowShape {
   int chunks = 0;  // chunks of columns
 };
 
+// Shared memory of one team, in bytes from its slice: two barriers, then one or two
+// buffers of tile values, the source values (overlaid by the partial sums) and the
+// pass-through sums (forward).
+struct RowsSmem {
+  int kc = 1;                // staged columns per chunk
+  unsigned buf = 0;          // bytes of one value buffer
+  unsigned ds = 0, cu = 0;   // offsets
+  unsigned team_bytes = 0;
+};
+
+constexpr size_t kRowsSmem = 220 * 1024;  // most of a CTA
+
+// The layout for tiles of these sizes, teams of ts threads and chunks of rb right-hand
+// sides; the teams of a CTA take kRowsSmem at most.
+RowsSmem rows_smem(const RowShape& P, int vr, int rb, int ts);
+
 // One tree level: its tiles (teams of ts threads), then its batches.
 struct RowLevel {
   int first = 0, n_tile = 0, n_batch = 0, ts = kRowsThreads;
