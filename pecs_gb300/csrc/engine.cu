@@ -813,7 +813,7 @@ struct Engine {
            (dp ? lp + 3 : lp * (1 + ir_iters(1)) + elem_launches_per_solve(1)) + (dc && dp ? 2 : 3);
   }
   // algorithmic bytes of one application of a bank to all of its right-hand
-  // sides: every stored factor entry once, plus the vectors (b read, y write +
+  // sides: every factor value that its kernels read once, plus the vectors (b read, y write +
   // read, x write, update vectors write + read, in the sweep's vector type:
   // float for FP32 panel banks, else double)
   double solve_bytes(int which) const {
@@ -825,7 +825,7 @@ struct Engine {
       const double vb = S_.f32 ? 4.0 : 8.0;
       vec += (double)S_.R * (4.0 * vb * S_.n + 2.0 * vb * B.set_wtotal(si));
     }
-    return (double)B.bytes() + vec;
+    return (double)B.sweep_bytes() + vec;
   }
   double time_solves(int which, int reps) {
     cudaEvent_t e0, e1;
@@ -1163,7 +1163,9 @@ struct Engine {
       min_rc = std::min(min_rc, n_inst * (int)f.size());
       max_rc = std::max(max_rc, n_inst * (int)f.size());
     }
-    const PanelTuning tu{opt.panel_chunk, opt.panel_min_ctas};
+    // a flow sweep may be chosen by the autotuner or forced
+    const PanelTuning tu{opt.panel_chunk, opt.panel_min_ctas,
+                         opt.autotune ? opt.flow_sweep >= 0 : opt.flow_sweep > 0, opt.autotune != 0};
     bank_c.build(cf, fprec, min_rc >= kPanelMinRhs, tu, max_rc);
     bank_p.build({&fp}, fprec, n_inst >= kPanelMinRhs, tu, n_inst);
     // free host copies of the factor values (structure is kept for stats)

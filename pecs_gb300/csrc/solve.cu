@@ -6,6 +6,8 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
+#include <numeric>
 #include <type_traits>
 
 #include "bulk_copy.cuh"
@@ -516,7 +518,7 @@ __device__ __forceinline__ void tile_apply(const TilesView& B, const SV& st, con
   const int lg = P.lg_nw, nw = warp & ((1 << lg) - 1), kg = warp >> lg, KG = nthr >> (5 + lg);
   const int BN = 32 << lg, R = st.nrhs, K = I.cols, kc_max = P.kc, K4 = (K + 3) & ~3;
   const unsigned bar = smem_u32(smem);
-  const T* val = static_cast<const T*>(B.val) + I.off;
+  const T* val = static_cast<const T*>(B.val) + (I.off - B.val0);
   const int* idx = reinterpret_cast<const int*>(smem + 16);
   if (tid == 0) {
     bar_init(bar);
@@ -1039,8 +1041,10 @@ void launch_panel_warp(bool forward, const BankView& B, const SVT& S, const Pane
   const int rows_pad = (L.warp_rows + 3) & ~3, n = (int)L.warp.n;
   const size_t smem = kWarpNodesPerCta * panel_warp_bytes<T>(L.max_k, rows_pad, RC);
   const dim3 grid((n + kWarpNodesPerCta - 1) / kWarpNodesPerCta, (max_nrhs + RC - 1) / RC);
+  BankView V = B;
+  V.G = V.H = L.warp_val.p();  // the items' offsets
   launch_pdl(forward ? k_panel_warp<T, RPL, true, SVT> : k_panel_warp<T, RPL, false, SVT>, grid, kSolveThreads, smem, st,
-             B, S, (const PanelItem*)L.warp.p, n, L.max_k, rows_pad);
+             V, S, (const PanelItem*)L.warp.p, n, L.max_k, rows_pad);
 }
 
 // The valid options of a level for rpl_max right-hand sides per lane.
@@ -1251,14 +1255,37 @@ BankView FactorBank::view() const {
   v.cmap_ptr = cmap_ptr_.p;
   v.cmap_idx = cmap_idx_.p;
   v.node_set = node_set_.p;
-  v.G = prec_ == PECS_PREC_FP64 ? (const void*)G64_.p : (const void*)G32_.p;
-  v.H = prec_ == PECS_PREC_FP64 ? (const void*)H64_.p : (const void*)H32_.p;
+  v.G = G_.p();
+  v.H = H_.p();
   return v;
 }
 
-TilesView FactorBank::tiles_view(int d) const {
-  return TilesView{tiles_[d].p, prec_ == PECS_PREC_FP64 ? (const void*)tval64_[d].p : (const void*)tval32_[d].p,
-                   tidx_[d].p, rec_.p, more_.p};
+TilesView FactorBank::tiles_view(int d, const PanelPlan& L) const {
+  return TilesView{tiles_[d].p, L.val.p(), L.val0, tidx_[d].p, rec_.p, more_.p};
+}
+
+long long FactorBank::bytes() const {
+  if (!panel_) return rows_.bytes();
+  long long n = G_.bytes() + H_.bytes();
+  for (auto* plans : {&pfwd_, &pbwd_})
+    for (const PanelPlan& L : *plans) n += L.val.bytes() + L.warp_val.bytes();
+  return n;
+}
+
+long long FactorBank::sweep_bytes() const {
+  if (!panel_) return rows_.bytes();
+  const int top = flow_sel_ < 0 ? 0 : flow_cfg_[flow_sel_].top;
+  long long n = flow_sel_ < 0 ? 0 : flow_cfg_[flow_sel_].values;
+  for (int d = 0; d < 2; ++d) {
+    const std::vector<PanelPlan>& plans = d == 0 ? pfwd_ : pbwd_;
+    for (size_t l = 0; l < plans.size(); ++l) {
+      if (d == 0 ? l + top >= plans.size() : (int)l < top) continue;  // in the flow sweep
+      const PanelPlan& L = plans[l];
+      // untuned levels take leaf warps where they have them
+      n += L.tuned.kind == 2 || (L.tuned.kind < 0 && L.warp.n > 0) ? L.n_warp_val : L.n_val;
+    }
+  }
+  return n * (prec_ == PECS_PREC_FP64 ? 8 : 4);
 }
 
 int FactorBank::kernel_launches_per_solve() const {
@@ -1291,14 +1318,13 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
   if (!panel) {
     rows_.build(factors, precision, max_nrhs);
     entries_ = rows_.entries();
-    bytes_ = rows_.bytes();
     for (int si = 0; si < n_sets_; ++si) set_wtotal_[si] = rows_.set_wtotal(si);
     return;
   }
   std::vector<int> hs, hm, own_off, upd_off, w_off, cm_off, own_idx, upd_idx, cmap_ptr, cmap_idx,
       node_set;
   std::vector<long long> goff, hoff;
-  std::vector<double> G, H;
+  std::vector<int> node_at;  // of its factor
   long long go = 0, ho = 0;
   int wtot = 0;
   struct LevelNodes {
@@ -1332,16 +1358,7 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
       node_set.push_back(fi);
       goff.push_back(go);
       hoff.push_back(ho);
-      {
-        // every block column-major
-        const int s_ = nd.s, f_ = nd.s + nd.m;
-        const std::vector<double>& g = F.Gf[j];  // f_ x s_ row-major
-        for (int c = 0; c < s_; ++c)
-          for (int r = 0; r < f_; ++r) G.push_back(g[(size_t)r * s_ + c]);
-        const std::vector<double>& h = F.Hb[j];  // s_ x f_ row-major
-        for (int c = 0; c < f_; ++c)
-          for (int r = 0; r < s_; ++r) H.push_back(h[(size_t)r * f_ + c]);
-      }
+      node_at.push_back(j);
       go += (long long)F.Gf[j].size();
       ho += (long long)F.Hb[j].size();
       // extend-add gather lists per front position
@@ -1387,15 +1404,35 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
   node_set_.upload(node_set);
   goff_.upload(goff);
   hoff_.upload(hoff);
-  if (prec_ == PECS_PREC_FP64) {
-    G64_.upload(G);
-    H64_.upload(H);
-    bytes_ = (long long)(G.size() + H.size()) * 8;
-  } else {
-    std::vector<float> g32(G.begin(), G.end()), h32(H.begin(), H.end());
-    G32_.upload(g32);
-    H32_.upload(h32);
-    bytes_ = (long long)(G.size() + H.size()) * 4;
+  // blocks of these nodes (forward Gf, backward Hb), column-major, one after another
+  auto column_major = [&](const std::vector<int>& nodes, bool forward, BankValues& out) {
+    size_t n = 0;
+    for (int g : nodes) n += (size_t)hs[g] * (hs[g] + hm[g]);
+    auto fill = [&](auto* o) {
+      using T = typename std::remove_pointer<decltype(o)>::type;
+      for (int g : nodes) {
+        const MfFactor& F = *factors[node_set[g]];
+        const int f = hs[g] + hm[g], rows = forward ? f : hs[g], cols = forward ? hs[g] : f;
+        const std::vector<double>& v = forward ? F.Gf[node_at[g]] : F.Hb[node_at[g]];
+        for (int c = 0; c < cols; ++c)
+          for (int r = 0; r < rows; ++r) *o++ = (T)v[(size_t)r * cols + c];
+      }
+    };
+    if (prec_ == PECS_PREC_FP64) {
+      std::vector<double> v(n);
+      fill(v.data());
+      out.f64.upload(v);
+    } else {
+      std::vector<float> v(n);
+      fill(v.data());
+      out.f32.upload(v);
+    }
+  };
+  if (tune_.flow) {
+    std::vector<int> all(hs.size());
+    std::iota(all.begin(), all.end(), 0);
+    column_major(all, true, G_);
+    column_major(all, false, H_);
   }
   {
     // level plans: tiles of packed values (panel_plan.hpp), and leaf warps
@@ -1408,15 +1445,12 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
       const PanelTilesPlan::Dir& D = H.dir[d];
       tiles_[d].upload(D.tiles);
       tidx_[d].upload(D.idx);
-      if (prec_ == PECS_PREC_FP64) {
-        std::vector<double> v(D.n_values);
-        pack_panel(H, factors, d, v.data());
-        tval64_[d].upload(v);
-      } else {
-        std::vector<float> v(D.n_values);
-        pack_panel(H, factors, d, v.data());
-        tval32_[d].upload(v);
-      }
+      std::unique_ptr<double[]> v64(prec_ == PECS_PREC_FP64 ? new double[D.n_values] : nullptr);
+      std::unique_ptr<float[]> v32(prec_ == PECS_PREC_FP64 ? nullptr : new float[D.n_values]);
+      if (v64)
+        pack_panel(H, factors, d, v64.get());
+      else
+        pack_panel(H, factors, d, v32.get());
       std::vector<PanelPlan>& out = forward ? pfwd_ : pbwd_;
       const std::vector<LevelNodes>& lv = forward ? fl : bl;
       out.clear();
@@ -1425,6 +1459,15 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
         PanelPlan& L = out[l];
         L.tiles = D.levels[l];
         for (int q = 0; q < n_sets_; ++q) L.assembled = L.assembled || (forward && L.tiles.n_rec[q] > 0);
+        const size_t end = (size_t)L.tiles.first + L.tiles.n;
+        L.val0 = L.tiles.n > 0 ? D.tiles[L.tiles.first].off : 0;
+        L.n_val = L.tiles.n > 0 ? (end < D.tiles.size() ? D.tiles[end].off : D.n_values) - L.val0 : 0;
+        auto upload_tiles = [&] {
+          if (v64)
+            L.val.f64.upload(v64.get() + L.val0, (size_t)L.n_val);
+          else
+            L.val.f32.upload(v32.get() + L.val0, (size_t)L.n_val);
+        };
         // leaf level: every node small and, forward, without children
         bool leaf = true;
         for (int g : lv[l].nodes) {
@@ -1438,10 +1481,14 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
         }
         const size_t rows_pad = (size_t)((L.warp_rows + 3) & ~3);
         const size_t wb = (((size_t)L.max_k * 32 + (size_t)L.max_k * rows_pad) * esz + (size_t)L.max_k * 4 + 15) & ~(size_t)15;
-        if (!leaf || kWarpNodesPerCta * wb > kWarpSmem) continue;
+        const bool warps = leaf && kWarpNodesPerCta * wb <= kWarpSmem;
+        if (!warps || tune_.options) upload_tiles();  // untuned, leaf levels take the warps
+        if (!warps) continue;
+        column_major(lv[l].nodes, forward, L.warp_val);
         std::vector<PanelItem> items;
         for (int g : lv[l].nodes) {
-          const long long off = forward ? goff[g] : hoff[g];
+          const long long off = L.n_warp_val;
+          L.n_warp_val += (long long)hs[g] * (hs[g] + hm[g]);
           PanelItem it;
           it.a = make_int4(g, 0, forward ? hs[g] + hm[g] : hs[g], 32);
           it.b = make_int4(hs[g], hm[g], node_set[g], w_off[g]);
@@ -1486,10 +1533,15 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
     for (int t : {7, 5, 3})
       if (t < n_levels) tops.push_back(t);
     for (int top : tops) {
+      if (!tune_.flow) break;
+      long long values = 0;  // bl is fl from the root down
+      for (size_t l = 0; l < std::min((size_t)top, bl.size()); ++l)
+        for (int g : bl[l].nodes) values += 2ll * hs[g] * (hs[g] + hm[g]);
       for (int kc : {64, 32}) {
         for (int rpl : {1, 2, 4}) {
           FlowConfig cfg;
           cfg.top = top;
+          cfg.values = values;
           cfg.kc = tune_.chunk > 0 ? std::min(kc, tune_.chunk) : kc;
           cfg.rpl = rpl;
           bool ok = true;
@@ -1628,7 +1680,7 @@ void FactorBank::solve_flow(const SVT& sets, int max_nrhs, int cfg, cudaStream_t
   int* queue[2] = {base + 2 * (size_t)n_nodes_, base + 2 * (size_t)n_nodes_ + 1};
   int* err = base + 2 * (size_t)n_nodes_ + 2;
   for (size_t l = 0; l + C.top < pfwd_.size(); ++l)
-    launch_panel_level<T, SVT>(true, B, tiles_view(0), sets, n_sets_, pfwd_[l], max_nrhs, lrpl, tune_, st);
+    launch_panel_level<T, SVT>(true, B, tiles_view(0, pfwd_[l]), sets, n_sets_, pfwd_[l], max_nrhs, lrpl, tune_, st);
   for (int d = 0; d < 2; ++d) {
     const FlowPlan& FP = C.plan[d];
     const FlowView F{FP.entries.p, FP.items.p, FP.sync.p, ctr[d], ctr[1 - d], n_nodes_,
@@ -1640,7 +1692,7 @@ void FactorBank::solve_flow(const SVT& sets, int max_nrhs, int cfg, cudaStream_t
     }
   }
   for (size_t l = C.top; l < pbwd_.size(); ++l)
-    launch_panel_level<T, SVT>(false, B, tiles_view(1), sets, n_sets_, pbwd_[l], max_nrhs, lrpl, tune_, st);
+    launch_panel_level<T, SVT>(false, B, tiles_view(1, pbwd_[l]), sets, n_sets_, pbwd_[l], max_nrhs, lrpl, tune_, st);
 }
 
 template <typename SVT>
@@ -1655,9 +1707,9 @@ void FactorBank::solve_panel(const SVT& sets, int max_nrhs, cudaStream_t st) con
     const bool fwd = pass == 0;
     for (const PanelPlan& L : fwd ? pfwd_ : pbwd_) {
       if constexpr (std::is_same<SVT, IlSetsViewF>::value)
-        launch_panel_level<float, SVT>(fwd, B, tiles_view(pass), sets, n_sets_, L, max_nrhs, rpl, tune_, st);
+        launch_panel_level<float, SVT>(fwd, B, tiles_view(pass, L), sets, n_sets_, L, max_nrhs, rpl, tune_, st);
       else
-        launch_panel_level<double, SVT>(fwd, B, tiles_view(pass), sets, n_sets_, L, max_nrhs, rpl, tune_, st);
+        launch_panel_level<double, SVT>(fwd, B, tiles_view(pass, L), sets, n_sets_, L, max_nrhs, rpl, tune_, st);
     }
   }
 }
@@ -1684,14 +1736,16 @@ void FactorBank::force_flow_impl(const SVT& sets, int max_nrhs) {
 
 void FactorBank::force_flow(const IlSetsViewF& sets, int max_nrhs) {
   force_flow_impl(sets, max_nrhs);
-  release_unused_flow();
+  release_unused();
 }
 void FactorBank::force_flow(const IlSetsView& sets, int max_nrhs) {
   force_flow_impl(sets, max_nrhs);
-  release_unused_flow();
+  release_unused();
 }
 
-void FactorBank::release_unused_flow() {
+// Once the kernels are chosen: the flow plans and the forms of the blocks that none of them
+// reads.  (A chosen flow sweep keeps the levels' too: they are timed on request.)
+void FactorBank::release_unused() {
   for (int c = 0; c < (int)flow_cfg_.size(); ++c) {
     if (c == flow_sel_) continue;
     for (FlowPlan& P : flow_cfg_[c].plan) {
@@ -1701,11 +1755,21 @@ void FactorBank::release_unused_flow() {
       P.n_entries = 0;
     }
   }
+  if (flow_sel_ >= 0) return;
+  G_.release();
+  H_.release();
+  for (auto* plans : {&pfwd_, &pbwd_})
+    for (PanelPlan& L : *plans) {
+      if (L.tuned.kind == 2) L.val.release();
+      if (L.tuned.kind == 0) L.warp.release(), L.warp_val.release();
+    }
 }
 
 template <typename SVT>
 void FactorBank::autotune_panel(const SVT& sets, int max_nrhs, cudaStream_t st, int reps, int flow_mode) {
   using T = typename std::conditional<std::is_same<SVT, IlSetsViewF>::value, float, double>::type;
+  if (!tune_.flow && flow_mode >= 0) throw PecsError(PECS_E_STATE, "bank built without flow sweeps");
+  if (!tune_.options) throw PecsError(PECS_E_STATE, "bank built for the untuned kernels only");
   const int rpl = panel_rpl(sets, max_nrhs);
   cudaEvent_t e0, e1;
   PECS_CUDA(cudaEventCreate(&e0));
@@ -1776,7 +1840,7 @@ void FactorBank::autotune_panel(const SVT& sets, int max_nrhs, cudaStream_t st, 
     best_sweep = best_flow_ms;
     flow_sel_ = best_flow;
   }
-  release_unused_flow();
+  release_unused();
   tuned_ms_ = best_sweep;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -1796,7 +1860,7 @@ std::vector<double> FactorBank::time_levels(const IlSetsViewF& sets, int max_nrh
     PECS_CUDA(cudaEventRecord(ev[0], st));
     for (int pass = 0; pass < 2; ++pass)
       for (const PanelPlan& L : pass == 0 ? pfwd_ : pbwd_) {
-        launch_panel_level<float, IlSetsViewF>(pass == 0, B, tiles_view(pass), sets, n_sets_, L, max_nrhs, rpl, tune_, st);
+        launch_panel_level<float, IlSetsViewF>(pass == 0, B, tiles_view(pass, L), sets, n_sets_, L, max_nrhs, rpl, tune_, st);
         PECS_CUDA(cudaEventRecord(ev[++l], st));
       }
     PECS_CUDA(cudaEventSynchronize(ev[nl]));

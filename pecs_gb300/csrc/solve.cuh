@@ -75,10 +75,11 @@ struct IlSetsViewF {
   IlSetViewF set[kMaxSets];
 };
 
-// Device pointers of one direction's level plan.
+// Device pointers of one level's plan; `val` holds the plan's values from val0 on.
 struct TilesView {
   const PanelTile* tiles;
   const void* val;
+  long long val0;
   const int* idx;
   const RowRec* rec;
   const int* more;
@@ -95,6 +96,15 @@ struct __align__(16) PanelItem {
   int unused[3];
 };
 
+// Factor values on the device, FP64 or FP32 as the bank's.
+struct BankValues {
+  DBuf<double> f64;
+  DBuf<float> f32;
+  const void* p() const { return f64.p ? (const void*)f64.p : (const void*)f32.p; }
+  long long bytes() const { return (long long)(f64.n * 8 + f32.n * 4); }
+  void release() { f64.release(), f32.release(); }
+};
+
 // How a panel level is launched.
 struct PanelOption {
   int kind = -1;  // -1 untuned, 0 tiles, 2 leaf warps
@@ -104,8 +114,13 @@ struct PanelOption {
 
 struct PanelPlan {
   PanelLevel tiles;      // panel_plan.hpp
+  BankValues val;          // the tiles' values
+  long long val0 = 0;      // ... from this one of the plan on
+  long long n_val = 0;     // ... so many
   bool assembled = false;  // forward: nodes with children, whose positions are assembled first
   DBuf<PanelItem> warp;  // leaf levels: one item per node, a warp each (else empty)
+  BankValues warp_val;   // ... and the nodes' blocks, column-major
+  long long n_warp_val = 0;
   int max_k = 0;         // leaf levels: largest column count
   int warp_rows = 0;     // leaf levels: most rows of a node
   PanelOption tuned;     // the autotuner's choice (kind -1: heuristic)
@@ -170,15 +185,15 @@ FlowPlanHost plan_flow(const FlowNodes& nd, bool forward, int top, int rpl, int 
 struct PanelTuning {
   int chunk = 0;     // most staged block columns per chunk (0: what shared memory holds)
   int min_ctas = 0;  // CTAs a level must reach before shorter tiles are used (0: one per SM)
+  bool flow = true;      // hold what the flow sweeps read until one is chosen or none
+  bool options = true;   // ... and what every option of a level reads (autotune needs both)
 };
 
 class FactorBank {
  public:
   // factors[i] is bound to RHS set i.  precision: PECS_PREC_FP64 or FP32_IR.
-  // panel: store every block column-major and apply it with the panel
-  // kernels (many right-hand sides per set, interleaved layout only).
-  // max_nrhs: the most right-hand sides any set will carry (panel banks size
-  // their split-K scratch with it)
+  // panel: many right-hand sides per set (the panel kernels, interleaved layout only).
+  // max_nrhs: the most right-hand sides any set will carry
   void build(const std::vector<const MfFactor*>& factors, int precision, bool panel = false,
              PanelTuning tuning = PanelTuning(), int max_nrhs = 0);
   // y = forward(b), x = backward(y); w is workspace.  All sets must be bound.
@@ -189,7 +204,11 @@ class FactorBank {
   int set_wtotal(int set) const { return set_wtotal_[set]; }
   int precision() const { return prec_; }
   long long entries() const { return entries_; }
-  long long bytes() const { return bytes_; }
+  // Device bytes of the factor values, and those that one sweep reads: zeros outside the
+  // blocks' triangles are left out, rows padded.  A panel bank holds several forms of
+  // its blocks until its kernels are chosen, then one -- with a flow sweep two.
+  long long bytes() const;
+  long long sweep_bytes() const;
   int kernel_launches_per_solve() const;
   bool panel() const { return panel_; }
   // Panel banks: choose each level's tiling option by timing whole sweeps on
@@ -232,21 +251,18 @@ class FactorBank {
   int prec_ = PECS_PREC_FP64;
   int n_sets_ = 0, max_nrhs_ = 0;
   int set_wtotal_[kMaxSets] = {0, 0, 0, 0};
-  long long entries_ = 0, bytes_ = 0;
+  long long entries_ = 0;
   DBuf<int> s_, m_, own_off_, upd_off_, w_off_, cm_off_, own_idx_, upd_idx_, cmap_ptr_, cmap_idx_,
       node_set_;
   DBuf<long long> goff_, hoff_;
-  DBuf<double> G64_, H64_;
-  DBuf<float> G32_, H32_;
+  BankValues G_, H_;  // flow sweeps: every block, column-major
   std::vector<PanelPlan> pfwd_, pbwd_;
   bool panel_ = false;
   PanelTuning tune_;
-  DBuf<PanelTile> tiles_[2];  // level sweeps: tiles, their values and index lists per direction
-  DBuf<double> tval64_[2];
-  DBuf<float> tval32_[2];
+  DBuf<PanelTile> tiles_[2];  // level sweeps: tiles and their index lists per direction
   DBuf<int> tidx_[2], more_;
   DBuf<RowRec> rec_;
-  TilesView tiles_view(int d) const;
+  TilesView tiles_view(int d, const PanelPlan& L) const;
   template <typename SVT>
   void solve_panel(const SVT& sets, int max_nrhs, cudaStream_t st) const;
   template <typename SVT>
@@ -262,6 +278,7 @@ class FactorBank {
   struct FlowConfig {
     int top = 0, kc = 0, rpl = 0;
     FlowPlan plan[2];  // forward, backward
+    long long values = 0;  // factor values that both read
   };
   std::vector<FlowConfig> flow_cfg_;
   int flow_sel_ = -1;     // the configuration in use (-1: level launches only)
@@ -270,7 +287,7 @@ class FactorBank {
   int stall_node_ = -1;  // the first factor's root (debug_arm_flow_stall)
   RowsSweep rows_;       // banks with few right-hand sides per set (not panel_)
   RowSets row_sets(const IlSetsView& sets) const;
-  void release_unused_flow();
+  void release_unused();
   template <typename SVT>
   bool flow_ok(const SVT& sets, int max_nrhs, int cfg) const;
   template <typename SVT>
