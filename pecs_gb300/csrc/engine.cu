@@ -793,7 +793,7 @@ struct Engine {
   int elem_launches_per_solve(int which) const {
     const int iters = ir_iters(which);
     const bool mixed = opt.precision == PECS_PREC_FP32_MIXED, f32 = il_f32(which);
-    int n = 2 + iters;
+    int n = 2 + iters * (mixed ? residual_df_launches(which) : 1);
     for (int it = 0; it < iters; ++it) {
       if (mixed ? !(f32 && it == 0) : (f32 && it == 0)) ++n;  // split / widen
       if (it + 1 < iters) ++n;                                // update
@@ -809,8 +809,8 @@ struct Engine {
     // increment solves: gather of the previous solution, residual and
     // scatter, one sweep
     const bool dc = delta_solves() && il_f32(0), dp = delta_solves() && il_f32(1);
-    return 1 + (dc ? lc + 3 : lc * (1 + ir_iters(0)) + elem_launches_per_solve(0)) + 1 +
-           (dp ? lp + 3 : lp * (1 + ir_iters(1)) + elem_launches_per_solve(1)) + (dc && dp ? 2 : 3);
+    return 1 + (dc ? lc + 2 + residual_df_launches(0) : lc * (1 + ir_iters(0)) + elem_launches_per_solve(0)) + 1 +
+           (dp ? lp + 2 + residual_df_launches(1) : lp * (1 + ir_iters(1)) + elem_launches_per_solve(1)) + (dc && dp ? 2 : 3);
   }
   // algorithmic bytes of one application of a bank to all of its right-hand
   // sides: every factor value that its kernels read once, plus the vectors (b read, y write +
@@ -979,20 +979,39 @@ struct Engine {
     for (int si = 0; si < I.n_sets; ++si) m = std::max(m, (size_t)I.set[si].n * I.set[si].R);
     return dim3((unsigned)((m + 255) / 256), I.n_sets);
   }
+  // Residuals in pairs: sets of whole groups of four right-hand sides that fill most of a
+  // warp's 128 take four per lane, the others a thread each -- by set, since one region's
+  // sets may be half as wide as the other's (distinct mobilities).  64x64+64x64 cells,
+  // distinct mobilities in the semiconductor, increment solves, us a step: 64 instances
+  // 1,158 with a thread each throughout, 1,104 by set; 48 instances 1,029 and 1,005.
+  static bool four_rhs(int R) { return R % 4 == 0 && R >= 96; }
+  int residual_df_launches(int which) const {
+    const IlBank& I = il[which];
+    bool four = false, one = false;
+    for (int si = 0; si < I.n_sets; ++si) (four_rhs(I.set[si].R) ? four : one) = true;
+    return four && one ? 2 : 1;
+  }
   template <typename X, typename RT>
   void launch_residual_df(int which, const ElemSets& E, bool in_place, cudaStream_t s) const {
-    const IlBank& I = il[which];
-    bool four = true;
-    int n = 0;
-    for (int si = 0; si < I.n_sets; ++si) {
-      four = four && I.set[si].R % 4 == 0 && I.set[si].R >= 96;
-      n = std::max(n, I.set[si].n);
+    for (bool four : {true, false}) {
+      ElemSets G;
+      int k = 0, n = 0, R = 0;
+      size_t m = 0;
+      for (int si = 0; si < il[which].n_sets; ++si) {
+        const ElemSet& e = E.s[si];
+        if (four_rhs(e.R) != four) continue;
+        G.s[k++] = e;
+        n = std::max(n, e.n);
+        R = std::max(R, e.R);
+        m = std::max(m, (size_t)e.n * e.R);
+      }
+      if (k == 0) continue;
+      if (four)
+        k_residual_df_il4<X, RT><<<dim3((n + 7) / 8, (R + 127) / 128, k), 256, 0, s>>>(G, in_place);
+      else
+        k_residual_df_il<X, RT><<<dim3((unsigned)((m + 255) / 256), k), 256, 0, s>>>(G, in_place);
+      PECS_CUDA(cudaGetLastError());
     }
-    if (four)
-      k_residual_df_il4<X, RT><<<dim3((n + 7) / 8, (I.max_R + 127) / 128, I.n_sets), 256, 0, s>>>(E, in_place);
-    else
-      k_residual_df_il<X, RT><<<elem_grid(which), 256, 0, s>>>(E, in_place);
-    PECS_CUDA(cudaGetLastError());
   }
 
   void solve_bank_delta(const FactorBank& bank, int which, int target, cudaStream_t s) {
