@@ -128,11 +128,12 @@ __device__ __forceinline__ double rec_value(const RowRec& q, const RowSet& st, c
     u[j] = 0.0;
     if (q.slot[j] >= 0) u[j] = __ldcg(w + (size_t)q.slot[j] * R);
   }
-  // most positions have few children; the rest is skipped by whole warps, so that
-  // it does not pass through the FP64 unit
+  // most positions have few children; the rest is a branch, so that it does not pass
+  // through the FP64 unit where no lane of a warp has more (a vote of the whole warp in
+  // its place, behind the records' loads: 16x16 junction 26.73 ms for 100 steps, 26.55)
   double s = u[0];
   if (q.slot[1] >= 0) s += u[1];
-  if (__any_sync(__activemask(), q.slot[2] >= 0)) {
+  if (q.slot[2] >= 0) {
 #pragma unroll
     for (int j = 2; j < kRowsSlots; ++j)
       if (q.slot[j] >= 0) s += u[j];
