@@ -21,7 +21,7 @@ void parallel_nodes(int n, F f) {
 }
 }  // namespace
 
-PanelTilesPlan plan_panel(const std::vector<const MfFactor*>& factors, int chunks, int min_ctas) {
+PanelTilesPlan plan_panel(const std::vector<const MfFactor*>& factors, int chunks, int min_ctas, int most_rows) {
   PanelTilesPlan P;
   const int n_sets = (int)factors.size();
   int n_levels = 0;
@@ -80,10 +80,10 @@ PanelTilesPlan plan_panel(const std::vector<const MfFactor*>& factors, int chunk
       const auto& nodes = lv[fwd ? l : n_levels - 1 - l];
       L.first = (int)D.tiles.size();
       auto rows_of = [&](const MfNode& x) { return fwd ? x.s + x.m : x.s; };
-      // 32-row tiles, 16 where those are fewer than min_ctas
+      // tiles of most_rows rows, half of them where those are fewer than min_ctas
       long long n = 0;
-      for (auto [q, j] : nodes) n += (rows_of(factors[q]->nodes[j]) + 31) / 32;
-      const int cap = n * chunks < min_ctas ? 16 : 32;
+      for (auto [q, j] : nodes) n += (rows_of(factors[q]->nodes[j]) + most_rows - 1) / most_rows;
+      const int cap = most_rows > kPanelRowsF64 && n * chunks < min_ctas ? most_rows / 2 : most_rows;
       for (auto [q, j] : nodes) {
         const MfNode& x = factors[q]->nodes[j];
         const NodeSpans& sp = P.spans[P.base[q] + j];
@@ -99,7 +99,7 @@ PanelTilesPlan plan_panel(const std::vector<const MfFactor*>& factors, int chunk
           PanelTile t{};
           t.off = D.n_values;
           t.rows = r1 - r0;
-          t.pad = t.rows <= 8 ? 8 : (t.rows <= 16 ? 16 : 32);
+          t.pad = cap <= 4 ? 4 : t.rows <= 8 ? 8 : (t.rows <= 16 ? 16 : 32);
           t.cols = K;
           t.set = q;
           t.idx = (int)D.idx.size();

@@ -664,7 +664,9 @@ __global__ void __launch_bounds__(kSolveThreads)
   const auto& st = S.set[I.set];
   const int c0 = (int)blockIdx.y * (32 << P.lg_nw);
   if (c0 >= st.nrhs) return;
-  if (I.pad == 32)
+  if constexpr (sizeof(T) == 8)
+    tile_apply<T, 1, FWD>(B, st, I, P, c0, smem_raw);
+  else if (I.pad == 32)
     tile_apply<T, 8, FWD>(B, st, I, P, c0, smem_raw);
   else if (I.pad == 16)
     tile_apply<T, 4, FWD>(B, st, I, P, c0, smem_raw);
@@ -1436,7 +1438,8 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
   }
   {
     // level plans: tiles of packed values (panel_plan.hpp), and leaf warps
-    const PanelTilesPlan H = plan_panel(factors, (std::max(1, max_nrhs) + 31) / 32, tune_.min_ctas);
+    const PanelTilesPlan H = plan_panel(factors, (std::max(1, max_nrhs) + 31) / 32, tune_.min_ctas,
+                                        prec_ == PECS_PREC_FP64 ? kPanelRowsF64 : kPanelRowsF32);
     const int esz = prec_ == PECS_PREC_FP64 ? 8 : 4;
     rec_.upload(H.rec);
     more_.upload(H.more);

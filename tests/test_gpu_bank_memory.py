@@ -36,7 +36,7 @@ def test_one_form_of_the_factors_stays(pecs_lib, kw):
     if list(b.info().flow_rpl) != [0, 0]:
         pytest.skip("a flow sweep was chosen: it keeps a form of its own")
     print(few / MIB, f_few / MIB, many / MIB, f_many / MIB)
-    assert f_many > 150 * MIB and 0.8 < f_many / f_few < 1.2
+    assert f_many > 2 * 48 * MIB and 0.8 < f_many / f_few < 1.2  # a second form could not hide in the allowance
     assert many < few * 16 / 15 + 48 * MIB
     for ctx in (a, b):
         ctx.initialize()
