@@ -768,17 +768,21 @@ void Setup::compute_instance_data(const pecs_params& Pi, InstanceData& d, int th
       const CarrierSystem& CS = reg == 0 ? semi : elec;
       const Grid& g = CS.grid;
       const int nc = g.nc();
-      // generation rows, the same for both carriers: one evaluation per quadrature
-      // point (an exponential each; per basis function and carrier they took nearly
-      // all of the 5.8 ms of a 64x64+64x64 instance)
-      std::vector<double> gen;
-      if (reg == 0 && Pi.gen_kind != 0) {
-        gen.resize((size_t)nc * n1);
+      // generation rows, the same for both carriers: evaluated once per quadrature point,
+      // in the first carrier's loop (an exponential each; per basis function and carrier they
+      // took nearly all of the 5.8 ms of a 64x64+64x64 instance)
+      const bool generates = reg == 0 && Pi.gen_kind != 0;
+      std::vector<double> gen(generates ? (size_t)nc * n1 : 0);
+      for (int cc = 0; cc < 2; ++cc) {
+        int fld = 2 * reg + cc;
+        std::vector<double> b(CS.ndofs, 0.0);
+        // every cell writes only its own rows of b (and gen)
         par_range(nc, threads, [&](int K0, int K1) {
-          std::vector<double> gq(Q);
-          for (int K = K0; K < K1; ++K) {
-            double x0, y0, hx, hy;
-            g.geom(K, x0, y0, hx, hy);
+        std::vector<double> gq(Q);
+        for (int K = K0; K < K1; ++K) {
+          double x0, y0, hx, hy;
+          g.geom(K, x0, y0, hx, hy);
+          if (generates && cc == 0) {
             for (int q = 0; q < Q; ++q) gq[q] = generation(Pi, x0 + hx * ct.qx[q], y0 + hy * ct.qy[q]);
             for (int a = 0; a < n1; ++a) {
               double sacc = 0.0;
@@ -786,17 +790,8 @@ void Setup::compute_instance_data(const pecs_params& Pi, InstanceData& d, int th
               gen[(size_t)K * n1 + a] = sacc;
             }
           }
-        });
-      }
-      for (int cc = 0; cc < 2; ++cc) {
-        int fld = 2 * reg + cc;
-        std::vector<double> b(CS.ndofs, 0.0);
-        if (!gen.empty()) std::copy(gen.begin(), gen.end(), b.begin() + 2 * (size_t)nc * n1);
-        // every cell writes only its own rows of b
-        par_range(nc, threads, [&](int K0, int K1) {
-        for (int K = K0; K < K1; ++K) {
-          double x0, y0, hx, hy;
-          g.geom(K, x0, y0, hx, hy);
+          if (generates)
+            for (int a = 0; a < n1; ++a) b[2 * (size_t)nc * n1 + (size_t)K * n1 + a] = gen[(size_t)K * n1 + a];
           double diam = std::sqrt(hx * hx + hy * hy);
           for (int f = 0; f < 4; ++f) {
             if (g.face_bid(K, f) != kDirichlet) continue;
