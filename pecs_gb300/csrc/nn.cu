@@ -19,6 +19,7 @@
 #include <memory>
 #include <random>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "common.hpp"
@@ -111,23 +112,24 @@ void gemm(int M, int N, int K, const TAe* A, int lda, const TBe* B, int ldb, flo
 
 // ---- tensor-core GEMM: tcgen05.mma, BF16 operands, FP32 accumulator in TMEM ----
 // The layers' GEMMs op(A) op(B) with BF16-rounded operands run on the
-// 5th-generation tensor cores.  They are small (at most batch x 1024 x 1024), so
-// the latency of one tile and the number of SMs that have one decide: a CTA owns a
-// 128 x 32 tile of C (32 TMEM columns; 88 tiles of a 256 x 704 layer, where 128
-// columns gave 12).  Per K chunk of 64 its 256 threads convert op(A) (128 x 64) and
-// op(B)^T (32 x 64) to BF16, eight K values per 16-byte store, into the canonical
-// K-major layout without swizzle (8-row x 16-byte core matrices; K-adjacent core
-// matrices 128 B apart, 8-row groups 1024 B apart), one thread issues four
-// tcgen05.mma (K = 16 each) and commits them to the buffer's mbarrier, and the loads
-// of the next two chunks run under them (two buffers, three register sets).  Waits poll a bounded number of
-// times: one that runs out sets the error flag, the tile is skipped and the TMEM is
-// still freed.  The epilogue reads the accumulator with tcgen05.ld (warp w: TMEM
-// lanes 32 (w % 4).. = rows, half of the columns each).  Measured at batch 256 with
-// 6-704-704-704-64 layers against 128 x 128 tiles staged value by value: the forward
-// pass and its call 488 -> 91 us, loss and gradients without their copy to the host
-// 1,025 -> 161 us; the sums are the same bits.
+// 5th-generation tensor cores.  Most are small (batch 256 x 704 x 704), so the latency
+// of one tile and the number of SMs that have one decide: a CTA owns a 128 x 32 tile
+// of C (32 TMEM columns; 88 tiles of a 256 x 704 layer, where 128 columns gave 12), and
+// forward, where those are more than the SMs, 64 or 128 columns (Mlp::forward).  Per K
+// chunk of 64 its 256 threads convert op(A) (128 x 64) and op(B)^T (a row per column) to
+// BF16, eight K values per 16-byte store, into the canonical K-major layout without
+// swizzle (8-row x 16-byte core matrices; K-adjacent core matrices 128 B apart, 8-row
+// groups 1024 B apart), one thread issues four tcgen05.mma (K = 16 each) and commits
+// them to the buffer's mbarrier, and the loads of the next two chunks run under them
+// (two buffers, three register sets).  Waits poll a bounded number of times: one that
+// runs out sets the error flag, the tile is skipped and the TMEM is still freed.  The
+// epilogue reads the accumulator with tcgen05.ld (warp w: TMEM lanes 32 (w % 4).. =
+// rows, 16 of each 32 columns).  Measured at batch 256 with 6-704-704-704-64 layers
+// against 128 x 128 tiles staged value by value: the forward pass and its call 488 -> 91
+// us, loss and gradients without their copy to the host 1,025 -> 161 us; the sums are
+// the same bits.
 constexpr int kTcM = 128, kTcN = 32, kTcK = 64, kTcThreads = 256;
-constexpr uint32_t kTcCols = 32;
+constexpr int kTcSms = 152;  // multiprocessors of a GB300
 constexpr long long kTcPollLimit = 1LL << 24;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -212,25 +214,26 @@ struct Raw8Of<__nv_bfloat16> {
   using type = Raw8H;
 };
 
+template <int TN>
 struct GemmSmem {
   __align__(1024) unsigned char a[2][kTcM * kTcK * 2];
-  __align__(1024) unsigned char b[2][kTcN * kTcK * 2];
+  __align__(1024) unsigned char b[2][TN * kTcK * 2];
   __align__(8) unsigned long long mbar[2];
   uint32_t tmem;
 };
 
-// One 128 x 32 tile at (m0, n0) of op(A)[M,K] op(B)[K,N]: op(A)(m,k) = TA ?
+// One 128 x TN tile at (m0, n0) of op(A)[M,K] op(B)[K,N]: op(A)(m,k) = TA ?
 // A[k*lda+m] : A[m*lda+k]; op(B)(k,n) = TB ? B[n*ldb+k] : B[k*ldb+n].  wait() is
 // called before the first operand is read.  epilogue(row, column, values[16]) gets
 // the sums of one row's columns [column, column + 16).
-template <typename TAe, typename TBe, bool TA, bool TB, typename Wait, typename Epi>
-__device__ __forceinline__ void gemm_tile(GemmSmem& s, int M, int N, int K, const TAe* __restrict__ A, int lda,
+template <typename TAe, typename TBe, bool TA, bool TB, int TN, typename Wait, typename Epi>
+__device__ __forceinline__ void gemm_tile(GemmSmem<TN>& s, int M, int N, int K, const TAe* __restrict__ A, int lda,
                                           const TBe* __restrict__ B, int ldb, int m0, int n0, int* err, Wait wait,
                                           Epi epilogue) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s.tmem)),
-                 "r"(kTcCols)
+                 "r"((uint32_t)TN)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
@@ -239,7 +242,7 @@ __device__ __forceinline__ void gemm_tile(GemmSmem& s, int M, int N, int K, cons
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar[0]) : "memory");
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar[1]) : "memory");
   }
-  // this thread's 16-byte pieces: four of A, one of B.  Along K-contiguous
+  // this thread's 16-byte pieces: four of A, one of B per 32 columns.  Along K-contiguous
   // operands lanes take 8 rows x 4 pieces (whole sectors, and shared-memory stores
   // without bank conflicts), else consecutive rows.
   const bool va = lda % 4 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
@@ -253,9 +256,10 @@ __device__ __forceinline__ void gemm_tile(GemmSmem& s, int M, int N, int K, cons
       k8 = idx / rows;
     }
   };
+  constexpr int NB = TN / 32;
   struct Set {
     typename Raw8Of<TAe>::type a[4];
-    typename Raw8Of<TBe>::type b;
+    typename Raw8Of<TBe>::type b[NB];
   } set[3];
   auto load = [&](Set& r, int k0) {
 #pragma unroll
@@ -265,10 +269,13 @@ __device__ __forceinline__ void gemm_tile(GemmSmem& s, int M, int N, int K, cons
       const int m = m0 + row, k = k0 + k8 * 8, n = m < M ? min(8, K - k) : 0;
       r.a[q].template load<!TA>(TA ? A + (size_t)k * lda + m : A + (size_t)m * lda + k, lda, n, va);
     }
-    int row, k8;
-    place(TB, tid, kTcN, row, k8);
-    const int c = n0 + row, k = k0 + k8 * 8, n = c < N ? min(8, K - k) : 0;
-    r.b.template load<TB>(TB ? B + (size_t)c * ldb + k : B + (size_t)k * ldb + c, ldb, n, vb);
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      int row, k8;
+      place(TB, tid + q * kTcThreads, TN, row, k8);
+      const int c = n0 + row, k = k0 + k8 * 8, n = c < N ? min(8, K - k) : 0;
+      r.b[q].template load<TB>(TB ? B + (size_t)c * ldb + k : B + (size_t)k * ldb + c, ldb, n, vb);
+    }
   };
   auto piece = [](int row, int k8) { return (row >> 3) * 1024 + k8 * 128 + (row & 7) * 16; };
   const int nk = (K + kTcK - 1) / kTcK;
@@ -280,8 +287,8 @@ __device__ __forceinline__ void gemm_tile(GemmSmem& s, int M, int N, int K, cons
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   const uint32_t tmem = s.tmem;
   // instruction descriptor (kind::f16): FP32 accumulator, BF16 A and B, both
-  // K-major, N = 32, M = 128
-  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTcN >> 3) << 17) |
+  // K-major, N = TN, M = 128
+  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) |
                          ((uint32_t)(kTcM >> 4) << 24);
   bool ok = true;
   // chunk kc from registers `cur` into shared memory and multiplied, while the
@@ -296,10 +303,11 @@ __device__ __forceinline__ void gemm_tile(GemmSmem& s, int M, int N, int K, cons
       place(!TA, tid + q * kTcThreads, kTcM, row, k8);
       *reinterpret_cast<uint4*>(s.a[buf] + piece(row, k8)) = cur.a[q].pack();
     }
-    {
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
       int row, k8;
-      place(TB, tid, kTcN, row, k8);
-      *reinterpret_cast<uint4*>(s.b[buf] + piece(row, k8)) = cur.b.pack();
+      place(TB, tid + q * kTcThreads, TN, row, k8);
+      *reinterpret_cast<uint4*>(s.b[buf] + piece(row, k8)) = cur.b[q].pack();
     }
     // the staged tiles are read by the tensor cores (async proxy)
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -334,23 +342,27 @@ __device__ __forceinline__ void gemm_tile(GemmSmem& s, int M, int N, int K, cons
     if (tid == 0) atomicExch(err, 1);
     tc_wait(bar[(nk - 1) & 1], ((nk - 1) >> 1) & 1);  // MMAs still in flight (bounded) before the TMEM is freed
   } else {
-    const int row = m0 + (warp & 3) * 32 + lane, c0 = (warp >> 2) * 16;
-    uint32_t v[16];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                 : "r"(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0)
-                 : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-    float f[16];
+    const int row = m0 + (warp & 3) * 32 + lane;
+#pragma unroll 1
+    for (int c0 = (warp >> 2) * 16; c0 < TN; c0 += 32) {
+      uint32_t v[16];
+      asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+                   : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                     "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                   : "r"(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0)
+                   : "memory");
+      asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+      float f[16];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) f[j] = __uint_as_float(v[j]);
-    if (row < M) epilogue(row, n0 + c0, f);
+      for (int j = 0; j < 16; ++j) f[j] = __uint_as_float(v[j]);
+      if (row < M) epilogue(row, n0 + c0, f);
+      __syncwarp();
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kTcCols) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"((uint32_t)TN) : "memory");
 }
 
 // 16 consecutive values of one row, those below column N
@@ -372,12 +384,14 @@ __device__ __forceinline__ void next_may_launch() { asm volatile("griddepcontrol
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
 // Y (B x N) = X (B x K) W^T + bias, W stored N x K; act: tanh.
+template <int TN>
 __global__ void __launch_bounds__(kTcThreads)
     k_mlp_layer(int B, int N, int K, const float* __restrict__ X, const __nv_bfloat16* __restrict__ W,
                 const float* __restrict__ bias, int act, float* __restrict__ Y, int* err) {
-  __shared__ GemmSmem s;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  GemmSmem<TN>& s = *reinterpret_cast<GemmSmem<TN>*>(smem_raw);
   next_may_launch();
-  gemm_tile<float, __nv_bfloat16, false, true>(s, B, N, K, X, K, W, K, (int)blockIdx.y * kTcM, (int)blockIdx.x * kTcN,
+  gemm_tile<float, __nv_bfloat16, false, true>(s, B, N, K, X, K, W, K, (int)blockIdx.y * kTcM, (int)blockIdx.x * TN,
                                                err, [] { wait_previous(); }, [&](int row, int n, float (&f)[16]) {
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
@@ -395,7 +409,7 @@ __global__ void __launch_bounds__(kTcThreads)
     k_mlp_layer_bwd(int B, int N, int K, const float* __restrict__ dZ, const float* __restrict__ X,
                     const __nv_bfloat16* __restrict__ W, float* __restrict__ dW, float* __restrict__ db,
                     float* __restrict__ dX, int w_blocks, int x_blocks, int* err) {
-  __shared__ GemmSmem s;
+  __shared__ GemmSmem<kTcN> s;
   next_may_launch();
   const int nk = (K + kTcN - 1) / kTcN;  // column tiles of both products
   int q = blockIdx.x;
@@ -436,13 +450,14 @@ __global__ void __launch_bounds__(kTcThreads)
 }
 
 template <typename... P, typename... A>
-void launch_after(void (*fn)(P...), dim3 grid, cudaStream_t st, A... args) {
+void launch_after(void (*fn)(P...), dim3 grid, size_t smem, cudaStream_t st, A... args) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(kTcThreads);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
@@ -553,11 +568,30 @@ struct Mlp {
       PECS_CUDA(cudaMemcpyAsync(y, act.back().p, ny, cudaMemcpyDeviceToDevice, s));
       return;
     }
-    for (int l = 0; l < L; ++l)
+    for (int l = 0; l < L; ++l) {
       // act[l+1] = act(act[l] W_l^T + b_l); W_l stored out x in (row-major)
-      launch_after(k_mlp_layer, dim3(tiles(w[l + 1], kTcN), tiles(B, kTcM)), s, B, w[l + 1], w[l],
-                   l == 0 ? x : (const float*)act[l].p, Wb(l), bias(l), l < L - 1 ? 1 : 0,
-                   l == L - 1 && y ? y : act[l + 1].p, &host->err);
+      auto go = [&](auto tn) {
+        constexpr int TN = decltype(tn)::value;
+        constexpr size_t smem = sizeof(GemmSmem<TN>);
+        if (smem > 48 * 1024)
+          PECS_CUDA(cudaFuncSetAttribute(k_mlp_layer<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        launch_after(k_mlp_layer<TN>, dim3(tiles(w[l + 1], TN), tiles(B, kTcM)), smem, s, B, w[l + 1], w[l],
+                     l == 0 ? x : (const float*)act[l].p, Wb(l), bias(l), l < L - 1 ? 1 : 0,
+                     l == L - 1 && y ? y : act[l + 1].p, &host->err);
+      };
+      // The narrowest tile that leaves no more tiles than SMs (none wider than the layer):
+      // with fewer tiles SMs idle, with more the activations are converted again for every
+      // tile of a row.  us per forward pass for 32 / 64 / 128 columns: 6-704-704-704-64,
+      // batch 256 90 / 108 / 134, 1,000 134 / 108 / 134, 4,096 287 / 231 / 217;
+      // 64-2048-2048-64, batch 256 140 / 165 / 194, 512 204 / 165 / 195, 4,096 968 / 630 / 498.
+      auto fits = [&](int tn) { return w[l + 1] <= tn || tiles(w[l + 1], tn) * (long long)tiles(B, kTcM) <= kTcSms; };
+      if (fits(32))
+        go(std::integral_constant<int, 32>());
+      else if (fits(64))
+        go(std::integral_constant<int, 64>());
+      else
+        go(std::integral_constant<int, 128>());
+    }
   }
 
   // gradients of mean((y - t)^2) into G; the loss's partial sums into host->loss
@@ -569,7 +603,7 @@ struct Mlp {
     for (int l = L - 1; l >= 0; --l) {
       const int N = w[l + 1], K = w[l], wb = tiles(N, kTcM) * tiles(K, kTcN),
                 xb = l > 0 ? tiles(B, kTcM) * tiles(K, kTcN) : 0;
-      launch_after(k_mlp_layer_bwd, dim3(wb + xb + tiles(N, kTcThreads)), s, B, N, K, (const float*)dact[l + 1].p,
+      launch_after(k_mlp_layer_bwd, dim3(wb + xb + tiles(N, kTcThreads)), 0, s, B, N, K, (const float*)dact[l + 1].p,
                    l == 0 ? x : (const float*)act[l].p, Wb(l), G.p + woff[l], G.p + boff[l],
                    l > 0 ? dact[l].p : nullptr, wb, xb, &host->err);
     }
