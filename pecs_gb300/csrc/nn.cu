@@ -858,6 +858,37 @@ __global__ void __launch_bounds__(256, 4)
   }
 }
 
+// Few outputs of few coefficients: a thread per value.  Bound by its launch; the tiles'
+// staging and their 32 values per thread take 2 to 6 us more: n_u = 64, r = 3, batch 256 25.2
+// -> 19.0 us the call, n_u = 1,000, r = 17, batch 16 24.7 -> 19.1.  The tiles are faster from
+// kWsFew densities on (n_u = 1,000, batch 256: 25.0 against 26.6), and where a thread's
+// coefficients are more than a stage (n_u = 16,384, r = 64, batch 1: 25.3 against 35.2: its
+// loads of V are not coalesced).  The same sums in the same order.
+constexpr long long kWsFew = 1 << 18;
+
+__global__ void __launch_bounds__(256)
+    k_warm_start_few(int r, int n_u, const float* __restrict__ c, const float* __restrict__ V,
+                     const float* __restrict__ mean, int nd, int u_off, double* __restrict__ vn,
+                     double* __restrict__ vp) {
+  __shared__ float cs[kWsK];
+  const size_t row = blockIdx.y;
+  if ((int)threadIdx.x < r) cs[threadIdx.x] = c[row * r + threadIdx.x];
+  __syncthreads();
+  for (long long t = blockIdx.x * 256 + threadIdx.x; t < 2LL * nd; t += (long long)gridDim.x * 256) {
+    const bool hole = t >= nd;
+    const int d = (int)(hole ? t - nd : t), i = d - u_off;
+    double x = 0.0;
+    if (i >= 0 && i < n_u) {
+      const int o = hole ? n_u + i : i;
+      const float* v = V + (size_t)o * r;
+      float y = mean[o];
+      for (int j = 0; j < r; ++j) y = fmaf(v[j], cs[j], y);
+      x = f2d_exact(expf(y));
+    }
+    (hole ? vp : vn)[row * nd + d] = x;
+  }
+}
+
 // FP32 decoder: y (batch x n) = mean (n) + c (batch x r) V^T, V stored n x r (row-major)
 int pecs_decode(int batch, int r, int n, const float* c_dev, const float* V_dev, const float* mean_dev,
                 float* y_dev, void* stream) {
@@ -882,6 +913,13 @@ int pecs_warm_start_vectors(int batch, int r, int n_u, const float* c_dev, const
         !mean_dev || !vn_dev || !vp_dev)
       throw PecsError(PECS_E_ARG, "invalid arguments");
     cudaStream_t s = (cudaStream_t)stream;
+    if (r <= kWsK && batch <= 65535 && 2LL * n_u * batch <= kWsFew) {
+      const unsigned nx = (unsigned)std::min<long long>((2LL * nd + 255) / 256, 1024);
+      k_warm_start_few<<<dim3(nx, batch), 256, 0, s>>>(r, n_u, c_dev, V_dev, mean_dev, nd, u_off, vn_dev, vp_dev);
+      PECS_CUDA(cudaGetLastError());
+      PECS_CUDA(cudaStreamSynchronize(s));
+      return PECS_OK;
+    }
     const long long n_tiles = (2LL * n_u + kWsOut - 1) / kWsOut, b_tiles = (batch + kWsRows - 1) / kWsRows;
     const long long z_parts = ((long long)(nd - n_u) + kWsZeros - 1) / kWsZeros;
     const long long blocks = n_tiles * b_tiles + 2LL * batch * z_parts;
