@@ -126,9 +126,11 @@ typedef struct pecs_options {
   int host_setup_only; /* 1: build meshes, matrices and factors on the host only
                           (no device work; for inspecting the setup) */
   int panel_chunk;     /* panel solve kernels (>= 32 right-hand sides per factor): staged
-                          block columns per chunk (0 = default: 128 FP32, 64 FP64) */
-  int panel_min_ctas;  /* panel solve kernels: CTAs a level must reach before shorter row
-                          tiles or fewer right-hand sides per CTA are used (0 = default 152) */
+                          block columns per chunk, at most 128 (0 = default: what shared
+                          memory holds) */
+  int panel_min_ctas;  /* panel solve kernels: CTAs that a level with fewer takes shorter row
+                          tiles (FP32) or fewer right-hand sides per CTA for (0 = default
+                          152) */
   int autotune;        /* panel solve kernels: at creation, choose every tree level's
                           tiling by timing whole sweeps (1 = yes, the default;
                           0 = the heuristic above) */
@@ -147,7 +149,8 @@ typedef struct pecs_options {
                            one FP32 sweep, u = u_prev + increment -- instead of a sweep and a
                            refinement sweep from zero; the residual vanishes at the fixed
                            point, which is therefore the refined mixed mode's.  Initial and
-                           refill solves keep the refinement.  (1 = on, 0 = default: off) */
+                           refill solves keep the refinement, and so do all solves of factors
+                           with fewer than 32 right-hand sides.  (1 = on, 0 = default: off) */
 } pecs_options;
 
 typedef struct pecs_info {
@@ -156,7 +159,7 @@ typedef struct pecs_info {
   long long factor_entries[3]; /* stored entries: semi carriers, elec carriers, Poisson */
   int factor_levels[3];
   int factor_nodes[3];
-  long long factor_bytes;  /* device bytes of all factors */
+  long long factor_bytes;  /* device bytes of the factor values held */
   double setup_seconds;    /* host assembly + factorisation */
   int n_distinct_carrier_factors;
   int launches_per_step;   /* kernel launches of one step incl. steady-state test */

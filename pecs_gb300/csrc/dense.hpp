@@ -8,6 +8,8 @@
 // vectorises the micro-kernel on x86-64 and aarch64 alike.
 #pragma once
 
+#include <algorithm>
+#include <atomic>
 #include <condition_variable>
 #include <functional>
 #include <mutex>
@@ -44,6 +46,17 @@ class Team {
 // Runs fn(t) for t in [0, n) on n threads (the caller takes t = 0) and joins
 // them; if starting a thread fails, joins the started ones and rethrows.
 void run_threads(int n, const std::function<void(int)>& fn);
+
+// f(i) for i in [0, n), handed out one at a time, on a host thread per `each` of them (16 at
+// most): a thread takes about as long to start as 64 nodes of a small mesh to plan.
+template <typename F>
+void parallel_for(int n, int each, F f) {
+  const int most = (int)std::max(1u, std::min(std::thread::hardware_concurrency(), 16u));
+  std::atomic<int> next(0);
+  run_threads(std::max(1, std::min(most, n / each)), [&](int) {
+    for (int i; (i = next.fetch_add(1)) < n;) f(i);
+  });
+}
 
 // C[M x N] += alpha * A[M x K] * B[K x N]; threads from `team` (may be null).
 void gemm(int M, int N, int K, double alpha, const double* A, int lda, const double* B, int ldb,

@@ -9,10 +9,11 @@
 //   bconst[field]    time-independent RHS parts (generation, Dirichlet data,
 //                    doping), per instance.
 //   carrier and Poisson FactorBanks (solve.cuh) + per-RHS update workspaces.
-// A step is: carrier RHS (1 launch) -> carrier solves (one launch per tree
-// level for all carriers and instances) -> Poisson RHS (1) -> Poisson solve
-// -> steady-state reduction (2) + snapshot (1).  pecs_run_to_steady_state
-// replays a CUDA graph of two steps (even/odd ping-pong).
+// A step is: carrier RHS (1 launch) -> carrier solves (one or two launches per
+// tree level for all carriers and instances) -> Poisson RHS (1) -> Poisson solve
+// -> changes (1; none where increment solves add them up), steady-state test (1)
+// + snapshot (1).  pecs_run_to_steady_state replays a CUDA graph of two steps
+// (even/odd ping-pong).
 #include <cuda_runtime.h>
 #include <sys/mman.h>
 #include <unistd.h>
@@ -196,7 +197,7 @@ __global__ void __launch_bounds__(256) k_gather_pairs_il(ElemSets E) {
 struct ChangeSums {
   double2* out = nullptr;
   int stride = 0;
-  int first[kMaxSets] = {}, fields[kMaxSets] = {};  // field slots of each set's columns
+  int first[kMaxSets] = {};  // each set's first field slot
 };
 
 // dst_k[d] = old_k[d] + D32[d * R + k]: the previous step's solution plus the
@@ -353,9 +354,9 @@ __global__ void k_residual_df_il(ElemSets E, int in_place) {
 // pairs' arithmetic keeps the FMA pipe and the x rows the L1 busy about half of the time
 // each: 49,152 rows x 128 right-hand sides x 2 sets take 155 us with the right-hand
 // sides of the CTA's eight rows read together, 169 with each row's by its own lanes.
-// Tried without gain: two right-hand sides per instruction (f32x2) and two or
-// four entries in flight (12 and 30 us more: fewer warps), the x rows of the eight rows
-// staged in shared memory (8 us more).
+// Tried without gain, us a step of 64 instances (1,000): two right-hand sides per
+// instruction (f32x2) and two or four entries in flight (12 and 42 more: fewer warps), the
+// x rows of the eight rows staged in shared memory (8 more).
 __device__ __forceinline__ void ld_pairs4(const float* p, float2 (&v)[4]) {
   const float4 t = *reinterpret_cast<const float4*>(p);
   v[0] = make_float2(t.x, 0.f);
@@ -1029,9 +1030,8 @@ struct Engine {
       C.stride = partial_stride;
       const IlBank& I = il[which];
       for (int si = 0; si < I.n_sets; ++si) {
-        C.fields[si] = I.set[si].R / n_inst;
         C.first[si] = which == 1 ? n_fields - 1 : I.set[si].mat;
-        for (int f = 0; f < C.fields[si]; ++f)
+        for (int f = 0; f < I.set[si].R / n_inst; ++f)
           change_chunks.n[C.first[si] + f] = (I.set[si].n + 32 * kDeltaTiles - 1) / (32 * kDeltaTiles);
       }
       k_scatter_delta_il<true><<<dg, tb, 0, s>>>(E, scatter_mask, n_inst, C);

@@ -22,29 +22,20 @@
 #include <type_traits>
 #include <vector>
 
+#include "bulk_copy.cuh"
 #include "common.hpp"
 #include "fp_bits.cuh"
+#include "sweep_sync.cuh"
 
 namespace pecs {
 namespace {
 
 constexpr int kBM = 64, kBN = 64, kBK = 16, kGemmThreads = 256;
 
-template <typename T>
-__device__ __forceinline__ float to_f(T v);
-template <>
-__device__ __forceinline__ float to_f<float>(float v) { return v; }
-
-__device__ __forceinline__ float round_bf16(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-
-// C[M,N] = alpha * op(A)[M,K] op(B)[K,N] + beta * C + bias[n], then act.
-// op(A)(m,k) = TA ? A[k*lda+m] : A[m*lda+k]; op(B)(k,n) = TB ? B[n*ldb+k] : B[k*ldb+n].
-// kBf16In rounds both operands to BF16 before the product (FP32 accumulate).
-template <typename TAe, typename TBe, bool TA, bool TB, bool kBf16In>
+// The decoder's GEMM in FP32: C[M,N] = A[M,K] B[N,K]^T + mean[n].
 __global__ void __launch_bounds__(kGemmThreads)
-    k_gemm(int M, int N, int K, const TAe* __restrict__ A, int lda, const TBe* __restrict__ B, int ldb,
-           float* __restrict__ C, int ldc, float alpha, float beta, const float* __restrict__ bias,
-           int act) {
+    k_decode(int M, int N, int K, const float* __restrict__ A, const float* __restrict__ B,
+             const float* __restrict__ mean, float* __restrict__ C) {
   __shared__ float As[kBK][kBM + 1];
   __shared__ float Bs[kBK][kBN + 1];
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
@@ -56,18 +47,12 @@ __global__ void __launch_bounds__(kGemmThreads)
     for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
   for (int k0 = 0; k0 < K; k0 += kBK) {
     for (int t = threadIdx.x; t < kBK * kBM; t += kGemmThreads) {
-      const int kk = t % kBK, mm = t / kBK;
-      const int m = m0 + mm, k = k0 + kk;
-      float v = 0.f;
-      if (m < M && k < K) v = to_f(TA ? A[(size_t)k * lda + m] : A[(size_t)m * lda + k]);
-      As[kk][mm] = kBf16In ? round_bf16(v) : v;
+      const int kk = t % kBK, mm = t / kBK, m = m0 + mm, k = k0 + kk;
+      As[kk][mm] = m < M && k < K ? A[(size_t)m * K + k] : 0.f;
     }
     for (int t = threadIdx.x; t < kBK * kBN; t += kGemmThreads) {
-      const int nn = t % kBN, kk = t / kBN;
-      const int n = n0 + nn, k = k0 + kk;
-      float v = 0.f;
-      if (n < N && k < K) v = to_f(TB ? B[(size_t)n * ldb + k] : B[(size_t)k * ldb + n]);
-      Bs[kk][nn] = kBf16In ? round_bf16(v) : v;
+      const int nn = t % kBN, kk = t / kBN, n = n0 + nn, k = k0 + kk;
+      Bs[kk][nn] = n < N && k < K ? B[(size_t)n * K + k] : 0.f;
     }
     __syncthreads();
 #pragma unroll
@@ -91,23 +76,9 @@ __global__ void __launch_bounds__(kGemmThreads)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int n = n0 + tx * 4 + j;
-      if (n >= N) continue;
-      float v = alpha * acc[i][j];
-      if (beta != 0.f) v += beta * C[(size_t)m * ldc + n];
-      if (bias) v += bias[n];
-      if (act == 1) v = tanhf(v);
-      C[(size_t)m * ldc + n] = v;
+      if (n < N) C[(size_t)m * N + n] = acc[i][j] + mean[n];
     }
   }
-}
-
-template <typename TAe, typename TBe, bool TA, bool TB, bool kBf16In>
-void gemm(int M, int N, int K, const TAe* A, int lda, const TBe* B, int ldb, float* C, int ldc,
-          float alpha, float beta, const float* bias, int act, cudaStream_t st) {
-  dim3 grid((N + kBN - 1) / kBN, (M + kBM - 1) / kBM);
-  k_gemm<TAe, TBe, TA, TB, kBf16In><<<grid, kGemmThreads, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc,
-                                                                    alpha, beta, bias, act);
-  PECS_CUDA(cudaGetLastError());
 }
 
 // ---- tensor-core GEMM: tcgen05.mma, BF16 operands, FP32 accumulator in TMEM ----
@@ -131,10 +102,6 @@ void gemm(int M, int N, int K, const TAe* A, int lda, const TBe* B, int ldb, flo
 constexpr int kTcM = 128, kTcN = 32, kTcK = 64, kTcThreads = 256;
 constexpr int kTcSms = 152;  // multiprocessors of a GB300
 constexpr long long kTcPollLimit = 1LL << 24;
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
 
 // shared-memory matrix descriptor: start address, leading-dimension byte
 // offset (K direction, 128 B), stride byte offset (8-row groups, 1024 B),
@@ -378,11 +345,6 @@ __device__ __forceinline__ void store16(float* __restrict__ C, int ldc, int N, i
   }
 }
 
-// The next kernel of a pass may be launched (its blocks set up) while this one
-// runs; before it reads anything it waits for this one's end.
-__device__ __forceinline__ void next_may_launch() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-
 // Y (B x N) = X (B x K) W^T + bias, W stored N x K; act: tanh.
 template <int TN>
 __global__ void __launch_bounds__(kTcThreads)
@@ -390,9 +352,9 @@ __global__ void __launch_bounds__(kTcThreads)
                 const float* __restrict__ bias, int act, float* __restrict__ Y, int* err) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   GemmSmem<TN>& s = *reinterpret_cast<GemmSmem<TN>*>(smem_raw);
-  next_may_launch();
+  pdl_trigger();
   gemm_tile<float, __nv_bfloat16, false, true>(s, B, N, K, X, K, W, K, (int)blockIdx.y * kTcM, (int)blockIdx.x * TN,
-                                               err, [] { wait_previous(); }, [&](int row, int n, float (&f)[16]) {
+                                               err, [] { pdl_wait(); }, [&](int row, int n, float (&f)[16]) {
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       if (n + j < N) f[j] += bias[n + j];
@@ -410,19 +372,19 @@ __global__ void __launch_bounds__(kTcThreads)
                     const __nv_bfloat16* __restrict__ W, float* __restrict__ dW, float* __restrict__ db,
                     float* __restrict__ dX, int w_blocks, int x_blocks, int* err) {
   __shared__ GemmSmem<kTcN> s;
-  next_may_launch();
+  pdl_trigger();
   const int nk = (K + kTcN - 1) / kTcN;  // column tiles of both products
   int q = blockIdx.x;
   if (q < w_blocks) {
     gemm_tile<float, float, true, false>(s, N, K, B, dZ, N, X, K, q / nk * kTcM, q % nk * kTcN, err,
-                                         [] { wait_previous(); },
+                                         [] { pdl_wait(); },
                                          [&](int row, int n, float (&f)[16]) { store16(dW, K, K, row, n, f); });
     return;
   }
   q -= w_blocks;
   if (q < x_blocks) {
     gemm_tile<float, __nv_bfloat16, false, false>(s, B, K, N, dZ, N, W, K, q / nk * kTcM, q % nk * kTcN, err,
-                                                  [] { wait_previous(); }, [&](int row, int n, float (&f)[16]) {
+                                                  [] { pdl_wait(); }, [&](int row, int n, float (&f)[16]) {
 #pragma unroll
       for (int j = 0; j < 16; ++j)
         if (n + j < K) {
@@ -434,7 +396,7 @@ __global__ void __launch_bounds__(kTcThreads)
     return;
   }
   q -= x_blocks;
-  wait_previous();
+  pdl_wait();
   const int n = q * kTcThreads + threadIdx.x;
   if (n >= N) return;
   float t = 0.f;
@@ -447,21 +409,6 @@ __global__ void __launch_bounds__(kTcThreads)
       if (b0 + j < B) t += v[j];
   }
   db[n] = t;
-}
-
-template <typename... P, typename... A>
-void launch_after(void (*fn)(P...), dim3 grid, size_t smem, cudaStream_t st, A... args) {
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(kTcThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  PECS_CUDA(cudaLaunchKernelEx(&cfg, fn, args...));
 }
 
 // dy = 2 (y - t) / (B N); per-block partial loss sums
@@ -502,11 +449,6 @@ __global__ void k_adam(float* __restrict__ w, float* __restrict__ m, float* __re
 __global__ void k_to_bf16(const float* __restrict__ w, __nv_bfloat16* __restrict__ wb, size_t n) {
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i < n) wb[i] = __float2bfloat16_rn(w[i]);
-}
-
-__global__ void k_add_rowvec(float* __restrict__ y, const float* __restrict__ mean, int B, int N) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i < (size_t)B * N) y[i] += mean[i % N];
 }
 
 }  // namespace
@@ -575,7 +517,7 @@ struct Mlp {
         constexpr size_t smem = sizeof(GemmSmem<TN>);
         if (smem > 48 * 1024)
           PECS_CUDA(cudaFuncSetAttribute(k_mlp_layer<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        launch_after(k_mlp_layer<TN>, dim3(tiles(w[l + 1], TN), tiles(B, kTcM)), smem, s, B, w[l + 1], w[l],
+        launch_pdl(k_mlp_layer<TN>, dim3(tiles(w[l + 1], TN), tiles(B, kTcM)), kTcThreads, smem, s, B, w[l + 1], w[l],
                      l == 0 ? x : (const float*)act[l].p, Wb(l), bias(l), l < L - 1 ? 1 : 0,
                      l == L - 1 && y ? y : act[l + 1].p, &host->err);
       };
@@ -603,7 +545,7 @@ struct Mlp {
     for (int l = L - 1; l >= 0; --l) {
       const int N = w[l + 1], K = w[l], wb = tiles(N, kTcM) * tiles(K, kTcN),
                 xb = l > 0 ? tiles(B, kTcM) * tiles(K, kTcN) : 0;
-      launch_after(k_mlp_layer_bwd, dim3(wb + xb + tiles(N, kTcThreads)), 0, s, B, N, K, (const float*)dact[l + 1].p,
+      launch_pdl(k_mlp_layer_bwd, dim3(wb + xb + tiles(N, kTcThreads)), kTcThreads, 0, s, B, N, K, (const float*)dact[l + 1].p,
                    l == 0 ? x : (const float*)act[l].p, Wb(l), G.p + woff[l], G.p + boff[l],
                    l > 0 ? dact[l].p : nullptr, wb, xb, &host->err);
     }
@@ -896,10 +838,8 @@ int pecs_decode(int batch, int r, int n, const float* c_dev, const float* V_dev,
     if (batch < 1 || r < 1 || n < 1 || !c_dev || !V_dev || !mean_dev || !y_dev)
       throw PecsError(PECS_E_ARG, "invalid arguments");
     cudaStream_t s = (cudaStream_t)stream;
-    gemm<float, float, false, true, false>(batch, n, r, c_dev, r, V_dev, r, y_dev, n, 1.f, 0.f, nullptr,
-                                           0, s);
-    const size_t tot = (size_t)batch * n;
-    k_add_rowvec<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(y_dev, mean_dev, batch, n);
+    k_decode<<<dim3((n + kBN - 1) / kBN, (batch + kBM - 1) / kBM), kGemmThreads, 0, s>>>(batch, n, r, c_dev, V_dev,
+                                                                                         mean_dev, y_dev);
     PECS_CUDA(cudaGetLastError());
     PECS_CUDA(cudaStreamSynchronize(s));
   })

@@ -2,24 +2,11 @@
 #include "panel_plan.hpp"
 
 #include <algorithm>
-#include <atomic>
 #include <stdexcept>
-#include <thread>
 
 #include "dense.hpp"
 
 namespace pecs {
-
-namespace {
-template <typename F>
-void parallel_nodes(int n, F f) {
-  const int threads = (int)std::max(1u, std::min(std::thread::hardware_concurrency(), 16u));
-  std::atomic<int> next(0);
-  dense::run_threads(std::max(1, std::min(threads, n / 8)), [&](int) {
-    for (int i; (i = next.fetch_add(1)) < n;) f(i);
-  });
-}
-}  // namespace
 
 PanelTilesPlan plan_panel(const std::vector<const MfFactor*>& factors, int chunks, int min_ctas, int most_rows) {
   PanelTilesPlan P;
@@ -33,7 +20,7 @@ PanelTilesPlan plan_panel(const std::vector<const MfFactor*>& factors, int chunk
     }
   }
   for (int q = 0; q < n_sets; ++q)
-    parallel_nodes((int)factors[q]->nodes.size(), [&](int j) { P.spans[P.base[q] + j] = node_spans(*factors[q], j); });
+    dense::parallel_for((int)factors[q]->nodes.size(), 64, [&](int j) { P.spans[P.base[q] + j] = node_spans(*factors[q], j); });
   // update slots, and the nodes of each height
   std::vector<std::vector<int>> w_off(n_sets);
   std::vector<std::vector<std::pair<int, int>>> lv(n_levels);  // (set, node), set by set
@@ -132,7 +119,7 @@ namespace {
 template <typename T>
 void pack(const PanelTilesPlan& P, const std::vector<const MfFactor*>& factors, int d, T* out) {
   const PanelTilesPlan::Dir& D = P.dir[d];
-  parallel_nodes((int)D.tiles.size(), [&](int i) {
+  dense::parallel_for((int)D.tiles.size(), 64, [&](int i) {
     const PanelTile& t = D.tiles[i];
     const MfFactor& F = *factors[t.set];
     const int j = D.node[i], s = F.nodes[j].s, f = s + F.nodes[j].m;

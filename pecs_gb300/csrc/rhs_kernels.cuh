@@ -87,15 +87,11 @@ struct Dims {
   static constexpr int nphi = KP * KP;
 };
 
-// state values into the quadrature type, and quadrature sums back: on the
-// integer pipe for the FP32 path (fp_bits.cuh), plain for FP64
+// state values into the quadrature type: on the integer pipe for the FP32 path
+// (fp_bits.cuh), plain for FP64
 template <typename Tq>
 __device__ __forceinline__ Tq to_q(double x) {
   if constexpr (sizeof(Tq) == 4) return d2f_trunc(x); else return x;
-}
-template <typename Tq>
-__device__ __forceinline__ double from_q(Tq x) {
-  if constexpr (sizeof(Tq) == 4) return f2d_exact(x); else return x;
 }
 
 // Sums of products in double, or in FP32 pairs: products exact through fmaf, the

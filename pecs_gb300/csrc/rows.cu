@@ -624,22 +624,6 @@ void check_smem(size_t bytes) {
   if (bytes > kRowsSmem) throw PecsError(PECS_E_ARG, "front too large for shared memory");
 }
 
-// launches with programmatic stream serialisation
-template <typename... P, typename... A>
-void launch_pdl(void (*fn)(P...), dim3 grid, size_t smem, cudaStream_t st, A... args) {
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(kRowsThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  PECS_CUDA(cudaLaunchKernelEx(&cfg, fn, args...));
-}
-
 template <typename T, int RB, bool FWD, bool ASM>
 void launch_level(const RowsDirView& B, const RowSets& S, int n_sets, const RowLevel& L, int max_nrhs,
                   cudaStream_t st) {
@@ -652,13 +636,13 @@ void launch_level(const RowsDirView& B, const RowSets& S, int n_sets, const RowL
       A.set[q] = AsmRange{L.col[q], L.n_col[q], L.d[q], L.upd[q], L.n_upd[q]};
       most = std::max(most, (long long)(L.n_col[q] + L.n_upd[q]) * S.set[q].nrhs);
     }
-    launch_pdl(k_assemble<T>, dim3((unsigned)((most + 255) / 256), n_sets), 0, st, B, S, A);
+    launch_pdl(k_assemble<T>, dim3((unsigned)((most + 255) / 256), n_sets), 256, 0, st, B, S, A);
   }
   const RowsSmem m = smem_of<T>(L.shape, RB, L.ts);
   check_smem((size_t)m.team_bytes * teams);
   const int tb = (L.n_tile + teams - 1) / teams;
-  launch_pdl(k_rows<T, RB, FWD, ASM>, dim3(tb + L.n_batch, (max_nrhs + RB - 1) / RB), (size_t)m.team_bytes * teams, st, B,
-             S, L.first, L.n_tile, tb, lg, m);
+  launch_pdl(k_rows<T, RB, FWD, ASM>, dim3(tb + L.n_batch, (max_nrhs + RB - 1) / RB), kRowsThreads,
+             (size_t)m.team_bytes * teams, st, B, S, L.first, L.n_tile, tb, lg, m);
 }
 
 void allow_smem(const void* fn) {

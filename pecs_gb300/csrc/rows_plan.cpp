@@ -2,11 +2,9 @@
 #include "rows_plan.hpp"
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <numeric>
 #include <stdexcept>
-#include <thread>
 
 #include "dense.hpp"
 
@@ -84,16 +82,6 @@ RowsSmem rows_smem(const RowShape& P, int vr, int rb, int ts) {
 
 namespace {
 
-template <typename F>
-void parallel(int n, F f) {
-  const int threads = (int)std::max(1u, std::min(std::thread::hardware_concurrency(), 16u));
-  std::atomic<int> next(0);
-  // a thread takes about as long to start as 64 nodes of a small mesh to plan
-  dense::run_threads(std::max(1, std::min(threads, n / 64)), [&](int) {
-    for (int i; (i = next.fetch_add(1)) < n;) f(i);
-  });
-}
-
 // A batch applies small leaves thread by output; its columns are read once per
 // output, so only FP64 values (no conversions) and short rows.
 constexpr int kBatchArea = 1280, kBatchCols = 64, kBatchRows = 256;
@@ -104,7 +92,7 @@ void pack(const RowsPlan& P, const std::vector<const MfFactor*>& factors, int d,
   std::vector<char> batch(D.items.size(), 0);
   for (const RowLevel& L : D.levels)
     for (int i = 0; i < L.n_batch; ++i) batch[L.first + L.n_tile + i] = 1;
-  parallel((int)D.items.size(), [&](int i) {
+  dense::parallel_for((int)D.items.size(), 64, [&](int i) {
     const RowItem& it = D.items[i];
     T* p = out + it.off;
     // a batch's nodes follow one another in the source list
@@ -184,7 +172,7 @@ RowsPlan plan_rows(const std::vector<const MfFactor*>& factors, int vr, int max_
     if (is_batch(g, 1)) nodes[g].level[1] = nl[1] - 1;
   const int N = (int)nodes.size();
   R.spans.resize(N);
-  parallel(N, [&](int g) { R.spans[g] = node_spans(*factors[nodes[g].set], nodes[g].j); });
+  dense::parallel_for(N, 64, [&](int g) { R.spans[g] = node_spans(*factors[nodes[g].set], nodes[g].j); });
   // nodes in level order (tiles, then batches by shape), and the lists
   std::vector<std::vector<int>> lv[2];
   for (int d = 0; d < 2; ++d) {

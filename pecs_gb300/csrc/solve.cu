@@ -208,7 +208,6 @@ struct PanelShape {
 // every thread once the block tile's copies are in flight and before any
 // vector is read; it returns false when the inputs could not be waited for,
 // and the item then writes NaN (the solve's results are flagged non-finite).
-// main_done() is called once the item no longer reads its inputs.
 template <typename T, int RPL, bool FWD, typename SVT, typename Wait>
 __device__ __forceinline__ void panel_tile(const BankView& B, const SVT& S, const PanelItem& I, int rc0,
                                            const PanelShape& P, unsigned char* smem_raw, Wait wait_inputs) {
@@ -756,7 +755,8 @@ __host__ __device__ constexpr size_t panel_warp_bytes(int max_k, int rows_pad, i
 // One leaf-level node applied by one warp to the right-hand-side chunk at rc0;
 // `base` is the warp's shared-memory slice.  wait_inputs() (every lane) is
 // called once the block's copies are in flight and before any vector is read;
-// false: the inputs could not be waited for and the node writes NaN.
+// false: the inputs could not be waited for and the node writes NaN.  main_done() is
+// called once the node no longer reads its inputs.
 template <typename T, int RPL, bool FWD, typename SVT, typename Wait, typename Done>
 __device__ __forceinline__ void panel_warp_node(const BankView& B, const SVT& S, const PanelItem& I, int rc0,
                                                 int max_k, int rows_pad, unsigned char* base, Wait wait_inputs,
@@ -858,7 +858,7 @@ __global__ void __launch_bounds__(kSolveThreads)
 // ---- flow sweeps -------------------------------------------------------------
 // One persistent launch per sweep direction instead of one launch per tree
 // level.  The direction's work entries are listed in topological order
-// (forward: by height, backward: by depth); every CTA repeatedly takes the
+// (forward from the lowest height up, backward from the greatest down); every CTA repeatedly takes the
 // next entry from a ticket counter and, before reading any vector, waits until
 // the entry's node has its inputs: forward, every item of its children has
 // finished (their update rows are written); backward, every item of its
@@ -968,22 +968,6 @@ void set_panel_smem_limit() {
   };
   set((const void*)k_panel_tiles<T, true, SVT>, kTileSmem);
   set((const void*)k_panel_tiles<T, false, SVT>, kTileSmem);
-}
-
-// launches with programmatic stream serialisation
-template <typename... P, typename... A>
-void launch_pdl(void (*fn)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  PECS_CUDA(cudaLaunchKernelEx(&cfg, fn, args...));
 }
 
 // Shared memory of a level's tiles: the columns of its longest tile at once where
@@ -1104,9 +1088,9 @@ FlowPlanHost plan_flow(const FlowNodes& nd, bool forward, int top, int rpl, int 
                        int n_sm) {
   FlowPlanHost H;
   const int n_nodes = (int)nd.s.size();
-  const std::vector<std::vector<int>>& lv_all = forward ? nd.by_height : nd.by_depth;
-  // the covered levels in ticket order (forward: the highest heights, from
-  // the lowest of them up; backward: depths 0 .. top-1)
+  const std::vector<std::vector<int>>& lv_all = forward ? nd.up : nd.down;
+  // the covered levels in ticket order (forward: the greatest heights, from the
+  // lowest of them up; backward: the same from the greatest down)
   const int L = (int)lv_all.size();
   top = std::min(std::max(top, 1), L);
   const std::vector<std::vector<int>> lv(forward ? lv_all.begin() + (L - top) : lv_all.begin(),
@@ -1244,19 +1228,10 @@ FlowPlanHost plan_flow(const FlowNodes& nd, bool forward, int top, int rpl, int 
 
 BankView FactorBank::view() const {
   BankView v;
-  v.s = s_.p;
-  v.m = m_.p;
-  v.goff = goff_.p;
-  v.hoff = hoff_.p;
-  v.own_off = own_off_.p;
-  v.upd_off = upd_off_.p;
-  v.w_off = w_off_.p;
-  v.cm_off = cm_off_.p;
   v.own_idx = own_idx_.p;
   v.upd_idx = upd_idx_.p;
   v.cmap_ptr = cmap_ptr_.p;
   v.cmap_idx = cmap_idx_.p;
-  v.node_set = node_set_.p;
   v.G = G_.p();
   v.H = H_.p();
   return v;
@@ -1393,19 +1368,10 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
   // Levels by depth mix cell blocks of 8 rows with separators of hundreds.
   bl.assign(fl.rbegin(), fl.rend());
   entries_ = go + ho;
-  s_.upload(hs);
-  m_.upload(hm);
-  own_off_.upload(own_off);
-  upd_off_.upload(upd_off);
-  w_off_.upload(w_off);
-  cm_off_.upload(cm_off);
   own_idx_.upload(own_idx);
   upd_idx_.upload(upd_idx);
   cmap_ptr_.upload(cmap_ptr);
   cmap_idx_.upload(cmap_idx);
-  node_set_.upload(node_set);
-  goff_.upload(goff);
-  hoff_.upload(hoff);
   // blocks of these nodes (forward Gf, backward Hb), column-major, one after another
   auto column_major = [&](const std::vector<int>& nodes, bool forward, BankValues& out) {
     size_t n = 0;
@@ -1527,8 +1493,8 @@ void FactorBank::build(const std::vector<const MfFactor*>& factors, int precisio
     PECS_CUDA(cudaGetDevice(&dev));
     PECS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
     FlowNodes nodes{hs, hm, node_set, w_off, own_off, upd_off, cm_off, cmap_ptr, goff, hoff, parent, {}, {}};
-    for (auto& l : fl) nodes.by_height.push_back(l.nodes);
-    for (auto& l : bl) nodes.by_depth.push_back(l.nodes);
+    for (auto& l : fl) nodes.up.push_back(l.nodes);
+    for (auto& l : bl) nodes.down.push_back(l.nodes);
     flow_cfg_.clear();
     flow_sel_ = -1;
     const int n_levels = (int)std::max(fl.size(), bl.size());

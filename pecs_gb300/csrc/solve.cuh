@@ -5,7 +5,8 @@
 // factor is bound to a "RHS set": a list of right-hand sides that share the
 // factor (e.g. electrons and holes of every instance when their mobilities
 // are equal), so that every stored factor entry read from HBM is applied to
-// all of them.  One kernel launch processes one tree level of every factor in
+// all of them.  One or two kernel launches process one tree level of every factor in
+// the bank.  Few right-hand sides per set: rows.cuh.  Many: each node's block is a
 // small dense GEMM: forward, a level's columns -- right-hand side minus the children's
 // updates -- are assembled once per node, then every tile of rows takes its packed
 // values by one bulk copy and the vectors' rows (interleaved layout: a dof's values
@@ -23,24 +24,16 @@
 namespace pecs {
 
 constexpr int kMaxSets = 4;
-constexpr int kTargetCtas = 152; // SMs of a GB300: levels with fewer wide items split rows
+constexpr int kTargetCtas = 152; // SMs of a GB300: FP32 levels with fewer tiles take shorter ones
 constexpr int kSolveThreads = 256;
 constexpr int kPanelMinRhs = 32;  // right-hand sides per set from which banks use the panel kernels
 
-struct BankView {  // device pointers, passed by value to kernels
-  const int* s;
-  const int* m;
-  const long long* goff;
-  const long long* hoff;
-  const int* own_off;
-  const int* upd_off;
-  const int* w_off;
-  const int* cm_off;
+// Flow sweeps and leaf warps: device pointers, passed by value to kernels.
+struct BankView {
   const int* own_idx;
   const int* upd_idx;
   const int* cmap_ptr;
   const int* cmap_idx;
-  const int* node_set;
   const void* G;
   const void* H;
 };
@@ -145,7 +138,7 @@ struct FlowPlan {
 
 // Host description of the factor tree a flow plan is built from (bank-wide
 // node numbering; per node: sizes, RHS set, offsets, child-map pointer and
-// parent, and the nodes of each height and depth).
+// parent, and the nodes of each height).
 struct FlowNodes {
   const std::vector<int>& s;
   const std::vector<int>& m;
@@ -158,7 +151,7 @@ struct FlowNodes {
   const std::vector<long long>& goff;
   const std::vector<long long>& hoff;
   const std::vector<int>& parent;
-  std::vector<std::vector<int>> by_height, by_depth;
+  std::vector<std::vector<int>> up, down;  // by height, from the leaves and from the root
 };
 
 // A flow plan before upload: the launch shape, the items with their waits and
@@ -175,8 +168,7 @@ struct FlowPlanHost {
 };
 
 // Builds one direction's flow plan over the `top` tree levels nearest the root
-// (forward: the highest heights; backward: the smallest depths; top >= the
-// level count: all of them) for rpl right-hand sides per lane and at most
+// (the greatest heights; top >= the level count: all of them) for rpl right-hand sides per lane and at most
 // max_nrhs right-hand sides per set (host only; esz: bytes per value; kc_max:
 // staged block columns per chunk; n_sm: multiprocessors to fill).
 FlowPlanHost plan_flow(const FlowNodes& nd, bool forward, int top, int rpl, int max_nrhs, int kc_max, int esz,
@@ -252,9 +244,7 @@ class FactorBank {
   int n_sets_ = 0, max_nrhs_ = 0;
   int set_wtotal_[kMaxSets] = {0, 0, 0, 0};
   long long entries_ = 0;
-  DBuf<int> s_, m_, own_off_, upd_off_, w_off_, cm_off_, own_idx_, upd_idx_, cmap_ptr_, cmap_idx_,
-      node_set_;
-  DBuf<long long> goff_, hoff_;
+  DBuf<int> own_idx_, upd_idx_, cmap_ptr_, cmap_idx_;
   BankValues G_, H_;  // flow sweeps: every block, column-major
   std::vector<PanelPlan> pfwd_, pbwd_;
   bool panel_ = false;
