@@ -354,9 +354,9 @@ __global__ void k_residual_df_il(ElemSets E, int in_place) {
 // pairs' arithmetic keeps the FMA pipe and the x rows the L1 busy about half of the time
 // each: 49,152 rows x 128 right-hand sides x 2 sets take 155 us with the right-hand
 // sides of the CTA's eight rows read together, 169 with each row's by its own lanes.
-// Tried without gain, us a step of 64 instances (1,000): two right-hand sides per
-// instruction (f32x2) and two or four entries in flight (12 and 42 more: fewer warps), the
-// x rows of the eight rows staged in shared memory (8 more).
+// Tried without gain: two right-hand sides per instruction (f32x2) with two or four
+// entries in flight (fewer warps), the x rows of the eight rows staged in shared memory by
+// bulk copies (175 us).
 __device__ __forceinline__ void ld_pairs4(const float* p, float2 (&v)[4]) {
   const float4 t = *reinterpret_cast<const float4*>(p);
   v[0] = make_float2(t.x, 0.f);
@@ -1327,8 +1327,9 @@ struct Engine {
       };
       n = 0;
       for (auto& x : src) {
-        if (piece.size() + x.size() > kPiece / 8) copy(piece), piece.clear();
-        if (x.size() >= kWhole / 8)
+        const bool whole = x.size() >= kWhole / 8;
+        if (whole || piece.size() + x.size() > kPiece / 8) copy(piece), piece.clear();
+        if (whole)
           copy(x);
         else
           piece.insert(piece.end(), x.begin(), x.end());
